@@ -226,10 +226,11 @@ int lbm_implicit_step_adjoint(int prec, const lbm_implicit_adj_args* a, void* st
  *   af   [E][M][J][K][7] cplx  weighted Fourier inputs of the analysis
  *   afs  [E][M][J][2] cplx     gt_pi, pi(t-dt)
  *   tend [E][4][NS][K] cplx, tends [E][2][NS] cplx   explicit tendencies
- *   grid6 [E][J][6 + 6K][I] float (FP32 mode; NULL in FP64 mode): grid rows
- *        pi, pi_x, pi_y, U-sum, V-sum, D-sum, then per level u, v, vor,
- *        div, T, q (u and v divided by a cos)
- *   grid9 [E][J][2 + 9K][I] float (FP32 mode): gt_pi, pi(t - dt), then per
+ *   grid6 [E][J][6 + 6K][I] real (of the working precision; required in FP32
+ *        mode; in FP64 mode both grid6 and grid9, or both NULL for the slower
+ *        one-kernel grid part): grid rows pi, pi_x, pi_y, U-sum, V-sum, D-sum,
+ *        then per level u, v, vor, div, T, q (u and v divided by a cos)
+ *   grid9 [E][J][2 + 9K][I] real (as grid6): gt_pi, pi(t - dt), then per
  *        level gt, xu, g, yu, fu, fv, ke, xv, yv
  *   symp, symh [NS][J/2]       P and H at the northern latitudes, packed rows
  *   tw [I] cplx; jfac [4][J]: gw, gwdel*coslat, 1/(a coslat), coslat
@@ -346,7 +347,7 @@ int lbm_stepper_run(const lbm_stepper_desc* d, const lbm_step_ctl* ctl,
  * grid-point tendency with the longitude transforms, 1 = Legendre analysis,
  * 2 = implicit update, 3 = Legendre synthesis.  Launching 0..3 in order is
  * the same as lbm_stepper_run for that step.  In FP32 mode kernel 0 is three
- * launches, also available one by one: 4 = longitude synthesis (sf, sfs ->
+ * launches (in FP64 mode too, where grid6 and grid9 are given), in FP32 also available one by one: 4 = longitude synthesis (sf, sfs ->
  * grid6), 5 = column algebra (grid6 -> grid9, grid ps), 6 = longitude
  * analysis (grid9 -> af, afs); 4, 5, 6 in order equal 0. */
 int lbm_stepper_launch(const lbm_stepper_desc* d, const lbm_step_ctl* ctl,
@@ -428,9 +429,10 @@ int lbm_link_copy(void* dst, const void* src, int64_t bytes, void* stream);
  * arrays through the array backend on every call.
  *
  * lbm_stepper_run_noalloc is lbm_stepper_prime followed by lbm_stepper_run
- * (same kernels, same results) for callers that cannot allocate device
- * memory for the intermediate buffers (sf, sfs, af, afs, tend, tends and the
- * FP32 grid rows grid6, grid9): a
+ * (same kernels, same results; FP64 without room for the grid rows runs the
+ * one-kernel grid part) for callers that cannot allocate device memory for the
+ * intermediate buffers (sf, sfs, af, afs, tend, tends and the grid rows grid6,
+ * grid9): a
  * host that embeds the dynamical core behind an FFI and hands the library
  * only its state, operator and forcing buffers -- for instance because all of
  * its device memory belongs to another runtime's pool, or because cudaMalloc

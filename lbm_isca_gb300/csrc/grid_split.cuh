@@ -1,11 +1,11 @@
-// FP32 grid-point step split into three kernels with full-size work per
-// launch (included by stepper.cu):
+// Grid-point step split into three kernels with full-size work per launch
+// (included by stepper.cu; the FP64 longitude transforms are in grid_fft.cuh):
 //
 //   k_idft  per (latitude, member): the longitude synthesis of the six
 //           surface rows and the 6 K level rows of sf/sfs -> grid6
 //           [E][J][6 + 6K][I] (surface pi, pi_x, pi_y, U-sum, V-sum, D-sum,
 //           then per level u cos-scaled, v, vor, div, T, q);
-//   k_alg   one thread per grid column: the grid-point algebra of
+//   k_alg   (FP32 and FP64) one thread per grid column: the grid-point algebra of
 //           dynamics.py:176-262 in one upward pass over the levels (sigma-dot,
 //           the reference-temperature split of the temperature equation and the
 //           hydrostatic prefix running in registers) -> grid9
@@ -181,130 +181,150 @@ __global__ void __launch_bounds__(IDFT_NT) k_idft(SD<float> d, const float2* __r
 }
 
 // ---------------------------------------------------------------------------
-// One thread per column (blockDim = I).  The kernel waits on global loads;
-// the minimum resident blocks per SM keep 92 / 80 / 80 registers at I = 64 /
-// 128 / 256 -- at 128 that is six blocks instead of five, 10% faster at 512
-// members (seven and eight spill and are slower).
-template <int I>
-__global__ void __launch_bounds__(I, I == 64 ? 10 : (I == 128 ? 6 : 3))
-    k_alg(SD<float> d, int ps_mode) {
-  const int j = blockIdx.x, e = blockIdx.y, c = threadIdx.x;
+// One thread per column, BT columns of one latitude per block (grid
+// (J I / BT, E)).  FP32: the kernel waits on global loads; the minimum resident
+// blocks per SM keep 92 / 80 / 80 registers at I = 64 / 128 / 256 -- at 128 that
+// is six blocks instead of five, 10% faster at 512 members (seven and eight
+// spill and are slower).  FP64: about 85 FP64 instructions per level (no
+// division: the reciprocal layer thickness is formed once per block; 27 us a member
+// at T42L20), bound by
+// the FP64 pipe; 32 columns per block spread one member over every SM.
+template <typename R, int I, int BT, int MINB>
+__global__ void __launch_bounds__(BT, MINB) k_alg(SD<R> d, int ps_mode) {
+  constexpr int NB = I / BT;
+  const int j = blockIdx.x / NB, e = blockIdx.y;
+  const int c = (blockIdx.x % NB) * BT + threadIdx.x;
   const int J = d.J, K = d.K;
-  __shared__ float vert[LBM_VERT_COUNT * 65];
-  for (int x = c; x < LBM_VERT_COUNT * (K + 1); x += I) vert[x] = d.vert[x];
+  __shared__ R vert[LBM_VERT_COUNT * 65];
+  __shared__ R rds[64];                              // 1 / dsig
+  for (int x = threadIdx.x; x < LBM_VERT_COUNT * (K + 1); x += BT) vert[x] = d.vert[x];
+  for (int x = threadIdx.x; x < K; x += BT) rds[x] = R(1) / vrow(d, LBM_VERT_DSIG, x);
   __syncthreads();
   const int VS = K + 1;
   auto V = [&](int row, int k) { return vert[row * VS + k]; };
-  const float* g6 = d.grid6 + ((size_t)e * J + j) * idft_rows(K) * I + c;
-  float* g9 = d.grid9 + ((size_t)e * J + j) * fdft_rows(K) * I + c;
-  const float eps = d.epsvt, kappa = d.kappa;
+  const R* g6 = d.grid6 + ((size_t)e * J + j) * idft_rows(K) * I + c;
+  R* g9 = d.grid9 + ((size_t)e * J + j) * fdft_rows(K) * I + c;
+  const R eps = d.epsvt, kappa = d.kappa;
 
   // ---- surface: column sums, pi tendency, grid ps filter ----
   const size_t g2 = (size_t)j * I + c;
-  const float* b2 = d.b2;
-  const float pixb = b2[(B2_PIX * J) * I + g2], piyb = b2[(B2_PIY * J) * I + g2];
-  const float psbar = b2[(B2_PSBAR * J) * I + g2];
-  const float usum = b2[(B2_USUM * J) * I + g2], vsum = b2[(B2_VSUM * J) * I + g2];
-  const float pi = g6[0], pix = g6[I], piy = g6[2 * I];
-  const float uh = g6[3 * I], vh = g6[4 * I], dh = g6[5 * I];
-  const float sx = pixb * uh + piyb * vh + pix * usum + piy * vsum;   // sum dsig v.grad(pi)
-  const float stot = dh + sx;
+  const R* b2 = d.b2;
+  const R pixb = b2[(B2_PIX * J) * I + g2], piyb = b2[(B2_PIY * J) * I + g2];
+  const R psbar = b2[(B2_PSBAR * J) * I + g2];
+  const R usum = b2[(B2_USUM * J) * I + g2], vsum = b2[(B2_VSUM * J) * I + g2];
+  const R pi = g6[0], pix = g6[I], piy = g6[2 * I];
+  const R uh = g6[3 * I], vh = g6[4 * I], dh = g6[5 * I];
+  const R sx = pixb * uh + piyb * vh + pix * usum + piy * vsum;   // sum dsig v.grad(pi)
+  const R stot = dh + sx;
   g9[0] = -sx;                                   // gt_pi
   {
     const size_t gp = (size_t)e * J * I + g2;
-    const float pscur = psbar * expm1f(pi);
-    float pb = d.psb[gp];
+    const R pscur = psbar * expm1(pi);
+    R pb = d.psb[gp];
     if (ps_mode == 1) {
       pb = d.psa[gp];
     } else if (ps_mode == 2) {
-      const float pa = d.psa[gp];
-      pb = pa + d.robert * (pb - 2.f * pa + pscur);
+      const R pa = d.psa[gp];
+      pb = pa + d.robert * (pb - R(2) * pa + pscur);
     }
     if (ps_mode != 0) {
       d.psb[gp] = pb;
       d.psa[gp] = pscur;
     }
-    g9[I] = log1pf(pb / psbar);                  // pi(t - dt)
+    g9[I] = log1p(pb / psbar);                   // pi(t - dt)
   }
 
   // ---- levels, bottom up ----
   // per-field offsets into b3 (int: the basic state of one latitude is small)
   const int b3f = J * K * I;
-  const float* bk = d.b3 + (size_t)j * K * I + c;             // level k, field 0
-  const float* bsk = d.bsd + (size_t)j * (K + 1) * I + c;     // interface k
-  const float* gl = g6 + (size_t)6 * I;                       // level k rows
-  float* go = g9 + (size_t)2 * I;
-  float sdlo = (V(LBM_VERT_SIGM, 0) - 1.f) * stot;   // sigma-dot at k - 1/2
-  float prefd = 0.f, prefp = 0.f, pref3 = 0.f;
+  const R* bk = d.b3 + (size_t)j * K * I + c;             // level k, field 0
+  const R* bsk = d.bsd + (size_t)j * (K + 1) * I + c;     // interface k
+  const R* gl = g6 + (size_t)6 * I;                       // level k rows
+  R* go = g9 + (size_t)2 * I;
+  R sdlo = (V(LBM_VERT_SIGM, 0) - R(1)) * stot;      // sigma-dot at k - 1/2
+  R prefd = R(0), prefp = R(0), pref3 = R(0);
   // level window: m = k-1, 0 = k, p = k+1 (u, v, T, q); vorticity and
   // divergence of level k only
-  float um = 0.f, vm = 0.f, tm_ = 0.f, qm = 0.f;
-  float u0 = gl[SF_U * I], v0 = gl[SF_V * I], t0 = gl[SF_T * I], q0 = gl[SF_Q * I];
-  float vo0 = gl[SF_VOR * I], dv0 = gl[SF_DIV * I];
-  float hum = 0.f, hvm = 0.f, htm = 0.f, hqm = 0.f;    // half differences at k - 1
-  float sb0 = __ldg(bsk);
+  R u0 = gl[SF_U * I], v0 = gl[SF_V * I], t0 = gl[SF_T * I], q0 = gl[SF_Q * I];
+  R vo0 = gl[SF_VOR * I], dv0 = gl[SF_DIV * I];
+  R um = R(0), vm = R(0), tm_ = R(0), qm = R(0);       // level k - 1
+  R hum = R(0), hvm = R(0), htm = R(0), hqm = R(0);    // half differences at k - 1
+  R sb0 = __ldg(bsk);
   for (int k = 0; k < K; ++k) {
     const bool hasm = k >= 1, hasp = k + 1 <= K - 1;
-    float up = u0, vp = v0, tp = t0, qp = q0, vop = 0.f, dvp = 0.f;
+    R up = u0, vp = v0, tp = t0, qp = q0, vop = R(0), dvp = R(0);
     if (hasp) {
-      const float* gn = gl + SF_N * I;
+      const R* gn = gl + SF_N * I;
       up = gn[SF_U * I]; vp = gn[SF_V * I]; tp = gn[SF_T * I]; qp = gn[SF_Q * I];
       vop = gn[SF_VOR * I]; dvp = gn[SF_DIV * I];
     }
-    const float ub = __ldg(bk + B_U * b3f), vb = __ldg(bk + B_V * b3f);
-    const float tb = __ldg(bk + B_T * b3f), qb = __ldg(bk + B_Q * b3f);
-    const float tvb = __ldg(bk + B_TV * b3f), absv = __ldg(bk + B_ABSVOR * b3f);
-    const float divb = __ldg(bk + B_DIV * b3f), x5b = __ldg(bk + B_X5 * b3f);
-    const float tdev = __ldg(bk + B_TDEV * b3f), tvdev = __ldg(bk + B_TVDEV * b3f);
-    const float hup = __ldg(bk + B_HDU * b3f), hvp = __ldg(bk + B_HDV * b3f);
-    const float htp = __ldg(bk + B_HDT * b3f), hqp = __ldg(bk + B_HDQ * b3f);
-    const float sb1 = __ldg(bsk + I);
-    const float dsk = V(LBM_VERT_DSIG, k), rdsk = 1.f / dsk;
+    const R ub = __ldg(bk + B_U * b3f), vb = __ldg(bk + B_V * b3f);
+    const R tb = __ldg(bk + B_T * b3f), qb = __ldg(bk + B_Q * b3f);
+    const R tvb = __ldg(bk + B_TV * b3f), absv = __ldg(bk + B_ABSVOR * b3f);
+    const R divb = __ldg(bk + B_DIV * b3f), x5b = __ldg(bk + B_X5 * b3f);
+    const R tdev = __ldg(bk + B_TDEV * b3f), tvdev = __ldg(bk + B_TVDEV * b3f);
+    const R hup = __ldg(bk + B_HDU * b3f), hvp = __ldg(bk + B_HDV * b3f);
+    const R htp = __ldg(bk + B_HDT * b3f), hqp = __ldg(bk + B_HDQ * b3f);
+    const R sb1 = __ldg(bsk + I);
+    const R dsk = V(LBM_VERT_DSIG, k), rdsk = rds[k];
     // column scans through level k
-    const float pa = u0 * pixb + ub * pix + v0 * piyb + vb * piy;      // v.grad(pi)
-    const float sdup = sdlo + dsk * (dv0 + pa - stot);               // sigma-dot at k + 1/2
+    const R pa = u0 * pixb + ub * pix + v0 * piyb + vb * piy;        // v.grad(pi)
+    const R sdup = sdlo + dsk * (dv0 + pa - stot);                   // sigma-dot at k + 1/2
     prefd += dsk * dv0;
     prefp += dsk * pa;
-    const float xv = eps * (t0 * qb + tb * q0);                       // Tv' - T'
-    const float phiv = pref3 + V(LBM_VERT_RALPHA, k) * xv;             // (WW (Tv'-T'))_k
+    const R xv = eps * (t0 * qb + tb * q0);                          // Tv' - T'
+    const R phiv = pref3 + V(LBM_VERT_RALPHA, k) * xv;               // (WW (Tv'-T'))_k
     pref3 += V(LBM_VERT_RDLOG3, k) * xv;
-    const float sdv = dh - prefd, spv = sx - prefp;                   // suffix sums above k
-    const float sd0 = hasm ? sdlo : 0.f, sd1 = hasp ? sdup : 0.f;
+    const R sdv = dh - prefd, spv = sx - prefp;                      // suffix sums above k
     // vertical advection of dynamics.py's _vert_advect written in differences,
     //   (s1 (f[k+1] - f[k]) / 2 + s0 (f[k] - f[k-1]) / 2) / dsig_k
     // (at the bottom / top the missing half becomes +s0 f[k] / -s1 f[k]),
     // equal to the flux form (F[k+1/2] - F[k-1/2] - f[k] (s1 - s0)) / dsig_k
     // without cancelling the f[k] (s1 - s0) part: perturbation fields by the
-    // basic sigma-dot, basic fields (half differences precomputed in FP64)
-    // by sigma-dot'
-    auto vp_ = [&](float fm, float f0, float fp) {
-      const float a = hasp ? 0.5f * sb1 * (fp - f0) : -sb1 * f0;
-      const float b = hasm ? 0.5f * sb0 * (f0 - fm) : sb0 * f0;
-      return (a + b) * rdsk;
+    // basic sigma-dot, basic fields (half differences precomputed in FP64; zero
+    // above the top level) by sigma-dot' (zero at the column's ends).  FP64
+    // takes the reciprocal thickness into the four interface factors first
+    // (7 operations a field instead of 12)
+    const R sd0 = hasm ? sdlo : R(0), sd1 = hasp ? sdup : R(0);
+    const R c1 = sb1 * (hasp ? R(0.5) * rdsk : -rdsk), c0 = sb0 * (hasm ? R(0.5) * rdsk : rdsk);
+    const R s1 = sd1 * rdsk, s0 = sd0 * rdsk;
+    // perturbation field f of basic field fb, half differences hm, hp of fb
+    auto vp_ = [&](R fm, R f0, R fp) {
+      if constexpr (sizeof(R) == 8) {
+        return c1 * (hasp ? fp - f0 : f0) + c0 * (hasm ? f0 - fm : f0);
+      } else {
+        const R a = hasp ? R(0.5) * sb1 * (fp - f0) : -sb1 * f0;
+        const R b = hasm ? R(0.5) * sb0 * (f0 - fm) : sb0 * f0;
+        return (a + b) * rdsk;
+      }
     };
-    auto vb_ = [&](float f0, float hm, float hp) {
-      const float a = hasp ? sd1 * hp : -sd1 * f0;
-      const float b = hasm ? sd0 * hm : sd0 * f0;
-      return (a + b) * rdsk;
+    auto vb_ = [&](R f0, R hm, R hp) {
+      if constexpr (sizeof(R) == 8) {
+        return s1 * hp + s0 * hm;
+      } else {
+        const R a = hasp ? sd1 * hp : -sd1 * f0;
+        const R b = hasm ? sd0 * hm : sd0 * f0;
+        return (a + b) * rdsk;
+      }
     };
     // temperature: adiabatic term and the reference-temperature matrix with
     // Tref cancelled algebraically
-    const float tv = t0 + xv;
-    const float al = V(LBM_VERT_ALPHA, k), w3 = V(LBM_VERT_W3, k);
-    const float adtm = -kappa * (tv * x5b + tvdev * (al * dv0 + w3 * sdv) +
-                                 tvb * (V(LBM_VERT_WP, k) * pa + w3 * spv));
-    const float hadv = t0 * divb + tdev * dv0;
-    go[0 * I] = adtm + hadv + vp_(tm_, t0, tp) + vb_(tb, htm, htp);  // gt
+    const R tv = t0 + xv;
+    const R al = V(LBM_VERT_ALPHA, k), w3 = V(LBM_VERT_W3, k);
+    const R adtm = -kappa * (tv * x5b + tvdev * (al * dv0 + w3 * sdv) +
+                             tvb * (V(LBM_VERT_WP, k) * pa + w3 * spv));
+    const R hadv = t0 * divb + tdev * dv0;
+    go[0 * I] = adtm + hadv + vp_(tm_, t0, tp) + vb_(tb, htm, htp);   // gt
     go[1 * I] = u0 * tdev + ub * t0;                                  // xu
-    const float rcpg = V(LBM_VERT_RCPG, k);
-    const float fu = v0 * absv + vb * vo0 - rcpg * (tv * pixb + tvdev * pix) +
-                     vp_(um, u0, up) + vb_(ub, hum, hup);
-    const float fv = -u0 * absv - ub * vo0 - rcpg * (tv * piyb + tvdev * piy) +
-                     vp_(vm, v0, vp) + vb_(vb, hvm, hvp);
+    const R rcpg = V(LBM_VERT_RCPG, k);
+    const R fu = v0 * absv + vb * vo0 - rcpg * (tv * pixb + tvdev * pix) +
+                 vp_(um, u0, up) + vb_(ub, hum, hup);
+    const R fv = -u0 * absv - ub * vo0 - rcpg * (tv * piyb + tvdev * piy) +
+                 vp_(vm, v0, vp) + vb_(vb, hvm, hvp);
     go[4 * I] = fu;
     go[5 * I] = fv;
-    float ke = phiv + u0 * ub + v0 * vb;
-    if (!d.strictly_linear) ke += 0.5f * (u0 * u0 + v0 * v0);
+    R ke = phiv + u0 * ub + v0 * vb;
+    if (!d.strictly_linear) ke += R(0.5) * (u0 * u0 + v0 * v0);
     go[6 * I] = ke;
     go[7 * I] = v0 * tdev + vb * t0;                                  // xv
     go[2 * I] = q0 * divb + qb * dv0 + vp_(qm, q0, qp) + vb_(qb, hqm, hqp);   // g

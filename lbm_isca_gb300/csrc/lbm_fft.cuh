@@ -145,13 +145,21 @@ LBM_D void team_rfft_fwd(int t, const R* x, int xs, C2<R>* scr, const C2<R>* tw,
     v[r] = cmk<R>(x[(2 * n) * xs], x[(2 * n + 1) * xs]);
   }
   team_cfft<-1, I>(t, v, scr, tw, mask);
+  const R half = scale * R(0.5);
   for (int m = t; m < M; m += R1) {
-    C2<R> zk = scr[m];
-    C2<R> zc = conj(scr[(L - m) & (L - 1)]);
-    C2<R> ev = (zk + zc) * R(0.5);
-    C2<R> od = mul_i<-1>(zk - zc) * R(0.5);
-    C2<R> X = ev + cmul(tw[m], od);
-    out(m, X * scale);
+    const C2<R> zk = scr[m], zc = conj(scr[(L - m) & (L - 1)]), w = tw[m];
+    if constexpr (sizeof(R) == 8) {
+      // (ev + w od) scale / 2 with ev = zk + zc, od = -i (zk - zc): 10
+      // operations where the FP32 form below takes 16
+      const C2<R> ev = zk + zc, od = mul_i<-1>(zk - zc);
+      out(m, cmk<R>(fma(w.x, od.x, fma(-w.y, od.y, ev.x)) * half,
+                    fma(w.x, od.y, fma(w.y, od.x, ev.y)) * half));
+    } else {
+      C2<R> ev = (zk + zc) * R(0.5);
+      C2<R> od = mul_i<-1>(zk - zc) * R(0.5);
+      C2<R> X = ev + cmul(w, od);
+      out(m, X * scale);
+    }
   }
   __syncwarp(mask);
 }
@@ -167,13 +175,38 @@ LBM_D void team_rfft_inv(int t, In in, int M, C2<R>* scr, const C2<R>* tw, R* x,
 #pragma unroll
   for (int r = 0; r < R2; ++r) {
     const int n = t + R1 * r;
-    C2<R> y = cmk<R>(R(0), R(0));
-    if (n < M) y = in(n);
-    if (n == 0) y.y = R(0);
-    C2<R> yc = cmk<R>(R(0), R(0));
-    if (n > 0 && L - n < M) yc = conj(in(L - n));
-    C2<R> w = conj(tw[n]);
-    v[r] = (y + yc) + mul_i<1>(cmul(w, y - yc));
+    if constexpr (sizeof(R) == 4) {
+      C2<R> y = cmk<R>(R(0), R(0));
+      if (n < M) y = in(n);
+      if (n == 0) y.y = R(0);
+      C2<R> yc = cmk<R>(R(0), R(0));
+      if (n > 0 && L - n < M) yc = conj(in(L - n));
+      C2<R> w = conj(tw[n]);
+      v[r] = (y + yc) + mul_i<1>(cmul(w, y - yc));
+      continue;
+    }
+    // z_n = (y + yc) + i conj(tw_n) (y - yc), y = X_n and yc = conj X_{L-n},
+    // each zero beyond the truncation: a whole team below L - M (or from M on)
+    // skips the half of the pairing that is zero (FP64, bound by its pipe)
+    const C2<R> w = tw[n];
+    C2<R> s, q;
+    if (R1 * r + R1 <= L - M + 1 && R1 * r + R1 <= M) {
+      s = in(n);
+      if (n == 0) s.y = R(0);
+      q = s;
+    } else if (R1 * r >= M) {
+      s = cmk<R>(R(0), R(0));
+      if (L - n < M) s = conj(in(L - n));
+      q = cmk<R>(-s.x, -s.y);
+    } else {
+      C2<R> y = cmk<R>(R(0), R(0)), yc = cmk<R>(R(0), R(0));
+      if (n < M) y = in(n);
+      if (n == 0) y.y = R(0);
+      if (n > 0 && L - n < M) yc = conj(in(L - n));
+      s = y + yc;
+      q = y - yc;
+    }
+    v[r] = cmk<R>(fma(w.y, q.x, fma(-w.x, q.y, s.x)), fma(w.x, q.x, fma(w.y, q.y, s.y)));
   }
   team_cfft<1, I>(t, v, scr, tw, mask);
   // z_k is at scr[k]; x[2k] = Re z_k, x[2k+1] = Im z_k

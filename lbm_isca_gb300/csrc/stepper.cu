@@ -2,7 +2,10 @@
 // (model.py:213-247) for many members at once, with the prognostic state in
 // packed spectral space.
 //
-// One step = four launches:
+// One step = four parts (each one launch or more):
+//   grid part   three launches (k_ifft / k_idft, k_alg, k_ffft / k_fdft:
+//               grid_split.cuh, grid_fft.cuh) where the caller gives buffers
+//               for the grid rows (always in FP32), else
 //   k_grid      per (member, latitude): inverse FFTs of the synthesised
 //               Fourier fields, the whole grid-point tendency algebra of
 //               dynamics.py:176-262 level by level, forward FFTs, weighting;
@@ -47,7 +50,7 @@ template <typename R> struct SD {
   C2<R> *sa3, *sas, *sb3;
   R *psa, *psb;
   C2<R> *sf, *sfs, *af, *afs, *tend, *tends;
-  float *grid6, *grid9;
+  R *grid6, *grid9;
   int* err;
   int* err_member;
   int legendre;                          // 0 FMA; 3 or 6: tensor-core products
@@ -79,7 +82,7 @@ template <typename R> SD<R> make_sd(const lbm_stepper_desc& d) {
   s.psa = (R*)d.psa; s.psb = (R*)d.psb;
   s.sf = (C2<R>*)d.sf; s.sfs = (C2<R>*)d.sfs; s.af = (C2<R>*)d.af; s.afs = (C2<R>*)d.afs;
   s.tend = (C2<R>*)d.tend; s.tends = (C2<R>*)d.tends;
-  s.grid6 = (float*)d.grid6; s.grid9 = (float*)d.grid9;
+  s.grid6 = (R*)d.grid6; s.grid9 = (R*)d.grid9;
   s.err = d.err;
   s.err_member = d.err_member;
   s.legendre = d.legendre;
@@ -1040,6 +1043,7 @@ __global__ void k_ps_flush(SD<R> d, int ps_mode) {
 
 }  // namespace lbm
 #include "grid_split.cuh"
+#include "grid_fft.cuh"
 #include "legendre_tc.cuh"
 #include "synth_tc.cuh"
 #include "dft_tc.cuh"
@@ -1053,6 +1057,9 @@ template <> struct Cfg<float> {
 template <> struct Cfg<double> {
   static constexpr int NC = 2, KCA = 10, JG = 1, KCS = 10, SHV = 1;
 };
+
+// Resident k_alg blocks of I threads (see the kernel).
+template <int I> constexpr int alg_minb() { return I == 64 ? 10 : (I == 128 ? 6 : 3); }
 
 template <typename R, int I> constexpr int grid_kb() { return (sizeof(R) == 8 && I == 256) ? 2 : 4; }
 template <typename R, int I> constexpr int grid_nt() {
@@ -1165,7 +1172,7 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
     if (only < 0 || only == 0 || only == 4)
       k_idft<I><<<dim3(d.J, d.E), IDFT_NT, idft_smem(I, d.M), st>>>(d, d.dft);
     if (only < 0 || only == 0 || only == 5)
-      k_alg<I><<<dim3(d.J, d.E), I, 0, st>>>(d, c.ps_mode);
+      k_alg<R, I, I, alg_minb<I>()><<<dim3(d.J, d.E), I, 0, st>>>(d, c.ps_mode);
     if ((only < 0 || only == 0 || only == 6) && d.legendre && !(d.tc_off & 4) &&
         ftc_supported(I, d.K, d.N)) {
       const FtcPlan pl = ftc_plan(d.E, d.J, I, d.K, d.N);
@@ -1182,9 +1189,20 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
       k_fdft<I><<<persistent_grid((const void*)k_fdft<I>, pl.nt, smem, nunits), pl.nt, smem,
                   st>>>(d, d.dft, pl);
     }
-  } else {
-    if (only < 0 || only == 0)
+  } else if (only < 0 || only == 0) {
+    if (d.grid6 && d.grid9) {
+      // workspace for the grid rows: the grid part as three launches with
+      // enough blocks for one member (1 member of T42L20 675 -> 181 us, 32
+      // members 9.27 -> 2.93 ms)
+      using G = GridFft<I>;
+      k_ifft<R, I><<<dim3(d.J, 1 + (d.K + G::LI - 1) / G::LI, d.E), G::NTI,
+                     G::template ifft_smem<R>(d.M), st>>>(d);
+      k_alg<R, I, 32, 1><<<dim3(d.J * (I / 32), d.E), 32, 0, st>>>(d, c.ps_mode);
+      k_ffft<R, I><<<dim3(d.J, 1 + (d.K + G::LF - 1) / G::LF, d.E), G::NTF,
+                     G::template ffft_smem<R>(d.M), st>>>(d);
+    } else {
       k_grid<R, I, KB, NT><<<dim3(d.J, d.E), NT, gsm, st>>>(d, c.ps_mode);
+    }
   }
   if (only < 0 || only == 1) {
     if constexpr (sizeof(R) == 4) {
@@ -1224,6 +1242,10 @@ template <typename R, int I> void set_attrs(const SD<R>& d) {
   } else {
     cudaFuncSetAttribute(k_grid<R, I, KB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)GridSmem<R, I, KB, NT>::bytes(d.M));
+    cudaFuncSetAttribute(k_ifft<R, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)GridFft<I>::template ifft_smem<R>(d.M));
+    cudaFuncSetAttribute(k_ffft<R, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)GridFft<I>::template ffft_smem<R>(d.M));
   }
   run_anal<R>(d, nullptr, true);
   if constexpr (sizeof(R) == 4) {
@@ -1384,18 +1406,18 @@ constexpr int NOALLOC_MAX_DEVICES = 64;
 static std::mutex g_noalloc_mu;
 static void* g_noalloc_base[NOALLOC_MAX_DEVICES];
 
-// Byte offsets of sf, sfs, af, afs, tend, tends (and in FP32 mode grid6,
-// grid9) in the scratch area, each rounded up to 256 bytes.  `need` is the
-// total, computed in double so that an absurd size cannot wrap around before
-// it is compared with the maximum.
-static void noalloc_layout(const lbm_stepper_desc& d, size_t off[8], double* need) {
+// Byte offsets of sf, sfs, af, afs, tend, tends (and with `rows` grid6, grid9)
+// in the scratch area, each rounded up to 256 bytes.  `need` is the total,
+// computed in double so that an absurd size cannot wrap around before it is
+// compared with the maximum.
+static void noalloc_layout(const lbm_stepper_desc& d, bool rows, size_t off[8], double* need) {
   const double c = 2.0 * (d.prec == LBM_F64 ? sizeof(double) : sizeof(float));
   const double E = d.nmem, M = d.nmax + 1.0, J = d.nlat, K = d.kmax, I = d.nlon;
   const double NS = M * (M + 1.0) / 2.0;
-  const double g = (d.prec == LBM_F32) ? 1.0 : 0.0;
+  const double r = rows ? 0.5 * c : 0.0;
   const double bytes[8] = {c * E * M * J * K * 6, c * E * M * J * 5, c * E * M * J * K * 7,
                            c * E * M * J * 2,     c * E * 4 * NS * K, c * E * 2 * NS,
-                           g * 4.0 * E * J * (6 + 6 * K) * I, g * 4.0 * E * J * (2 + 9 * K) * I};
+                           r * E * J * (6 + 6 * K) * I, r * E * J * (2 + 9 * K) * I};
   double t = 0.0;
   for (int i = 0; i < 8; ++i) {
     off[i] = (size_t)t;
@@ -1550,7 +1572,14 @@ int lbm_stepper_run_noalloc(const lbm_stepper_desc* d, const lbm_step_ctl* ctl, 
   if (d->nlon != 64 && d->nlon != 128 && d->nlon != 256) return LBM_ERR_ARG;
   size_t off[8];
   double need = 0.0;
-  noalloc_layout(*d, off, &need);
+  // FP32 needs the grid rows; FP64 takes them (the split grid part) where the
+  // scratch area has room, and runs k_grid otherwise
+  bool rows = true;
+  noalloc_layout(*d, rows, off, &need);
+  if (d->prec == LBM_F64 && need > (double)LBM_NOALLOC_SCRATCH_BYTES) {
+    rows = false;
+    noalloc_layout(*d, rows, off, &need);
+  }
   if (!(need > 0.0)) return LBM_ERR_ARG;
   if (need > (double)LBM_NOALLOC_SCRATCH_BYTES) return LBM_ERR_SCRATCH;
   for (int s = 0; s < nsteps; ++s)
@@ -1568,8 +1597,8 @@ int lbm_stepper_run_noalloc(const lbm_stepper_desc* d, const lbm_step_ctl* ctl, 
   w.afs = b + off[3];
   w.tend = b + off[4];
   w.tends = b + off[5];
-  w.grid6 = d->prec == LBM_F32 ? b + off[6] : nullptr;
-  w.grid9 = d->prec == LBM_F32 ? b + off[7] : nullptr;
+  w.grid6 = rows ? b + off[6] : nullptr;
+  w.grid9 = rows ? b + off[7] : nullptr;
   const size_t clear = (size_t)need;
   cudaStream_t st = (cudaStream_t)stream;
   return d->prec == LBM_F64 ? run_noalloc<double>(w, ctl, nsteps, clear, st)

@@ -134,6 +134,9 @@ class EnsembleStepper:
     #: keeps the T42L20 day-30 error at 6.3e-6 (with the Legendre
     #: contractions there too it reaches 1.1e-5, over the 1e-5 FP32 gate).
     TC_OFF = {"bf16x3": 3, "bf16split": 0}
+    #: largest FP64 grid-row workspace (20 MB per T42L20 member): bounds what
+    #: it adds to the 15 MB per member of the other buffers
+    GRID_ROWS_BYTES = 24 << 30
 
     def __init__(self, sp, vg, bst, damping, semi, vdiff, nmem, precision="fp64",
                  robert=0.04, strictly_linear=False, stream=None, tc_off=None):
@@ -230,9 +233,12 @@ class EnsembleStepper:
         # its plan applies (nlon <= 128, 9 kmax <= 256 rows)
         self.tc_dft = (tc_dft_image(N, I, dev) if self.legendre and I <= 128
                        and 9 * K <= 256 else None)
-        # FP32 grid rows between the longitude transforms and the column algebra
-        if precision != "fp64":
-            f = lambda *s_: torch.zeros(s_, device=dev, dtype=torch.float32)   # noqa: E731
+        # grid rows between the longitude transforms and the column algebra
+        # (FP64: up to GRID_ROWS_BYTES, else the one-kernel grid part, which
+        # keeps them in shared memory and is about three times slower)
+        rows = E * J * (8 + 15 * K) * I
+        if precision != "fp64" or 8 * rows <= self.GRID_ROWS_BYTES:
+            f = lambda *s_: torch.zeros(s_, device=dev, dtype=rd)   # noqa: E731
             self.grid6 = f(E, J, 6 + 6 * K, I)
             self.grid9 = f(E, J, 2 + 9 * K, I)
         else:
@@ -539,13 +545,14 @@ class EnsembleStepper:
         return spec, ps
 
     def launches_per_step(self):
-        """Kernel launches of one step (lbm_stepper_run): FP64 k_grid,
-        k_anal, k_implicit, k_synth; FP32 k_idft, k_alg, k_fdft, k_anal,
+        """Kernel launches of one step (lbm_stepper_run): FP64 k_ifft,
+        k_alg, k_ffft (without grid rows: k_grid), k_anal, k_implicit,
+        k_synth; FP32 k_idft, k_alg, k_fdft, k_anal,
         k_implicit, k_synth, where each contraction on the tensor cores is
         two launches (the tensor-core kernel and the surface fields' FMA
         kernel)."""
         if self.precision == "fp64":
-            return 4
+            return 6 if getattr(self, "grid6", None) is not None else 4
         n = 6
         if self.legendre:
             n += int(not (self.tc_off & 1)) + int(not (self.tc_off & 2))
