@@ -15,7 +15,7 @@ namespace lbm {
 struct FastDiv {
   unsigned m;
   int d;
-  LBM_D explicit FastDiv(int dv) : m((unsigned)((0x100000000ull + dv - 1) / dv)), d(dv) {}
+  LBM_D explicit FastDiv(int dv) : m(0xffffffffu / (unsigned)dv + 1u), d(dv) {}
   LBM_D int div(int x) const { return d == 1 ? x : (int)__umulhi((unsigned)x, m); }
 };
 

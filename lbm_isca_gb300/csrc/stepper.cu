@@ -29,6 +29,7 @@
 #include "lbm_common.cuh"
 #include "lbm_fft.cuh"
 #include "async_copy.cuh"
+#include "tc_common.cuh"
 #include <cmath>
 #include <mutex>
 #include <new>
@@ -363,217 +364,6 @@ __global__ void __launch_bounds__(NT) k_grid(SD<R> d, int ps_mode) {
 }
 
 // =============================================================================
-// Legendre analysis: af -> tend, per (member, m-pair, level chunk)
-// =============================================================================
-constexpr int AN_JC = 8;      // latitude pairs staged per pass
-
-template <typename R> struct PairRows {
-  int m1, m2, L1, L2, NR;
-  LBM_D PairRows(int p, int N) {
-    m1 = p;
-    m2 = N - p;
-    L1 = N + 1 - m1;
-    L2 = (m2 != m1) ? N + 1 - m2 : 0;
-    NR = L1 + L2;
-  }
-  LBM_D int m_of(int r) const { return r < L1 ? m1 : m2; }
-  LBM_D int n_of(int r) const { return r < L1 ? m1 + r : m2 + (r - L1); }
-};
-
-// Row groups of the analysis block: NC rows of an m-pair's N + 2 (at most
-// two partial groups).
-template <int NC> LBM_HD int anal_groups(int N) { return (N + 2 + NC - 1) / NC + 1; }
-
-// Members per block of the surface-only forms (one table staging serves them).
-constexpr int SURF_EB = 16;
-
-// SURF: only the surface part (tends), for the tensor-core analysis, which
-// computes the level part (k_anal_tc).
-template <typename R, int NC, int KC, bool SURF = false>
-__global__ void k_anal(SD<R> d) {
-  const int p = blockIdx.x, e = blockIdx.y, kc = blockIdx.z;
-  const int J = d.J, K = d.K, N = d.N, M = d.M, JH = J / 2;
-  const int k0 = kc * KC, kn = min(KC, K - k0);
-  const PairRows<R> pr(p, N);
-  const int G1 = (pr.L1 + NC - 1) / NC, G2 = (pr.L2 + NC - 1) / NC;
-  const int G = anal_groups<NC>(N);                    // row groups of the block
-  const int TS = NC * G + 1;                           // odd latitude stride of the tables
-  extern __shared__ unsigned char smraw[];
-  // P and H of the pair's rows as [JH][NC][G]: row rbase(g) + i at slot i G + g,
-  // so the row groups of a warp read adjacent words (no bank conflict)
-  R* tp = reinterpret_cast<R*>(smraw);
-  R* th = tp + (size_t)JH * TS;
-  // rows of AN_JC latitude pairs, two buffers, each
-  // [2 m][AN_JC][2 hemispheres][KC levels][7 fields] (16-byte aligned)
-  C2<R>* raw = reinterpret_cast<C2<R>*>(
-      (reinterpret_cast<uintptr_t>(th + (size_t)JH * TS) + 15) & ~uintptr_t(15));
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int off1 = spec_offset(pr.m1, N), off2 = spec_offset(pr.m2, N);
-  {
-    const FastDiv fjh(JH), fg(G);
-    for (int idx = tid; idx < NC * G * JH; idx += nt) {
-      const int sl = fjh.div(idx), jh = idx - sl * JH;     // latitude fastest
-      const int i = fg.div(sl), gg = sl - i * G;
-      int row = -1;
-      if (gg < G1) {
-        const int r = gg * NC + i;
-        if (r < pr.L1) row = off1 + r;
-      } else if (gg < G1 + G2) {
-        const int r = (gg - G1) * NC + i;
-        if (r < pr.L2) row = off2 + r;
-      }
-      tp[jh * TS + sl] = row >= 0 ? d.symp[(size_t)row * JH + jh] : R(0);
-      th[jh * TS + sl] = row >= 0 ? d.symh[(size_t)row * JH + jh] : R(0);
-    }
-  }
-  const int nm = pr.L2 ? 2 : 1;
-  if constexpr (!SURF) {
-  const int k = tid % KC, g = tid / KC;
-  const bool active = (k < kn) && (g < G1 + G2);
-  const int mi = (g < G1) ? 0 : 1;
-  const int rbase = (g < G1) ? g * NC : pr.L1 + (g - G1) * NC;
-  const int rend = (g < G1) ? pr.L1 : pr.NR;
-  C2<R> acc[NC][9];
-#pragma unroll
-  for (int i = 0; i < NC; ++i)
-#pragma unroll
-    for (int a = 0; a < 9; ++a) acc[i][a] = cmk<R>(0, 0);
-  const size_t jmK = (size_t)J * K;
-  const C2<R>* afe = d.af + (size_t)e * M * jmK * AF_N;
-  const int rowlen = kn * AF_N;                 // complex values per (m, latitude) row
-  const int rowst = KC * AF_N;                  // row stride in the buffer
-  const size_t rawbuf = (size_t)2 * AN_JC * 2 * rowst;
-  // 16-byte copies when every row starts and ends on a 16-byte boundary
-  constexpr int PER = 16 / (int)sizeof(C2<R>);
-  const bool wide = ((K * AF_N) % PER == 0) && ((k0 * AF_N) % PER == 0) &&
-                    (rowlen % PER == 0) && (rowst % PER == 0);
-  const int step = wide ? PER : 1;
-  const int nchunk = rowlen / step;
-  const FastDiv fch(nchunk);
-  auto prefetch = [&](int jh0, int b) {
-    const int jc = min(AN_JC, JH - jh0);
-    C2<R>* rb = raw + b * rawbuf;
-    // rows w = (mm AN_JC + jj) 2 + hemi; those with jj >= jc are skipped
-    for (int x = tid; x < nm * AN_JC * 2 * nchunk; x += nt) {
-      const int w = fch.div(x), c = (x - w * nchunk) * step;
-      const int hemi = w & 1, jj = (w >> 1) & (AN_JC - 1), mm = w / (2 * AN_JC);
-      if (jj >= jc) continue;
-      const int m = mm ? pr.m2 : pr.m1;
-      const int jn = jh0 + jj, j = hemi ? J - 1 - jn : jn;
-      C2<R>* dst = rb + ((mm * AN_JC + jj) * 2 + hemi) * rowst + c;
-      const C2<R>* src = afe + (((size_t)m * J + j) * K + k0) * AF_N + c;
-      if (wide) cp_async16(dst, src);
-      else cp_async_c2(dst, src);
-    }
-    cp_async_commit();
-  };
-  prefetch(0, 0);
-  int buf = 0;
-  for (int jh0 = 0; jh0 < JH; jh0 += AN_JC) {
-    const int jc = min(AN_JC, JH - jh0);
-    if (jh0 + AN_JC < JH) prefetch(jh0 + AN_JC, buf ^ 1);
-    else cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    if (active) {
-      const C2<R>* rb = raw + buf * rawbuf;
-      for (int jj = 0; jj < jc; ++jj) {
-        // north / south rows -> equatorially symmetric [0] and antisymmetric [1] parts
-        const C2<R>* xn = rb + ((mi * AN_JC + jj) * 2) * rowst + k * AF_N;
-        const C2<R>* xsth = xn + rowst;
-        C2<R> x[AF_N][2];
-#pragma unroll
-        for (int f = 0; f < AF_N; ++f) {
-          const C2<R> a = xn[f], b = xsth[f];
-          x[f][0] = a + b;
-          x[f][1] = a - b;
-        }
-        const int jh = jh0 + jj;
-#pragma unroll
-        for (int i = 0; i < NC; ++i) {
-          const int r = rbase + i;
-          if (r >= rend) break;
-          const R P = tp[jh * TS + i * G + g], H = th[jh * TS + i * G + g];
-          const int ps = (i & 1);          // parity of (n - m): rows alternate
-          const int hs = ps ^ 1;
-          cfma(acc[i][0], P, x[AF_FU][ps]);
-          cfma(acc[i][1], P, x[AF_FV][ps]);
-          cfma(acc[i][2], P, x[AF_KE][ps]);
-          cfma(acc[i][3], P, x[AF_T][ps]);
-          cfma(acc[i][4], P, x[AF_Q][ps]);
-          cfma(acc[i][5], H, x[AF_FU][hs]);
-          cfma(acc[i][6], H, x[AF_FV][hs]);
-          cfma(acc[i][7], H, x[AF_XV][hs]);
-          cfma(acc[i][8], H, x[AF_YV][hs]);
-        }
-      }
-    }
-    buf ^= 1;
-    __syncthreads();
-  }
-  if (active) {
-    const size_t NS = d.NS;
-#pragma unroll
-    for (int i = 0; i < NC; ++i) {
-      const int r = rbase + i;
-      if (r >= rend) break;
-      const int m = pr.m_of(r), n = pr.n_of(r);
-      const size_t idx = (size_t)spec_index(m, n, N);
-      const R rm = R(m);
-      const C2<R> vor = im_mul(acc[i][1], rm) + acc[i][5];
-      const C2<R> div = im_mul(acc[i][0], rm) - acc[i][6] + acc[i][2] * d.nn1a[n];
-      const C2<R> tt = acc[i][3] + acc[i][7];
-      const C2<R> qq = acc[i][4] + acc[i][8];
-      C2<R>* te = d.tend + (size_t)e * 4 * NS * K;
-      te[(0 * NS + idx) * K + k0 + k] = vor;
-      te[(1 * NS + idx) * K + k0 + k] = div;
-      te[(2 * NS + idx) * K + k0 + k] = tt;
-      te[(3 * NS + idx) * K + k0 + k] = qq;
-    }
-  }
-  }  // !SURF
-  // surface: wt_pi and pi(t - dt), one thread per row (first level chunk
-  // only; the surface-only form takes SURF_EB members per block)
-  auto surface = [&](int e) {
-  __syncthreads();
-  C2<R>* ss = raw;                                   // [2][JH][2 fields][2]
-  for (int idx = tid; idx < nm * JH * 2; idx += nt) {
-    const int f = idx % 2, jh = (idx / 2) % JH, mm = idx / (2 * JH);
-    const int m = mm ? pr.m2 : pr.m1;
-    const C2<R> xn = d.afs[(((size_t)e * M + m) * J + jh) * 2 + f];
-    const C2<R> xsouth = d.afs[(((size_t)e * M + m) * J + (J - 1 - jh)) * 2 + f];
-    C2<R>* dst = ss + ((mm * JH + jh) * 2 + f) * 2;
-    dst[0] = xn + xsouth;
-    dst[1] = xn - xsouth;
-  }
-  __syncthreads();
-  for (int r = tid; r < pr.NR; r += nt) {
-    const int m = pr.m_of(r), n = pr.n_of(r), mm = r < pr.L1 ? 0 : 1;
-    const int par = (n - m) & 1;
-    C2<R> a0 = cmk<R>(0, 0), a1 = cmk<R>(0, 0);
-    const int rr = r < pr.L1 ? r : r - pr.L1;
-    const int sl = (rr % NC) * G + (r < pr.L1 ? 0 : G1) + rr / NC;   // table slot of row r
-    for (int jh = 0; jh < JH; ++jh) {
-      const R P = tp[jh * TS + sl];
-      const C2<R>* x = ss + ((mm * JH + jh) * 2) * 2;
-      cfma(a0, P, x[0 * 2 + par]);
-      cfma(a1, P, x[1 * 2 + par]);
-    }
-    const size_t idx = (size_t)spec_index(m, n, N);
-    d.tends[((size_t)e * 2 + 0) * d.NS + idx] = a0;
-    d.tends[((size_t)e * 2 + 1) * d.NS + idx] = a1;
-  }
-  };
-  if constexpr (SURF) {
-    const int e1 = min(d.E, (int)(blockIdx.y + 1) * SURF_EB);
-    for (int ee = blockIdx.y * SURF_EB; ee < e1; ++ee) surface(ee);
-  } else {
-    if (kc != 0) return;
-    surface(e);
-  }
-}
-
-// =============================================================================
 // Implicit spectral update, per (member, n-pair)
 // =============================================================================
 constexpr int IM_THREADS = 256;
@@ -795,221 +585,6 @@ __global__ void k_colsum(SD<R> d) {
   d.sas[es + 3 * NS + idx] = sdv;
 }
 
-// Two adjacent complex values in one store (16 bytes in FP32; the six-field
-// rows of sf start on 16-byte boundaries).
-LBM_D void store_pair(C2<float>* o, C2<float> a, C2<float> b) {
-  *reinterpret_cast<float4*>(o) = make_float4(a.x, a.y, b.x, b.y);
-}
-LBM_D void store_pair(C2<double>* o, C2<double> a, C2<double> b) {
-  o[0] = a;
-  o[1] = b;
-}
-
-// =============================================================================
-// Legendre synthesis: state A -> sf, sfs, per (member, m-pair, level chunk)
-// =============================================================================
-constexpr int SY_THREADS = 320;
-
-// SURF: only the surface fields (sfs), for the tensor-core synthesis, which
-// computes the level fields (k_synth_tc).
-template <typename R, int JG, int KC, int HV, bool SURF = false>
-__global__ void __launch_bounds__(SY_THREADS, 2) k_synth(SD<R> d) {
-  const int p = blockIdx.x, e = blockIdx.y, kc = blockIdx.z;
-  const int J = d.J, K = d.K, N = d.N, M = d.M, JH = J / 2, NS = d.NS;
-  const int k0 = kc * KC, kn = min(KC, K - k0);
-  const PairRows<R> pr(p, N);
-  extern __shared__ unsigned char smraw[];
-  R* tp = reinterpret_cast<R*>(smraw);                 // [NR][JH]
-  R* th = tp + pr.NR * JH;
-  C2<R>* sv = reinterpret_cast<C2<R>*>(th + pr.NR * JH);    // [NR][6][KC]
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int off1 = spec_offset(pr.m1, N), off2 = spec_offset(pr.m2, N);
-  for (int idx = tid; idx < pr.NR * JH; idx += nt) {
-    const int r = idx / JH, jh = idx % JH;
-    const int row = r < pr.L1 ? off1 + r : off2 + (r - pr.L1);
-    tp[idx] = d.symp[(size_t)row * JH + jh];
-    th[idx] = d.symh[(size_t)row * JH + jh];
-  }
-  const int nm = pr.L2 ? 2 : 1;
-  if constexpr (!SURF) {
-  const size_t e3 = (size_t)e * 4 * NS * K;
-  for (int idx = tid; idx < pr.NR * kn; idx += nt) {
-    const int r = idx / kn, kk = idx % kn;
-    const int n = pr.n_of(r);
-    const int row = r < pr.L1 ? off1 + r : off2 + (r - pr.L1);
-    const size_t o = (size_t)row * K + k0 + kk;
-    const C2<R> vo = d.sa3[e3 + 0 * (size_t)NS * K + o], dv = d.sa3[e3 + 1 * (size_t)NS * K + o];
-    const R il = d.invlap[n];
-    C2<R>* s = sv + (size_t)r * 6 * KC + kk;         // field f at s[f * KC]
-    s[0 * KC] = vo * il;                               // psi
-    s[1 * KC] = dv * il;                               // chi
-    s[2 * KC] = vo;
-    s[3 * KC] = dv;
-    s[4 * KC] = d.sa3[e3 + 2 * (size_t)NS * K + o];
-    s[5 * KC] = d.sa3[e3 + 3 * (size_t)NS * K + o];
-  }
-  __syncthreads();
-  const int NJG = (JH + JG - 1) / JG;
-  const size_t jmK = (size_t)J * K;
-  C2<R>* sfe = d.sf + (size_t)e * M * jmK * SF_N;
-  // Items: (term half, latitude group, level), level fastest.  With HV = 2
-  // the first NJG KC items take the wind terms (P chi, H psi, P psi, H chi ->
-  // U, V), the rest the scalar terms (P vor, P div, P T, P q): each value read
-  // from shared memory then feeds JG latitudes of four terms, and the halves
-  // are whole warps apart.  HV = 1: every item takes all eight terms.  Every
-  // item walks the N + 2 rows of both m of the pair, so the pair's rows are
-  // balanced across threads.
-  const int nhalf = NJG * KC;
-  for (int it = tid; it < HV * nhalf; it += nt) {
-    const int half = HV == 2 ? (it >= nhalf ? 1 : 0) : -1;
-    const int ri = it - (half > 0 ? nhalf : 0);
-    const int kk = ri % KC;
-    const int jg = ri / KC;
-    if (kk >= kn) continue;
-   for (int mm = 0; mm < nm; ++mm) {
-    const int m = mm ? pr.m2 : pr.m1;
-    const int rb = mm ? pr.L1 : 0, re = mm ? pr.NR : pr.L1;
-    const R rm = R(m);
-    // rows alternate parity of (n - m), starting even; P of an even row is
-    // symmetric about the equator (plus), H of an even row antisymmetric.
-    // acc[jg][term][plus/minus]
-    auto wind = [&]() {
-      C2<R> acc[JG][4][2];
-#pragma unroll
-      for (int a = 0; a < JG; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = cmk<R>(0, 0);
-      auto row = [&](int r, auto par_tag) {
-        constexpr int PP = decltype(par_tag)::value, HP = PP ^ 1;
-        const C2<R>* sr = sv + r * 6 * KC + kk;
-        const C2<R> psi = sr[0 * KC], chi = sr[1 * KC];
-#pragma unroll
-        for (int a = 0; a < JG; ++a) {
-          const int jh = min(jg * JG + a, JH - 1);
-          const R P = tp[r * JH + jh], H = th[r * JH + jh];
-          cfma(acc[a][0][PP], P, chi);
-          cfma(acc[a][1][HP], H, psi);
-          cfma(acc[a][2][PP], P, psi);
-          cfma(acc[a][3][HP], H, chi);
-        }
-      };
-      for (int r = rb; r < re; r += 2) {
-        row(r, std::integral_constant<int, 0>{});
-        if (r + 1 < re) row(r + 1, std::integral_constant<int, 1>{});
-      }
-#pragma unroll
-      for (int a = 0; a < JG; ++a) {
-        const int jh = jg * JG + a;
-        if (jh >= JH) break;
-#pragma unroll
-        for (int hemi = 0; hemi < 2; ++hemi) {
-          const int j = hemi ? J - 1 - jh : jh;
-          const R sg = hemi ? R(-1) : R(1);
-          auto comb = [&](int b) { return acc[a][b][0] + acc[a][b][1] * sg; };
-          C2<R>* o = sfe + (((size_t)m * J + j) * K + k0 + kk) * SF_N;
-          store_pair(o + SF_U, im_mul(comb(0), rm) - comb(1), im_mul(comb(2), rm) + comb(3));
-        }
-      }
-    };
-    auto scalars = [&]() {
-      C2<R> acc[JG][4][2];
-#pragma unroll
-      for (int a = 0; a < JG; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = cmk<R>(0, 0);
-      auto row = [&](int r, auto par_tag) {
-        constexpr int PP = decltype(par_tag)::value;
-        const C2<R>* sr = sv + r * 6 * KC + kk;
-        const C2<R> vo = sr[2 * KC], dv = sr[3 * KC], tt = sr[4 * KC], qq = sr[5 * KC];
-#pragma unroll
-        for (int a = 0; a < JG; ++a) {
-          const int jh = min(jg * JG + a, JH - 1);
-          const R P = tp[r * JH + jh];
-          cfma(acc[a][0][PP], P, vo);
-          cfma(acc[a][1][PP], P, dv);
-          cfma(acc[a][2][PP], P, tt);
-          cfma(acc[a][3][PP], P, qq);
-        }
-      };
-      for (int r = rb; r < re; r += 2) {
-        row(r, std::integral_constant<int, 0>{});
-        if (r + 1 < re) row(r + 1, std::integral_constant<int, 1>{});
-      }
-#pragma unroll
-      for (int a = 0; a < JG; ++a) {
-        const int jh = jg * JG + a;
-        if (jh >= JH) break;
-#pragma unroll
-        for (int hemi = 0; hemi < 2; ++hemi) {
-          const int j = hemi ? J - 1 - jh : jh;
-          const R sg = hemi ? R(-1) : R(1);
-          auto comb = [&](int b) { return acc[a][b][0] + acc[a][b][1] * sg; };
-          C2<R>* o = sfe + (((size_t)m * J + j) * K + k0 + kk) * SF_N;
-          store_pair(o + SF_VOR, comb(0), comb(1));
-          store_pair(o + SF_T, comb(2), comb(3));
-        }
-      }
-    };
-    if (half <= 0) wind();
-    if (half != 0) scalars();
-   }
-  }
-  }  // !SURF
-  // surface fields (first level chunk only; the surface-only form takes
-  // SURF_EB members per block)
-  if constexpr (SURF) __syncthreads();
-  auto surface = [&](int e) {
-  const size_t es = (size_t)e * 4 * NS;
-  for (int it = tid; it < nm * JH; it += nt) {
-    const int jh = it % JH, mm = it / JH;
-    const int m = mm ? pr.m2 : pr.m1;
-    const int rb = mm ? pr.L1 : 0, re = mm ? pr.NR : pr.L1;
-    const int offm = mm ? off2 : off1;
-    // terms: Ppi Hpi Pchis Hpsis Ppsis Hchis Pds  [plus/minus]
-    C2<R> acc[7][2];
-#pragma unroll
-    for (int b = 0; b < 7; ++b) acc[b][0] = acc[b][1] = cmk<R>(0, 0);
-    auto row = [&](int r, auto par_tag) {
-      constexpr int PP = decltype(par_tag)::value, HP = PP ^ 1;
-      const size_t rowi = (size_t)offm + (r - rb);
-      const C2<R> pi = d.sas[es + 0 * NS + rowi], psis = d.sas[es + 1 * NS + rowi];
-      const C2<R> chis = d.sas[es + 2 * NS + rowi], ds = d.sas[es + 3 * NS + rowi];
-      const R P = tp[r * JH + jh], H = th[r * JH + jh];
-      cfma(acc[0][PP], P, pi);
-      cfma(acc[1][HP], H, pi);
-      cfma(acc[2][PP], P, chis);
-      cfma(acc[3][HP], H, psis);
-      cfma(acc[4][PP], P, psis);
-      cfma(acc[5][HP], H, chis);
-      cfma(acc[6][PP], P, ds);
-    };
-    for (int r = rb; r < re; r += 2) {
-      row(r, std::integral_constant<int, 0>{});
-      if (r + 1 < re) row(r + 1, std::integral_constant<int, 1>{});
-    }
-    const R rm = R(m);
-    for (int hemi = 0; hemi < 2; ++hemi) {
-      const int j = hemi ? J - 1 - jh : jh;
-      const R sg = hemi ? R(-1) : R(1);
-      auto comb = [&](int b) { return acc[b][0] + acc[b][1] * sg; };
-      C2<R>* o = d.sfs + (((size_t)e * M + m) * J + j) * SFS_N;
-      o[SFS_PI] = comb(0);
-      o[SFS_PIY] = comb(1);
-      o[SFS_UH] = im_mul(comb(2), rm) - comb(3);
-      o[SFS_VH] = im_mul(comb(4), rm) + comb(5);
-      o[SFS_DH] = comb(6);
-    }
-  }
-  };
-  if constexpr (SURF) {
-    const int e1 = min(d.E, (int)(blockIdx.y + 1) * SURF_EB);
-    for (int ee = blockIdx.y * SURF_EB; ee < e1; ++ee) surface(ee);
-  } else {
-    if (kc != 0) return;
-    surface(e);
-  }
-}
-
 // Apply the pending grid-ps update at the end of a run (see k_grid).
 template <typename R, int I>
 __global__ void k_ps_flush(SD<R> d, int ps_mode) {
@@ -1042,6 +617,7 @@ __global__ void k_ps_flush(SD<R> d, int ps_mode) {
 }
 
 }  // namespace lbm
+#include "legendre_fma.cuh"
 #include "grid_split.cuh"
 #include "grid_fft.cuh"
 #include "legendre_tc.cuh"
@@ -1050,14 +626,6 @@ __global__ void k_ps_flush(SD<R> d, int ps_mode) {
 namespace lbm {
 
 // ---- launch configuration ------------------------------------------------------
-template <typename R> struct Cfg;
-template <> struct Cfg<float> {
-  static constexpr int NC = 4, KCA = 20, JG = 4, KCS = 20, SHV = 2;
-};
-template <> struct Cfg<double> {
-  static constexpr int NC = 2, KCA = 10, JG = 1, KCS = 10, SHV = 1;
-};
-
 // Resident k_alg blocks of I threads (see the kernel).
 template <int I> constexpr int alg_minb() { return I == 64 ? 10 : (I == 128 ? 6 : 3); }
 
@@ -1066,66 +634,31 @@ template <typename R, int I> constexpr int grid_nt() {
   return I == 64 ? 128 : ((I == 256 && sizeof(R) == 8) ? 128 : 256);
 }
 
-template <typename R> size_t anal_smem(int N, int JH, int KC) {
-  constexpr int NC = Cfg<R>::NC;
-  const size_t TS = (size_t)NC * anal_groups<NC>(N) + 1;
-  return sizeof(R) * 2 * TS * JH + 16 + sizeof(C2<R>) * (size_t)2 * (2 * AN_JC * 2 * AF_N * KC);
-}
-// Level chunk of the analysis block (one thread per level and row group): the
-// preferred Cfg<R>::KCA, halved where that block would exceed 256 threads.
-template <typename R> int anal_kc(int N) {
-  constexpr int NC = Cfg<R>::NC;
-  const int G = anal_groups<NC>(N);
-  return (Cfg<R>::KCA * G > 256) ? Cfg<R>::KCA / 2 : Cfg<R>::KCA;
-}
-template <typename R, int KC> void launch_anal(const SD<R>& d, cudaStream_t st, bool attrs) {
-  constexpr int NC = Cfg<R>::NC;
-  const int JH = d.J / 2, NRmax = d.N + 2, NP = (d.M + 1) / 2;
-  const int G = anal_groups<NC>(d.N);
-  const int nt = ((KC * G + 31) / 32) * 32;
-  // the surface pass also needs 2 * JH * 2 staging elements
-  size_t sm = anal_smem<R>(d.N, JH, KC);
-  const size_t sm2 = sizeof(R) * 2 * ((size_t)NC * G + 1) * JH + 16 +
-                     sizeof(C2<R>) * (size_t)2 * JH * 2 * 2;
-  if (sm2 > sm) sm = sm2;
-  if (attrs) {
-    cudaFuncSetAttribute(k_anal<R, NC, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaFuncSetAttribute(k_anal<R, NC, KC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sm);
-  } else if (d.legendre && !(d.tc_off & 1) && sizeof(R) == 4) {
-    k_anal<R, NC, KC, true><<<dim3(NP, (d.E + SURF_EB - 1) / SURF_EB, 1), nt, sm, st>>>(d);
-  } else {
-    k_anal<R, NC, KC><<<dim3(NP, d.E, (d.K + KC - 1) / KC), nt, sm, st>>>(d);
-  }
-}
-template <typename R> void run_anal(const SD<R>& d, cudaStream_t st, bool attrs) {
-  if (anal_kc<R>(d.N) == Cfg<R>::KCA) launch_anal<R, Cfg<R>::KCA>(d, st, attrs);
-  else launch_anal<R, Cfg<R>::KCA / 2>(d, st, attrs);
-}
 inline int persistent_grid(const void* fn, int nt, size_t smem, int units);
-template <typename R> size_t synth_smem(int NR, int JH) {
-  return sizeof(R) * 2 * (size_t)NR * JH + sizeof(C2<R>) * (size_t)NR * Cfg<R>::KCS * 6;
-}
-// Legendre synthesis launch: HV NJG KC items, at most SY_THREADS threads.
-template <typename R> void launch_synth(const SD<R>& d, cudaStream_t st) {
-  constexpr int JG = Cfg<R>::JG, KC = Cfg<R>::KCS, HV = Cfg<R>::SHV;
-  const int JH = d.J / 2, NRmax = d.N + 2, NP = (d.M + 1) / 2;
-  const int NJG = (JH + JG - 1) / JG;
-  int nt = HV * NJG * KC;
-  nt = nt > SY_THREADS ? SY_THREADS : ((nt + 31) / 32) * 32;
+// Legendre synthesis launch; with the level fields on the tensor cores a second
+// kernel makes the surface fields.
+template <typename R> void launch_synth(const SD<R>& d, cudaStream_t st, bool attrs) {
+  const SynthPlan sp = synth_plan<R>(d.E, d.J, d.K, d.N);
+  const int NP = (d.M + 1) / 2;
   if constexpr (sizeof(R) == 4) {
     if (d.legendre && !(d.tc_off & 2)) {
-      // level fields on the tensor cores, surface fields by the FMA kernel
       const StcPlan pl = stc_plan(d.E, d.J, d.K, d.N, d.tc_g);
+      const int sm = sp.ox + (int)sizeof(C2<R>) * 4 * (d.N + 2);
+      if (attrs) {
+        cudaFuncSetAttribute(k_synth_surf, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        return;
+      }
       k_synth_tc<<<persistent_grid((const void*)k_synth_tc, STC_THREADS, pl.smem, pl.nunits),
                    STC_THREADS, pl.smem, st>>>(d, d.tc_synth, pl, d.legendre);
-      k_synth<R, JG, KC, HV, true><<<dim3(NP, (d.E + SURF_EB - 1) / SURF_EB, 1), nt,
-                                       synth_smem<R>(NRmax, JH), st>>>(d);
+      const int eb = members_per_block(d.E, NP);
+      k_synth_surf<<<dim3(NP, (d.E + eb - 1) / eb), 128, sm, st>>>(d, sp, eb);
       return;
     }
   }
-  k_synth<R, JG, KC, HV><<<dim3(NP, d.E, (d.K + KC - 1) / KC), nt, synth_smem<R>(NRmax, JH),
-                           st>>>(d);
+  if (attrs)
+    cudaFuncSetAttribute(k_synth<R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp.smem);
+  else
+    k_synth<R, 2><<<dim3(NP, (d.E + sp.eb - 1) / sp.eb, sp.nch + 1), sp.nt, sp.smem, st>>>(d, sp);
 }
 template <typename R> size_t impl_smem(int K) {
   return sizeof(R) * ((size_t)(2 + 4) * K * K + 7 * (size_t)K + (K & 1)) +
@@ -1212,12 +745,20 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
                     ATC_THREADS, pl.smem, st>>>(d, d.tc_anal, pl, d.legendre);
       }
     }
-    run_anal<R>(d, st, false);
+    bool level = true;
+    if constexpr (sizeof(R) == 4) {
+      if (d.legendre && !(d.tc_off & 1)) {
+        const int eb = members_per_block(d.E, NP);
+        k_anal_surf<<<dim3(NP, (d.E + eb - 1) / eb), 128, anal_surf_smem(d.J, d.N), st>>>(d, eb);
+        level = false;
+      }
+    }
+    if (level) launch_anal<R>(d, st, false);
   }
   if (only < 0 || only == 2)
     k_implicit<R><<<dim3(NP, d.E), IM_THREADS, impl_smem<R>(d.K), st>>>(d, R(c.dt), c.set,
                                                                          c.ra_mode);
-  if (only < 0 || only == 3) launch_synth<R>(d, st);
+  if (only < 0 || only == 3) launch_synth<R>(d, st, false);
   LBM_LAUNCH_CHECK();
   return LBM_OK;
 }
@@ -1247,22 +788,19 @@ template <typename R, int I> void set_attrs(const SD<R>& d) {
     cudaFuncSetAttribute(k_ffft<R, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)GridFft<I>::template ffft_smem<R>(d.M));
   }
-  run_anal<R>(d, nullptr, true);
+  launch_anal<R>(d, nullptr, true);
+  launch_synth<R>(d, nullptr, true);
   if constexpr (sizeof(R) == 4) {
     if (d.legendre) {
       const AtcPlan pl = atc_plan(d.E, d.J, d.K, d.N, d.tc_g);
       cudaFuncSetAttribute(k_anal_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+      cudaFuncSetAttribute(k_anal_surf, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)anal_surf_smem(d.J, d.N));
       persistent_grid((const void*)k_anal_tc, ATC_THREADS, pl.smem, 1);
     }
   }
   cudaFuncSetAttribute(k_implicit<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)impl_smem<R>(d.K));
-  cudaFuncSetAttribute(k_synth<R, Cfg<R>::JG, Cfg<R>::KCS, Cfg<R>::SHV>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)synth_smem<R>(NRmax, JH));
-  cudaFuncSetAttribute(k_synth<R, Cfg<R>::JG, Cfg<R>::KCS, Cfg<R>::SHV, true>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)synth_smem<R>(NRmax, JH));
   if constexpr (sizeof(R) == 4) {
     if (d.legendre) {
       const StcPlan pl = stc_plan(d.E, d.J, d.K, d.N, d.tc_g);
@@ -1343,19 +881,6 @@ template <typename R> int prepare_attrs(const lbm_stepper_desc* desc) {
   const SD<R> d = make_sd<R>(*desc);
   int rc = validate(d);
   if (rc) return rc;
-  {
-    // the analysis block holds one thread per (level, row group) of an m-pair
-    constexpr int NC = Cfg<R>::NC;
-    const int KC = anal_kc<R>(d.N);
-    const int G = anal_groups<NC>(d.N);
-    const int nt = ((KC * G + 31) / 32) * 32;
-    cudaFuncAttributes fa;
-    const cudaError_t ea = (KC == Cfg<R>::KCA)
-                               ? cudaFuncGetAttributes(&fa, k_anal<R, NC, Cfg<R>::KCA>)
-                               : cudaFuncGetAttributes(&fa, k_anal<R, NC, Cfg<R>::KCA / 2>);
-    if (ea != cudaSuccess) return LBM_ERR_LAUNCH;
-    if (nt > fa.maxThreadsPerBlock) return LBM_ERR_ARG;
-  }
   switch (d.I) {
     case 64: set_attrs<R, 64>(d); break;
     case 128: set_attrs<R, 128>(d); break;
@@ -1368,7 +893,7 @@ template <typename R> int prime(const lbm_stepper_desc* desc, cudaStream_t st) {
   const SD<R> d = make_sd<R>(*desc);
   int rc = validate(d);
   if (rc) return rc;
-  launch_synth<R>(d, st);
+  launch_synth<R>(d, st, false);
   LBM_LAUNCH_CHECK();
   return LBM_OK;
 }

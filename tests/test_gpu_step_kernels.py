@@ -57,6 +57,7 @@ def _stepper(torch, grid, K, nmem, precision, **kw):
 def _launch(torch, stp, kernel, desc=None, ps_mode=0):
     from lbm_isca_gb300._lib import check, lib
     ctl = stp._ctl([(stp._dts[0], False, ps_mode)])
+    torch.cuda.synchronize()          # the test writes its inputs on another stream
     check(lib().lbm_stepper_launch(C.byref(stp.desc() if desc is None else desc), ctl, kernel,
                                    C.c_void_p(stp.stream.cuda_stream)), "launch")
     torch.cuda.synchronize()
@@ -92,3 +93,132 @@ def test_fp64_split_grid_part_equals_the_one_kernel_form(torch, grid, K, nmem, p
     for f in range(2):
         assert _rel(got[1][..., f], stp.afs[..., f]) < 1e-11
     assert _rel(got[2], stp.psa) < 1e-12 and _rel(got[3], stp.psb) < 1e-12
+
+
+def _grid_stepper(torch, I, J, N, K, nmem, precision):
+    """Stepper on any grid (its arrays only: the state is set by the test)."""
+    from lbm_isca_gb300 import Config
+    from lbm_isca_gb300.ensemble import make_ensemble_model
+    sigm = configs.equal_sigma_half_levels(K)
+    cfg = dict(configs.plain_damping(max(K, 2)), ddragv=None, ddragd=None, ddragt=None)
+    m, _, _ = make_ensemble_model(configs.solid_body_basic_state(I, J, sigm), nmem,
+                                  Config(precision=precision, **cfg),
+                                  device="gb300", nlon=I, nlat=J, nmax=N, sigm=sigm)
+    stp = m.stepper()
+    stp.set_timesteps([600.0])
+    stp.load_zero()
+    torch.cuda.synchronize()
+    return stp
+
+
+def _full_tables(torch, stp):
+    """P, H [m][n][j] in FP64 from the stepper's northern, working-precision rows."""
+    M, JH = stp.M, stp.J // 2
+    sign = torch.where((stp.pn - stp.pm) % 2 == 0, 1.0, -1.0).double()[:, None]
+    out = []
+    for t, s in ((stp.symp.double(), sign), (stp.symh.double(), -sign)):
+        T = torch.zeros((M, M, stp.J), device=t.device, dtype=torch.float64)
+        T[stp.pm, stp.pn, :JH] = t
+        T[stp.pm, stp.pn, JH:] = (s * t).flip(1)
+        out.append(T)
+    return out
+
+
+def _noise(torch, like, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(tuple(like.shape) + (2,), generator=g, device="cuda", dtype=torch.float64)
+    like.copy_(torch.view_as_complex(x).to(like.dtype))
+
+
+SHAPES = [  # I, J, N, K, members: odd level counts, one level, J/2 odd, N odd and even,
+            # level chunks with remainders, one and many members, units beyond the SMs
+    (64, 32, 21, 1, 1), (64, 32, 21, 20, 1), (64, 30, 19, 5, 3), (64, 32, 21, 40, 9),
+    (128, 64, 42, 17, 2), (128, 64, 42, 20, 13), (128, 50, 31, 2, 1), (256, 128, 85, 9, 2),
+    (256, 128, 85, 40, 1), (64, 6, 3, 7, 40)]
+
+
+@pytest.mark.parametrize("I,J,N,K,nmem", SHAPES)
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_legendre_kernels_against_fp64_sums(torch, I, J, N, K, nmem, precision):
+    """k_anal and k_synth against plain FP64 contractions of the same working-
+    precision tables and rows.  Bound per value: the rounding of a sum of n <= 2 J
+    products (and the three or four operations around it), (n + 8) u times the
+    sum of the products' magnitudes, u the unit roundoff, plus gradual underflow:
+    half the least subnormal per operation, times m (near the poles P and H of
+    large m fall below the least normal number)."""
+    stp = _grid_stepper(torch, I, J, N, K, nmem, precision)
+    u, tiny = (2.0 ** -24, 2.0 ** -150) if precision == "fp32" else (2.0 ** -53, 1e-300)
+    P, H = _full_tables(torch, stp)
+    m = torch.arange(stp.M, device="cuda", dtype=torch.float64)
+    im = (1j * m)[None, :, None, None]
+    pm, pn = stp.pm, stp.pn
+
+    def mul(eq, T, X):
+        return torch.complex(torch.einsum(eq, T, X.real.contiguous()),
+                             torch.einsum(eq, T, X.imag.contiguous()))
+
+    def check(got, want, size, terms):
+        # size: sum of magnitudes, the largest of its (Re, Im) parts
+        err = torch.view_as_real(got.to(torch.complex128) - want).abs().amax(-1)
+        lim = (terms + 8) * (u * size + (1.0 + N) * tiny)
+        assert bool((err <= lim).all()), float((err / lim).max())
+
+    # ---- analysis
+    _noise(torch, stp.af, 1)
+    _noise(torch, stp.afs, 2)
+    for t in (stp.tend, stp.tends):
+        t.zero_()
+    _launch(torch, stp, 1)
+    af = stp.af.to(torch.complex128)                    # [E][M][J][K][7]
+    ab = af.abs()
+    fu, fv, ke, t, xv, q, yv = af.unbind(-1)
+    afu, afv, ake, at, axv, aq, ayv = ab.unbind(-1)
+    A = lambda T, X: mul("mnj,emjk->emnk", T, X)         # noqa: E731
+    B = lambda T, X: torch.einsum("mnj,emjk->emnk", T.abs(), X)     # noqa: E731
+    nn = stp.nn1a.double()[None, None, :, None]
+    mm = m[None, :, None, None]
+    want = [im * A(P, fv) + A(H, fu), im * A(P, fu) - A(H, fv) + nn * A(P, ke),
+            A(P, t) + A(H, xv), A(P, q) + A(H, yv)]
+    size = [mm * B(P, afv) + B(H, afu), mm * B(P, afu) + B(H, afv) + nn * B(P, ake),
+            B(P, at) + B(H, axv), B(P, aq) + B(H, ayv)]
+    for f in range(4):
+        check(stp.tend[:, f], want[f][:, pm, pn], size[f][:, pm, pn], J)
+    for f in range(2):
+        X = stp.afs.to(torch.complex128)[..., f]
+        check(stp.tends[:, f], mul("mnj,emj->emn", P, X)[:, pm, pn],
+              torch.einsum("mnj,emj->emn", P.abs(), X.abs())[:, pm, pn], J)
+
+    # ---- synthesis
+    _noise(torch, stp.sa3, 3)
+    _noise(torch, stp.sas, 4)
+    for t in (stp.sf, stp.sfs):
+        t.zero_()
+    _launch(torch, stp, 3)
+
+    def rect(x):                                         # [E][NS] + tail -> [E][M][M] + tail
+        r = torch.zeros((nmem, stp.M, stp.M) + tuple(x.shape[2:]), device="cuda",
+                        dtype=torch.complex128)
+        r[:, pm, pn] = x.to(torch.complex128)
+        return r
+
+    S = lambda T, X: mul("mnj,emnk->emjk", T, X)         # noqa: E731
+    Q = lambda T, X: torch.einsum("mnj,emnk->emjk", T.abs(), X.abs())   # noqa: E731
+    il = stp.invlap.double()[None, None, :, None]
+
+    def winds(psi, chi):
+        return ([im * S(P, chi) - S(H, psi), im * S(P, psi) + S(H, chi)],
+                [mm * Q(P, chi) + Q(H, psi), mm * Q(P, psi) + Q(H, chi)])
+
+    vo, dv, tt, qq = (rect(stp.sa3[:, f]) for f in range(4))
+    w, wz = winds(vo * il, dv * il)
+    want = w + [S(P, x) for x in (vo, dv, tt, qq)]
+    size = wz + [Q(P, x) for x in (vo, dv, tt, qq)]
+    for f in range(6):
+        check(stp.sf[..., f], want[f], size[f], N + 1)
+    pi, psi, chi, ds = (rect(stp.sas[:, f])[..., None] for f in range(4))
+    w, wz = winds(psi, chi)
+    want = [S(P, pi), S(H, pi)] + w + [S(P, ds)]
+    size = [Q(P, pi), Q(H, pi)] + wz + [Q(P, ds)]
+    for f in range(5):
+        check(stp.sfs[..., f], want[f][..., 0], size[f][..., 0], N + 1)
+    assert int(stp.err.item()) == 0
