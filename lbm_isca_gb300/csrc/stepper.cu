@@ -363,205 +363,6 @@ __global__ void __launch_bounds__(NT) k_grid(SD<R> d, int ps_mode) {
   }
 }
 
-// =============================================================================
-// Implicit spectral update, per (member, n-pair)
-// =============================================================================
-constexpr int IM_THREADS = 256;
-
-// The semi-implicit update in the order of integrator.py:264-315.  Three
-// places subtract nearly equal quantities, and the FP32 mode carries them in
-// float-float (XF) so that the difference keeps FP32 relative precision:
-// the divergence right-hand side (explicit tendency against the Laplacian of
-// the geopotential), the temperature update (heating against the
-// reference-temperature matrix on the mean divergence) and the pi update
-// (against the column-integrated divergence).  WW and tmtx enter through
-// their level-scan forms
-//   (WW x)_k   = R alpha_k x_k + sum_{l<k} R dlog3_l x_l,
-//   (tmtx D)_k = kappa Tref_k (alpha_k D_k + w3_k sum_{l>k} dsig_l D_l),
-// each level summing its own prefix / suffix.  Damping factors 1 / (1 + c)
-// are applied as x - x c / (1 + c) so that a small c keeps its precision.
-template <typename R>
-__global__ void __launch_bounds__(IM_THREADS) k_implicit(SD<R> d, R dt, int set, int ra_mode) {
-  const int p = blockIdx.x, e = blockIdx.y;
-  const int K = d.K, N = d.N, NS = d.NS;
-  const int n1 = p, n2 = N - p;
-  const int C1 = n1 + 1, C2n = (n2 != n1) ? n2 + 1 : 0;
-  const int ncoef = C1 + C2n;
-  const int CC = IM_THREADS / K;               // coefficients per chunk
-  extern __shared__ unsigned char smraw[];
-  R* mi = reinterpret_cast<R*>(smraw);          // [2][K][K] minv^T (l, k)
-  R* vdT = mi + 2 * K * K;                      // [4][K][K] (vdiff - I)^T (l, k)
-  R* vs = vdT + 4 * K * K;                      // [6][K] RALPHA RDLOG3 GG DSIG ALPHA W3
-  R* ktr = vs + 6 * K;                          // [K] KTREF
-  C2<R>* bA = reinterpret_cast<C2<R>*>(ktr + K + (K & 1));  // [CC][K]
-  C2<R>* bB = bA + CC * K;                                   // [CC][K]
-  const int tid = threadIdx.x;
-  const R* mset = d.minv + (size_t)set * d.M * K * K;
-  for (int idx = tid; idx < K * K; idx += IM_THREADS) {
-    mi[idx] = mset[(size_t)n1 * K * K + idx];
-    mi[K * K + idx] = mset[(size_t)n2 * K * K + idx];
-  }
-  for (int f = 0; f < 4; ++f)
-    if (d.vd_on[f])
-      for (int idx = tid; idx < K * K; idx += IM_THREADS)
-        vdT[f * K * K + idx] = d.vdiff[((size_t)set * 4 + f) * K * K + idx];
-  for (int idx = tid; idx < K; idx += IM_THREADS) {
-    vs[0 * K + idx] = vrow(d, LBM_VERT_RALPHA, idx);
-    vs[1 * K + idx] = vrow(d, LBM_VERT_RDLOG3, idx);
-    vs[2 * K + idx] = vrow(d, LBM_VERT_GG, idx);
-    vs[3 * K + idx] = vrow(d, LBM_VERT_DSIG, idx);
-    vs[4 * K + idx] = vrow(d, LBM_VERT_ALPHA, idx);
-    vs[5 * K + idx] = vrow(d, LBM_VERT_W3, idx);
-    ktr[idx] = vrow(d, LBM_VERT_KTREF, idx);
-  }
-  __syncthreads();
-  const R dt2 = R(2) * dt, gam = d.robert;
-  const C2<R> z = cmk<R>(0, 0);
-  const size_t e3 = (size_t)e * 4 * NS * K;
-  const size_t efrc3 = d.frc_shared ? 0 : e3;
-  const size_t efrcs = d.frc_shared ? 0 : (size_t)e * NS;
-  for (int c0 = 0; c0 < ncoef; c0 += CC) {
-    const int c = tid / K, k = tid % K;
-    const int coef = c0 + c;
-    const bool act = (c < CC) && (coef < ncoef);
-    int n = 0, m = 0, sel = 0;
-    if (act) {
-      if (coef < C1) { n = n1; m = coef; sel = 0; }
-      else { n = n2; m = coef - C1; sel = 1; }
-    }
-    const size_t idx = (size_t)spec_index(m, n, N);
-    const size_t o = idx * K + k;
-    C2<R> aV = z, aD = z, aT = z, aQ = z, bV = z, bD = z, bT = z, bQ = z;
-    C2<R> wV = z, wD = z, wT = z, wQ = z, wpi = z, pp = z;
-    R ktt = 0, kd = 0, kv = 0, kq = 0, lap = 0;
-    if (act) {
-      aV = d.sa3[e3 + 0 * NS * K + o]; aD = d.sa3[e3 + 1 * NS * K + o];
-      aT = d.sa3[e3 + 2 * NS * K + o]; aQ = d.sa3[e3 + 3 * NS * K + o];
-      bV = d.sb3[e3 + 0 * NS * K + o]; bD = d.sb3[e3 + 1 * NS * K + o];
-      bT = d.sb3[e3 + 2 * NS * K + o]; bQ = d.sb3[e3 + 3 * NS * K + o];
-      wV = d.tend[e3 + 0 * NS * K + o]; wD = d.tend[e3 + 1 * NS * K + o];
-      wT = d.tend[e3 + 2 * NS * K + o]; wQ = d.tend[e3 + 3 * NS * K + o];
-      wpi = d.tends[((size_t)e * 2 + 0) * NS + idx];
-      pp = d.tends[((size_t)e * 2 + 1) * NS + idx];
-      if (d.frc3) {
-        wV = wV + d.frc3[efrc3 + 0 * NS * K + o]; wD = wD + d.frc3[efrc3 + 1 * NS * K + o];
-        wT = wT + d.frc3[efrc3 + 2 * NS * K + o]; wQ = wQ + d.frc3[efrc3 + 3 * NS * K + o];
-      }
-      if (d.frcs) wpi = wpi + d.frcs[efrcs + idx];
-      ktt = d.ktt[n * K + k]; kd = d.kd[n * K + k]; kv = d.kv[n * K + k]; kq = d.kq[n * K + k];
-      lap = d.lap[n];
-    }
-    C2<R>* A = bA + c * K;
-    C2<R>* B = bB + c * K;
-    const R bt = dt2 * ktt;                      // 2 dt ktt; ft = 1 + bt
-    __syncthreads();
-    // wdx = T(t-dt) (1 + dt ktt) + dt wT  (integrator.py:287)
-    if (act) A[k] = bT + (bT * ktt + wT) * dt;
-    __syncthreads();
-    if (act) {
-      C2<R> pre = z;                                       // sum_{l<k} R dlog3_l wdx_l
-      for (int l = 0; l < k; ++l) cfma(pre, vs[1 * K + l], A[l]);
-      CX<R> phi = cx_add(cx_prod(vs[0 * K + k], A[k]), cx(pre));   // WW wdx
-      const C2<R> wdpix = pp + wpi * dt;
-      const R gk = vs[2 * K + k];
-      // wdphiy = WW wdx + ft gg wdpix, ft gg taken as gg + bt gg
-      phi = cx_add(phi, cx_add(cx_prod(gk, wdpix), cx_mul(cx_prod(bt, wdpix), gk)));
-      // dt (wD ft - lap wdphiy), the two terms nearly balancing
-      const CX<R> zz = cx_add(cx_add(cx(wD), cx_prod(bt, wD)), cx_mul(phi, -lap));
-      const R ad = dt * kd;
-      B[k] = bD + (bD * (ad + bt + ad * bt) + cx_val(zz) * dt);
-    }
-    __syncthreads();
-    C2<R> dbar = z;
-    if (act) {
-      const R* mm_ = mi + sel * K * K;
-      // M(n)^-1 rhs with exact products and compensated sums (the divergence
-      // of a balanced flow is small against the terms of this sum)
-      CX<R> acc = cx<R>(z);
-      for (int l = 0; l < K; ++l) acc = cx_add(acc, cx_prod(mm_[l * K + k], B[l]));   // minv (l, k)
-      dbar = cx_val(acc);
-    }
-    __syncthreads();
-    if (act) A[k] = dbar;
-    __syncthreads();
-    C2<R> nV = z, nD = z, nT = z, nQ = z, npi = z;
-    if (act) {
-      C2<R> suf = z;                                        // sum_{l>k} dsig_l dbar_l
-      for (int l = K - 1; l > k; --l) cfma(suf, vs[3 * K + l], A[l]);
-      const CX<R> sfx = cx(suf);
-      const CX<R> corr = cx_mul(cx_add(cx_prod(vs[4 * K + k], dbar), cx_mul(sfx, vs[5 * K + k])),
-                                ktr[k]);
-      const C2<R> yT = bT + cx_val(cx_add(cx(wT), cx_neg(corr))) * dt2;
-      nT = yT - yT * (bt / (R(1) + bt));
-      if (k == 0) {
-        const CX<R> dsum = cx_add(sfx, cx_prod(vs[3 * K], dbar));
-        npi = pp + cx_val(cx_add(cx(wpi), cx_neg(dsum))) * dt2;
-      }
-      nD = dbar * R(2) - bD;
-      const R av = dt2 * kv, aq = dt2 * kq;
-      const C2<R> xV = bV + wV * dt2, xQ = bQ + wQ * dt2;
-      nV = xV - xV * (av / (R(1) + av));
-      nQ = xQ - xQ * (aq / (R(1) + aq));
-    }
-    // implicit vertical diffusion (integrator.py:311-314); vdT holds the
-    // operator minus the identity
-    C2<R>* vals[4] = {&nV, &nD, &nT, &nQ};
-#pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      if (!d.vd_on[f]) continue;
-      __syncthreads();
-      if (act) A[k] = *vals[f];
-      __syncthreads();
-      if (act && !(f < 2 && n < 2)) {
-        C2<R> o2 = *vals[f];
-        const R* vm = vdT + f * K * K;
-        for (int l = 0; l < K; ++l) cfma(o2, vm[l * K + k], A[l]);
-        *vals[f] = o2;
-      }
-    }
-    // Robert-Asselin filter of the previous level (spectral part) and update
-    if (act) {
-      C2<R> fV, fD, fT, fQ;
-      if (ra_mode) {
-        fV = aV + (bV - aV * R(2) + nV) * gam;
-        fD = aD + (bD - aD * R(2) + nD) * gam;
-        fT = aT + (bT - aT * R(2) + nT) * gam;
-        fQ = aQ + (bQ - aQ * R(2) + nQ) * gam;
-      } else {
-        fV = aV; fD = aD; fT = aT; fQ = aQ;
-      }
-      d.sb3[e3 + 0 * NS * K + o] = fV; d.sb3[e3 + 1 * NS * K + o] = fD;
-      d.sb3[e3 + 2 * NS * K + o] = fT; d.sb3[e3 + 3 * NS * K + o] = fQ;
-      d.sa3[e3 + 0 * NS * K + o] = nV; d.sa3[e3 + 1 * NS * K + o] = nD;
-      d.sa3[e3 + 2 * NS * K + o] = nT; d.sa3[e3 + 3 * NS * K + o] = nQ;
-      const bool fin = isfinite(nV.x) && isfinite(nV.y) && isfinite(nD.x) && isfinite(nD.y) &&
-                       isfinite(nT.x) && isfinite(nT.y) && isfinite(nQ.x) && isfinite(nQ.y) &&
-                       isfinite(npi.x) && isfinite(npi.y);
-      if (!fin) {
-        atomicOr(d.err, 1);
-        if (d.err_member) atomicOr(d.err_member + e, 1);
-      }
-    }
-    // column sums for sigma-dot of the next step
-    __syncthreads();
-    if (act) { A[k] = nV; B[k] = nD; }
-    __syncthreads();
-    if (act && k == 0) {
-      C2<R> sv = z, sdv = z;
-      for (int l = 0; l < K; ++l) {
-        cfma(sv, vs[3 * K + l], A[l]);
-        cfma(sdv, vs[3 * K + l], B[l]);
-      }
-      const R il = d.invlap[n];
-      const size_t es = (size_t)e * 4 * NS;
-      d.sas[es + 0 * NS + idx] = npi;
-      d.sas[es + 1 * NS + idx] = sv * il;     // sum dsig psi
-      d.sas[es + 2 * NS + idx] = sdv * il;    // sum dsig chi
-      d.sas[es + 3 * NS + idx] = sdv;         // sum dsig div
-    }
-  }
-}
-
 // column sums of a freshly loaded current level
 template <typename R>
 __global__ void k_colsum(SD<R> d) {
@@ -618,6 +419,7 @@ __global__ void k_ps_flush(SD<R> d, int ps_mode) {
 
 }  // namespace lbm
 #include "legendre_fma.cuh"
+#include "implicit.cuh"
 #include "grid_split.cuh"
 #include "grid_fft.cuh"
 #include "legendre_tc.cuh"
@@ -660,9 +462,21 @@ template <typename R> void launch_synth(const SD<R>& d, cudaStream_t st, bool at
   else
     k_synth<R, 2><<<dim3(NP, (d.E + sp.eb - 1) / sp.eb, sp.nch + 1), sp.nt, sp.smem, st>>>(d, sp);
 }
-template <typename R> size_t impl_smem(int K) {
-  return sizeof(R) * ((size_t)(2 + 4) * K * K + 7 * (size_t)K + (K & 1)) +
-         sizeof(C2<R>) * 2 * (size_t)(IM_THREADS / K) * K;
+// Implicit update: 8- / 16-byte accesses where every complex array is so aligned.
+template <typename R> void launch_implicit(const SD<R>& d, R dt, int set, int ra_mode,
+                                           cudaStream_t st, bool attrs) {
+  const ImplPlan pl = impl_plan(d.E, d.K, d.N);
+  const int smem = (int)impl_smem<R>(d.K, pl.CC);
+  const uintptr_t all = (uintptr_t)d.sa3 | (uintptr_t)d.sb3 | (uintptr_t)d.tend |
+                        (uintptr_t)d.frc3;
+  auto go = [&](auto kern) {
+    if (attrs)
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    else
+      kern<<<dim3((d.M + 1) / 2, d.E, pl.nch), pl.nt, smem, st>>>(d, dt, set, ra_mode, pl.CC);
+  };
+  if (all & (2 * sizeof(R) - 1)) go(k_implicit<R, false>);
+  else go(k_implicit<R, true>);
 }
 
 // Grid of a persistent kernel: the CTAs that are resident at once on the
@@ -696,8 +510,6 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
                                              cudaStream_t st, int only = -1) {
   constexpr int KB = grid_kb<R, I>(), NT = grid_nt<R, I>();
   const int NP = (d.M + 1) / 2;
-  const int JH = d.J / 2;
-  const int NRmax = d.N + 2;
   const size_t gsm = GridSmem<R, I, KB, NT>::bytes(d.M);
   if constexpr (sizeof(R) == 4) {
     // grid-point part as three launches: longitude synthesis, column
@@ -756,8 +568,7 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
     if (level) launch_anal<R>(d, st, false);
   }
   if (only < 0 || only == 2)
-    k_implicit<R><<<dim3(NP, d.E), IM_THREADS, impl_smem<R>(d.K), st>>>(d, R(c.dt), c.set,
-                                                                         c.ra_mode);
+    launch_implicit<R>(d, R(c.dt), c.set, c.ra_mode, st, false);
   if (only < 0 || only == 3) launch_synth<R>(d, st, false);
   LBM_LAUNCH_CHECK();
   return LBM_OK;
@@ -765,7 +576,6 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
 
 template <typename R, int I> void set_attrs(const SD<R>& d) {
   constexpr int KB = grid_kb<R, I>(), NT = grid_nt<R, I>();
-  const int JH = d.J / 2, NRmax = d.N + 2;
   if constexpr (sizeof(R) == 4) {
     cudaFuncSetAttribute(k_idft<I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)idft_smem(I, d.M));
@@ -799,8 +609,7 @@ template <typename R, int I> void set_attrs(const SD<R>& d) {
       persistent_grid((const void*)k_anal_tc, ATC_THREADS, pl.smem, 1);
     }
   }
-  cudaFuncSetAttribute(k_implicit<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)impl_smem<R>(d.K));
+  launch_implicit<R>(d, R(0), 0, 0, nullptr, true);
   if constexpr (sizeof(R) == 4) {
     if (d.legendre) {
       const StcPlan pl = stc_plan(d.E, d.J, d.K, d.N, d.tc_g);

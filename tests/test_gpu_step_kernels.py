@@ -222,3 +222,102 @@ def test_legendre_kernels_against_fp64_sums(torch, I, J, N, K, nmem, precision):
     for f in range(5):
         check(stp.sfs[..., f], want[f][..., 0], size[f][..., 0], N + 1)
     assert int(stp.err.item()) == 0
+
+
+IMPL_SHAPES = [  # I, J, N, K, members: one coefficient per share and many, one level, the
+                 # most levels, shares that cross from one n of a pair to the other, N odd and even
+    (64, 32, 21, 1, 1), (64, 32, 21, 64, 1), (64, 6, 3, 7, 40), (128, 50, 31, 2, 3),
+    (128, 64, 42, 20, 1), (128, 64, 42, 17, 30), (256, 128, 85, 9, 2)]
+
+
+@pytest.mark.parametrize("I,J,N,K,nmem", IMPL_SHAPES)
+@pytest.mark.parametrize("vdiff", [False, True])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_implicit_kernel_against_fp64_formula(torch, I, J, N, K, nmem, vdiff, precision):
+    """k_implicit against the update written out in FP64 on the same operators.
+    Each result is a sum of products along a path of at most 4 K + 40 rounded
+    operations: that many u times the same formula on magnitudes.  Arrays moved
+    off their element alignment take the narrow accesses: the same bits."""
+    from lbm_isca_gb300._lib import StepperDesc
+    stp = _grid_stepper(torch, I, J, N, K, nmem, precision)
+    u = 2.0 ** -24 if precision == "fp32" else 2.0 ** -53
+    for x, seed, scale in ((stp.sa3, 1, 1.0), (stp.sb3, 2, 1.0), (stp.tend, 3, 1e-3),
+                           (stp.tends, 4, 1e-3)):
+        _noise(torch, x, seed)
+        x.mul_(scale)
+    stp.vd_on = [int(vdiff)] * 4
+    g = torch.Generator(device="cuda").manual_seed(5)
+    stp.vdm = torch.randn((1, 4, K, K), generator=g, device="cuda",
+                          dtype=torch.float64).mul(0.1).to(stp.minv.dtype)
+    stp._desc = None
+    dt, K1 = 600.0, K + 1
+    vert = stp.vert.double().reshape(-1, K1)[:, :K]
+    dsig, alpha, w3 = vert[0], vert[2], vert[3]
+    rdlog3, ralpha, ktref, gg = vert[6], vert[7], vert[9], vert[11]
+    pm, pn = stp.pm, stp.pn
+    cplx = lambda x: x.to(torch.complex128)                       # noqa: E731
+    prev = [cplx(stp.sa3[:, f]) for f in range(4)]
+    b = [cplx(stp.sb3[:, f]) for f in range(4)]
+    w = [cplx(stp.tend[:, f]) for f in range(4)]
+    wpi, pi = (cplx(stp.tends[:, f]) for f in range(2))
+    tab = lambda x: x.double().reshape(stp.M, K)[pn]              # noqa: E731
+    ktt, kd, kv, kq = tab(stp.ktt), tab(stp.kd), tab(stp.kv), tab(stp.kq)
+    lap, il = stp.lap.double()[pn][:, None], stp.invlap.double()[pn][:, None]
+    minv = stp.minv[0].double()[pn]
+    vdm, gam = stp.vdm[0].double(), float(torch.tensor(stp.robert, dtype=stp.minv.dtype))
+
+    def update(prev, b, w, wpi, pi, lap, il, minv, vdm, s):
+        """s = -1: the update; s = +1 with magnitudes: its bound."""
+        wdx = b[2] + dt * (b[2] * ktt + w[2])
+        run = torch.cumsum(wdx * rdlog3, -1) - wdx * rdlog3 if s < 0 else \
+            torch.cumsum(wdx * rdlog3, -1)
+        bt = 2 * dt * ktt
+        phi = ralpha * wdx + run + (1 + bt) * gg * (pi + dt * wpi)[..., None]
+        ad = dt * kd
+        rhs = b[1] + b[1] * (ad + bt + ad * bt) + dt * ((1 + bt) * w[1] + s * lap * phi)
+        dbar = torch.einsum("slk,esl->esk", minv.to(rhs.dtype), rhs)
+        x = dsig * dbar
+        after = x.flip(-1).cumsum(-1).flip(-1) + (s * x if s < 0 else 0)
+        damp = lambda y, c: y + s * y * (c / (1 + c))             # noqa: E731
+        t = damp(b[2] + 2 * dt * (w[2] + s * ktref * (alpha * dbar + w3 * after)), bt)
+        npi = pi + 2 * dt * (wpi + s * x.sum(-1))
+        new = [damp(b[0] + 2 * dt * w[0], 2 * dt * kv), 2 * dbar + s * b[1], t,
+               damp(b[3] + 2 * dt * w[3], 2 * dt * kq)]
+        if vdiff:
+            for f in range(4):
+                on = ((pn >= 2) | torch.tensor(f >= 2, device="cuda"))[:, None]
+                new[f] = new[f] + on * torch.einsum("lk,esl->esk", vdm[f].to(rhs.dtype), new[f])
+        old = [a + gam * (b_ + s * 2 * a + n) for a, b_, n in zip(prev, b, new)]
+        sv, sd = (new[0] * dsig).sum(-1), (new[1] * dsig).sum(-1)
+        il0 = il[:, 0]
+        return new, old, [npi, sv * il0, sd * il0, sd]
+
+    a = lambda xs: [x.abs() for x in xs]                          # noqa: E731
+    want = update(prev, b, w, wpi, pi, lap, il, minv, vdm, -1)
+    size = update(a(prev), a(b), a(w), wpi.abs(), pi.abs(), lap.abs(), il.abs(), minv.abs(),
+                  vdm.abs(), 1)
+    state = [x.clone() for x in (stp.sa3, stp.sb3)]
+    _launch(torch, stp, 2)
+    got = stp.sa3, stp.sb3, stp.sas
+    for gx, wx, sx in zip(got, want, size):
+        for f in range(4):
+            err = (cplx(gx[:, f]) - wx[f]).abs()
+            lim = (4 * K + 40) * u * sx[f] + 1e-300
+            assert bool((err <= lim).all()), (f, float((err / lim).max()))
+    assert int(stp.err.item()) == 0
+
+    first = [x.clone() for x in got]
+    moved, views = [], []
+    for x in (state[0], state[1], stp.tend):
+        r = torch.view_as_real(x).reshape(-1)
+        buf = torch.empty(r.numel() + 1, device="cuda", dtype=r.dtype)
+        buf[1:] = r
+        moved.append(buf)
+        views.append(buf[1:])
+    d = StepperDesc.from_buffer_copy(stp.desc())
+    d.sa3, d.sb3, d.tend = (v.data_ptr() for v in views)
+    stp.sas.zero_()
+    _launch(torch, stp, 2, desc=d)
+    for v, f in zip(views[:2], first):
+        assert torch.equal(v, torch.view_as_real(f).reshape(-1))
+    assert torch.equal(stp.sas, first[2])
