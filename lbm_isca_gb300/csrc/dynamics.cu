@@ -11,108 +11,150 @@ namespace lbm {
 constexpr int KMAX_LOCAL = 64;   // largest level count the column kernels hold
 
 // Vertical advection, SECOND_CENTERED ADVECTIVE_FORM with the overall +
-// sign of dynamics.py:117-143; f(l), s(l) are level accessors.
-template <typename R, typename F, typename S>
-LBM_D R vert_adv(int k, int K, F f, S s, R dsk) {
+// sign of dynamics.py:117-143: f(l) is a level accessor, s0 and s1 the
+// vertical velocities at the half levels k and k + 1.
+template <typename R, typename F>
+LBM_D R vert_adv(int k, int K, F f, R s0, R s1, R dsk, R rdsk) {
   const R fk = f(k);
-  const R flo = (k >= 1) ? s(k) * R(0.5) * (fk + f(k - 1)) : R(0);
-  const R fhi = (k + 1 <= K - 1) ? s(k + 1) * R(0.5) * (f(k + 1) + fk) : R(0);
-  return (fhi - flo - fk * (s(k + 1) - s(k))) / dsk;
+  const R flo = (k >= 1) ? s0 * R(0.5) * (fk + f(k - 1)) : R(0);
+  const R fhi = (k + 1 <= K - 1) ? s1 * R(0.5) * (f(k + 1) + fk) : R(0);
+  const R x = fhi - flo - fk * (s1 - s0);
+  if constexpr (sizeof(R) == 8) return x * rdsk;   // a division costs ten products
+  else return x / dsk;
+}
+
+// One thread per (column, level), TG_THREADS / K columns a block: consecutive
+// lanes read consecutive levels, the column sums come from shared memory, each
+// thread its own (the order of every sum is the level's).  Bound by the FP64 pipe
+// (about 165 multiply-adds a level at 20 levels).  One thread per column
+// with its level arrays in local memory left one member of T42 on 256 warps:
+// 291 -> 83 us at T42, 20 levels, one member, FP64.
+constexpr int TG_THREADS = 256;
+
+template <typename R> size_t tend_smem(int K) {
+  const int CB = TG_THREADS / K;
+  return sizeof(R) * ((size_t)2 * K * K + 4 * (size_t)CB * K + CB);
 }
 
 template <typename R>
-__global__ void k_tendency_grid(lbm_tend_grid_args a) {
-  const int J = a.nlat, I = a.nlon, K = a.kmax;
-  const size_t col = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(TG_THREADS) k_tendency_grid(lbm_tend_grid_args a) {
+  const int J = a.nlat, I = a.nlon, K = a.kmax, CB = TG_THREADS / K;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  R* mt = reinterpret_cast<R*>(smraw);     // [K][K] tmtx^T (l, k)
+  R* mw = mt + K * K;                      // [K][K] ww^T (l, k)
+  R* sw = mw + K * K;                      // [CB][K] div + padv
+  R* sp = sw + CB * K;                     // [CB][K] padv
+  R* sdv = sp + CB * K;                    // [CB][K] div
+  R* sx = sdv + CB * K;                    // [CB][K] tv' - t
+  R* s0s = sx + CB * K;                    // [CB] S[0]
   const size_t ncol2 = (size_t)J * I;
-  if (col >= (size_t)a.nmem * ncol2) return;
-  const size_t e = col / ncol2, ji = col % ncol2;
-  const R kappa = R(a.kappa), eps = R(a.epsvt), rair = R(a.rair);
+  const int tid = threadIdx.x, c = tid / K, k = tid - c * K;
+  const size_t col = (size_t)blockIdx.x * CB + c;
+  const bool act = c < CB && col < (size_t)a.nmem * ncol2;
   auto P = [](const void* p) { return (const R*)p; };
-  const R *dsig = P(a.dsig), *sigm = P(a.sigm), *alpha = P(a.alpha), *w3 = P(a.w3),
-          *wP = P(a.wP), *cpg = P(a.cpg), *sig = P(a.sig), *ww = P(a.ww), *tmtx = P(a.tmtx),
-          *tref = P(a.tref);
+  for (int x = tid; x < K * K; x += TG_THREADS) {
+    const int kk = x / K, l = x - kk * K;
+    mt[l * K + kk] = P(a.tmtx)[x];
+    mw[l * K + kk] = P(a.ww)[x];
+  }
+  const size_t e = act ? col / ncol2 : 0, ji = act ? col - e * ncol2 : 0;
+  const R kappa = R(a.kappa), eps = R(a.epsvt), rair = R(a.rair);
+  const R *dsig = P(a.dsig), *sigm = P(a.sigm);
   const size_t b3 = ji * K;                // basic-state column offset
-  const size_t p3 = col * K;               // perturbation column offset
+  const size_t p3 = (act ? col : 0) * K;   // perturbation column offset
   const R *ub = P(a.ub) + b3, *vb = P(a.vb) + b3, *tb = P(a.tb) + b3, *qb = P(a.qb) + b3,
           *tvb = P(a.tvb) + b3, *absv = P(a.absvor) + b3, *divb = P(a.divb) + b3,
           *x5b = P(a.x5b) + b3, *sdb = P(a.sdotb) + ji * (K + 1);
   const R *u = P(a.u) + p3, *v = P(a.v) + p3, *t = P(a.t) + p3, *q = P(a.q) + p3,
           *vor = P(a.vor) + p3, *div = P(a.div) + p3;
-  const R pixb = P(a.pixb)[ji], piyb = P(a.piyb)[ji], psb = P(a.psb)[ji];
-  const R pix = P(a.pix)[col], piy = P(a.piy)[col], ps = P(a.ps)[col];
-
-  R S[KMAX_LOCAL + 1], sd[KMAX_LOCAL + 1], padv[KMAX_LOCAL], x[KMAX_LOCAL];
-  for (int k = 0; k < K; ++k) padv[k] = u[k] * pixb + ub[k] * pix + v[k] * piyb + vb[k] * piy;
-  // S[k] = sum_{l>=k} dsig_l (div + padv)_l  (dynamics.py:96-102)
-  S[K] = R(0);
-  for (int k = K - 1; k >= 0; --k) S[k] = S[k + 1] + (div[k] + padv[k]) * dsig[k];
-  for (int k = 0; k <= K; ++k) sd[k] = sigm[k] * S[0] - S[k];   // dynamics.py:105-114
-  sd[0] = R(0);
-  sd[K] = R(0);
-  // gt_pi = -S[0] + sum dsig div (dynamics.py:188) = -sum dsig padv: summed
-  // directly, without the cancellation of two O(div) terms
-  R gtpi = R(0);
-  for (int k = 0; k < K; ++k) gtpi -= padv[k] * dsig[k];
-  if (a.frc_ps) gtpi += P(a.frc_ps)[e * a.frc_ps_stride + ji];
-  ((R*)a.gt_pi)[col] = gtpi;
-  for (int k = 0; k < K; ++k) x[k] = t[k] + eps * (t[k] * qb[k] + tb[k] * q[k]);  // tv'
-
-  R *fu = (R*)a.fu + p3, *fv = (R*)a.fv + p3, *ke = (R*)a.ke + p3, *gt = (R*)a.gt + p3,
-    *xu = (R*)a.xu + p3, *xv = (R*)a.xv + p3, *g = (R*)a.g + p3, *yu = (R*)a.yu + p3,
-    *yv = (R*)a.yv + p3;
-  const R* frt = a.frc_t ? P(a.frc_t) + e * a.frc_t_stride + b3 : nullptr;
-  const R* frq = a.frc_q ? P(a.frc_q) + e * a.frc_q_stride + b3 : nullptr;
-  auto fS = [&](int l) { return sd[l]; };
-  auto fSb = [&](int l) { return sdb[l]; };
-  for (int k = 0; k < K; ++k) {
-    const R tv = x[k];
-    const R x5p = alpha[k] * div[k] + wP[k] * padv[k] + w3[k] * S[k + 1];
-    const R adiab = -kappa * (tv * x5b[k] + tvb[k] * x5p);
-    const R tdev = tb[k] - tref[k];
-    xu[k] = u[k] * tdev + ub[k] * t[k];
-    xv[k] = v[k] * tdev + vb[k] * t[k];
-    const R hadv = t[k] * divb[k] + tdev * div[k];
-    const R vadv = vert_adv<R>(k, K, [&](int l) { return t[l]; }, fSb, dsig[k]) +
-                   vert_adv<R>(k, K, [&](int l) { return tb[l]; }, fS, dsig[k]);
-    R tm = R(0);
-    for (int l = 0; l < K; ++l) tm += div[l] * tmtx[k * K + l];
-    R gtk = adiab + hadv + vadv + tm;
-    if (frt) gtk += frt[k];
-    gt[k] = gtk;
-    // momentum (dynamics.py:224-237)
-    const R rcpg = rair * cpg[k];
-    const R tvdev = tvb[k] - tref[k];
-    R fuk = v[k] * absv[k] + vb[k] * vor[k];
-    R fvk = -u[k] * absv[k] - ub[k] * vor[k];
-    fuk -= rcpg * (tv * pixb + tvdev * pix);
-    fvk -= rcpg * (tv * piyb + tvdev * piy);
-    fuk += vert_adv<R>(k, K, [&](int l) { return u[l]; }, fSb, dsig[k]) +
-           vert_adv<R>(k, K, [&](int l) { return ub[l]; }, fS, dsig[k]);
-    fvk += vert_adv<R>(k, K, [&](int l) { return v[l]; }, fSb, dsig[k]) +
-           vert_adv<R>(k, K, [&](int l) { return vb[l]; }, fS, dsig[k]);
-    fu[k] = fuk;
-    fv[k] = fvk;
-    R phiv = R(0);
-    for (int l = 0; l < K; ++l) phiv += (x[l] - t[l]) * ww[k * K + l];
-    R kek = phiv + u[k] * ub[k] + v[k] * vb[k];
-    if (a.lin_u)   // tangent-linear: linearised about the trajectory (lin_u, lin_v)
-      kek += P(a.lin_u)[p3 + k] * u[k] + P(a.lin_v)[p3 + k] * v[k];
-    else if (!a.strictly_linear)
-      kek += R(0.5) * (u[k] * u[k] + v[k] * v[k]);
-    ke[k] = kek;
-    // humidity (dynamics.py:256-262)
-    yu[k] = u[k] * qb[k] + ub[k] * q[k];
-    yv[k] = v[k] * qb[k] + vb[k] * q[k];
-    R gk = q[k] * divb[k] + qb[k] * div[k] +
-           vert_adv<R>(k, K, [&](int l) { return q[l]; }, fSb, dsig[k]) +
-           vert_adv<R>(k, K, [&](int l) { return qb[l]; }, fS, dsig[k]);
-    if (frq) gk += frq[k];
-    g[k] = gk;
-    if (a.omega) ((R*)a.omega)[p3 + k] = -sig[k] * (x5p * psb + x5b[k] * ps);
+  R pixb = R(0), piyb = R(0), pix = R(0), piy = R(0), padv = R(0), tv = R(0), dv = R(0);
+  if (act) {
+    pixb = P(a.pixb)[ji];
+    piyb = P(a.piyb)[ji];
+    pix = P(a.pix)[col];
+    piy = P(a.piy)[col];
+    dv = div[k];
+    padv = u[k] * pixb + ub[k] * pix + v[k] * piyb + vb[k] * piy;
+    tv = t[k] + eps * (t[k] * qb[k] + tb[k] * q[k]);     // tv'
+    sw[tid] = dv + padv;
+    sp[tid] = padv;
+    sdv[tid] = dv;
+    sx[tid] = tv - t[k];
   }
-  if (a.sdot)
-    for (int k = 0; k <= K; ++k) ((R*)a.sdot)[col * (K + 1) + k] = sd[k];
+  __syncthreads();
+  // S_k = sum_{l>=k} dsig_l (div + padv)_l  (dynamics.py:96-102)
+  const int cK = c * K;
+  R Sk1 = R(0), Sk = R(0);
+  if (act) {
+    for (int l = K - 1; l > k; --l) Sk1 = Sk1 + sw[cK + l] * dsig[l];
+    Sk = Sk1 + sw[tid] * dsig[k];
+    if (k == 0) s0s[c] = Sk;
+    if (k == K - 1) {
+      // gt_pi = -S[0] + sum dsig div (dynamics.py:188) = -sum dsig padv: summed
+      // directly, without the cancellation of two O(div) terms
+      R gtpi = R(0);
+      for (int l = 0; l < K; ++l) gtpi -= sp[cK + l] * dsig[l];
+      if (a.frc_ps) gtpi += P(a.frc_ps)[e * a.frc_ps_stride + ji];
+      ((R*)a.gt_pi)[col] = gtpi;
+    }
+  }
+  __syncthreads();
+  if (!act) return;
+  const R S0 = s0s[c];
+  // sigma-dot at the half levels k and k + 1 (dynamics.py:105-114)
+  const R sd0 = k == 0 ? R(0) : sigm[k] * S0 - Sk;
+  const R sd1 = k == K - 1 ? R(0) : sigm[k + 1] * S0 - Sk1;
+  const R sb0 = sdb[k], sb1 = sdb[k + 1], dsk = dsig[k], rdsk = R(1) / dsk;
+  auto vadv = [&](const R* f, const R* fb) {
+    return vert_adv<R>(k, K, [&](int l) { return f[l]; }, sb0, sb1, dsk, rdsk) +
+           vert_adv<R>(k, K, [&](int l) { return fb[l]; }, sd0, sd1, dsk, rdsk);
+  };
+  const R x5p = P(a.alpha)[k] * dv + P(a.wP)[k] * padv + P(a.w3)[k] * Sk1;
+  const R adiab = -kappa * (tv * x5b[k] + tvb[k] * x5p);
+  const R tdev = tb[k] - P(a.tref)[k];
+  ((R*)a.xu)[p3 + k] = u[k] * tdev + ub[k] * t[k];
+  ((R*)a.xv)[p3 + k] = v[k] * tdev + vb[k] * t[k];
+  const R hadv = t[k] * divb[k] + tdev * dv;
+  R tm = R(0), phiv = R(0);
+#pragma unroll 4
+  for (int l = 0; l < K; ++l) {
+    tm += sdv[cK + l] * mt[l * K + k];
+    phiv += sx[cK + l] * mw[l * K + k];
+  }
+  R gtk = adiab + hadv + vadv(t, tb) + tm;
+  if (a.frc_t) gtk += P(a.frc_t)[e * a.frc_t_stride + b3 + k];
+  ((R*)a.gt)[p3 + k] = gtk;
+  // momentum (dynamics.py:224-237)
+  const R rcpg = rair * P(a.cpg)[k];
+  const R tvdev = tvb[k] - P(a.tref)[k];
+  R fuk = v[k] * absv[k] + vb[k] * vor[k];
+  R fvk = -u[k] * absv[k] - ub[k] * vor[k];
+  fuk -= rcpg * (tv * pixb + tvdev * pix);
+  fvk -= rcpg * (tv * piyb + tvdev * piy);
+  fuk += vadv(u, ub);
+  fvk += vadv(v, vb);
+  ((R*)a.fu)[p3 + k] = fuk;
+  ((R*)a.fv)[p3 + k] = fvk;
+  R kek = phiv + u[k] * ub[k] + v[k] * vb[k];
+  if (a.lin_u)   // tangent-linear: linearised about the trajectory (lin_u, lin_v)
+    kek += P(a.lin_u)[p3 + k] * u[k] + P(a.lin_v)[p3 + k] * v[k];
+  else if (!a.strictly_linear)
+    kek += R(0.5) * (u[k] * u[k] + v[k] * v[k]);
+  ((R*)a.ke)[p3 + k] = kek;
+  // humidity (dynamics.py:256-262)
+  ((R*)a.yu)[p3 + k] = u[k] * qb[k] + ub[k] * q[k];
+  ((R*)a.yv)[p3 + k] = v[k] * qb[k] + vb[k] * q[k];
+  R gk = q[k] * divb[k] + qb[k] * dv + vert_adv<R>(k, K, [&](int l) { return q[l]; }, sb0, sb1, dsk, rdsk) +
+         vert_adv<R>(k, K, [&](int l) { return qb[l]; }, sd0, sd1, dsk, rdsk);
+  if (a.frc_q) gk += P(a.frc_q)[e * a.frc_q_stride + b3 + k];
+  ((R*)a.g)[p3 + k] = gk;
+  if (a.omega)
+    ((R*)a.omega)[p3 + k] = -P(a.sig)[k] * (x5p * P(a.psb)[ji] + x5b[k] * P(a.ps)[col]);
+  if (a.sdot) {
+    R* o = (R*)a.sdot + col * (K + 1) + k;
+    o[0] = sd0;
+    if (k == K - 1) o[1] = sd1;
+  }
 }
 
 // One block per (e, m, n) coefficient, thread per level.
@@ -204,12 +246,17 @@ int lbm_tendency_grid(int prec, const lbm_tend_grid_args* a, void* stream) {
     return LBM_ERR_ARG;
   if ((a->lin_u == nullptr) != (a->lin_v == nullptr)) return LBM_ERR_ARG;
   const size_t cols = (size_t)a->nmem * a->nlat * a->nlon;
-  const int threads = 32;   // one member's 8192 columns (T42) over all SMs
-  const unsigned blocks = (unsigned)((cols + threads - 1) / threads);
+  const int CB = TG_THREADS / a->kmax;
+  const unsigned blocks = (unsigned)((cols + CB - 1) / CB);
+  auto go = [&](auto kern, size_t smem) {
+    // one limit for all level counts: other threads and captured launches rely on it
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    kern<<<blocks, TG_THREADS, smem, (cudaStream_t)stream>>>(*a);
+  };
   if (prec == LBM_F64)
-    k_tendency_grid<double><<<blocks, threads, 0, (cudaStream_t)stream>>>(*a);
+    go(k_tendency_grid<double>, tend_smem<double>(a->kmax));
   else if (prec == LBM_F32)
-    k_tendency_grid<float><<<blocks, threads, 0, (cudaStream_t)stream>>>(*a);
+    go(k_tendency_grid<float>, tend_smem<float>(a->kmax));
   else
     return LBM_ERR_ARG;
   LBM_LAUNCH_CHECK();

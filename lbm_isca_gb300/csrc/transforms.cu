@@ -84,94 +84,179 @@ k_fourier_inv(int J, int C, int M, const C2<R>* __restrict__ four, const R* __re
   }
 }
 
-constexpr int LG_COLS = 16;     // columns per block of the Legendre kernels
-constexpr int LG_ROWS = 16;     // thread rows (n or j)
+// Legendre sums of the transform API.  One thread per output value (n or j, column):
+// a block takes LG_NT consecutive values of one (m, batch, column chunk), walks the
+// summation index in tiles of LG_T and stages the tile's table rows and column
+// values in shared memory.  The order of each sum is the index's.
+//
+// FP64 is bound by its multiply-adds (about two per clock and SM): all lanes have
+// to hold values, and one batch item has to spread over the SMs.  So the columns
+// are cut evenly (20 stay one chunk, where fixed chunks of 16 left 38 % of the
+// lanes idle) and the values of a chunk are dealt out flat, four warps a block.
+// us at T42, 20 levels, before -> after: 32 members, analysis of two tables 559 -> 295,
+// of one 292 -> 154, synthesis (mean of three calls) 411 -> 260; one member, analysis
+// 56 -> 26, synthesis 65 -> 24.
+constexpr int LG_SMS = 152;     // SMs to fill
+constexpr int LG_NT = 128;      // threads of a block ...
+constexpr int LG_NTMAX = 512;   // ... of the synthesis of many batch items
+constexpr int LG_T = 32;        // summation indices per staged tile
+constexpr int LG_CMAX = 32;     // columns of a chunk at most
+
+inline int leg_cols(int C) {
+  const int n = (C + LG_CMAX - 1) / LG_CMAX;
+  return (C + n - 1) / n;
+}
+// Rows (n or j, of nrow) that nt consecutive values of cc columns touch at most.
+LBM_HD int leg_rows(int cc, int nrow, int nt) {
+  const int r = (nt + cc - 2) / cc + 1;
+  return r < nrow ? r : nrow;
+}
+
+template <typename R> size_t leg_smem1(int cc, int nrow, int nt) {
+  return 2 * (sizeof(C2<R>) * LG_T * (size_t)cc + sizeof(R) * leg_rows(cc, nrow, nt) * (LG_T + 1));
+}
+// Largest over the full chunks and the last one.
+template <typename R> size_t leg_smem(int C, int CC, int nrow, int nt) {
+  const size_t a = leg_smem1<R>(CC, nrow, nt),
+               b = leg_smem1<R>(C - (C - 1) / CC * CC, nrow, nt);
+  return a > b ? a : b;
+}
 
 // spec[b][m][n][c] (+)= nfac[n] (ca sum_j ta f_a + sb cb sum_j tb f_b)
 template <typename R>
-__global__ void __launch_bounds__(LG_COLS * LG_ROWS)
-k_leg_anal(int M, int J, int C, const C2<R>* __restrict__ fa, const R* __restrict__ ta,
-           int ima, const C2<R>* __restrict__ fb, const R* __restrict__ tb, int imb, R sb,
-           const R* __restrict__ nfac, int accumulate, C2<R>* __restrict__ spec) {
-  extern __shared__ unsigned char smraw[];
-  C2<R>* sa = reinterpret_cast<C2<R>*>(smraw);   // [J][LG_COLS]
-  C2<R>* sbb = sa + J * LG_COLS;
-  const int m = blockIdx.x, b = blockIdx.y, c0 = blockIdx.z * LG_COLS;
-  const int cc = min(LG_COLS, C - c0);
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * LG_COLS + tx;
-  for (int idx = tid; idx < J * LG_COLS; idx += LG_COLS * LG_ROWS) {
-    const int jj = idx / LG_COLS, c = idx % LG_COLS;
-    const size_t g = (((size_t)b * M + m) * J + jj) * C + c0 + c;
-    sa[idx] = (c < cc) ? fa[g] : cmk<R>(0, 0);
-    if (fb) sbb[idx] = (c < cc) ? fb[g] : cmk<R>(0, 0);
+__global__ void __launch_bounds__(LG_NT)
+k_leg_anal(int M, int J, int C, int CC, int nch, const C2<R>* __restrict__ fa,
+           const R* __restrict__ ta, int ima, const C2<R>* __restrict__ fb,
+           const R* __restrict__ tb, int imb, R sb, const R* __restrict__ nfac, int accumulate,
+           C2<R>* __restrict__ spec) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  constexpr int TS = LG_T + 1;
+  C2<R>* xs = reinterpret_cast<C2<R>*>(smraw);           // [2][LG_T][cc]
+  const int m = blockIdx.x, b = blockIdx.y;
+  const int ch = blockIdx.z % nch, part = blockIdx.z / nch;
+  const int c0 = ch * CC, cc = min(CC, C - c0), RR = leg_rows(cc, M, LG_NT);
+  R* ts = reinterpret_cast<R*>(xs + 2 * LG_T * cc);      // [2][RR][TS]
+  const int tid = threadIdx.x, v0 = part * LG_NT, v = v0 + tid;
+  C2<R>* out = spec + ((size_t)b * M + m) * M * C + c0;
+  if (!accumulate && v < m * cc) {                       // n < m: zeros
+    const int n = v / cc;
+    out[(size_t)n * C + v - n * cc] = cmk<R>(0, 0);
   }
-  __syncthreads();
-  if (tx >= cc) return;
-  const R mm = R(m);
-  for (int n = ty; n < M; n += LG_ROWS) {
-    const size_t o = (((size_t)b * M + m) * M + n) * C + c0 + tx;
-    if (n < m) {
-      if (!accumulate) spec[o] = cmk<R>(0, 0);
-      continue;
+  const int nval = (M - m) * cc;
+  if (v0 >= nval) return;
+  const bool act = v < nval;
+  const int row = act ? v / cc : 0, c = act ? v - row * cc : 0, n = m + row;
+  const int r0 = v0 / cc, nr = min(RR, M - m - r0);
+  const C2<R>* ga = fa + ((size_t)b * M + m) * J * C + c0;
+  const C2<R>* gb = fb ? fb + ((size_t)b * M + m) * J * C + c0 : nullptr;
+  const size_t trow = ((size_t)m * M + m + r0) * J;
+  C2<R> acc = cmk<R>(0, 0), accb = cmk<R>(0, 0);
+  for (int j0 = 0; j0 < J; j0 += LG_T) {
+    const int nj = min(LG_T, J - j0);
+    __syncthreads();
+    for (int x = tid; x < nj * cc; x += LG_NT) {
+      const int jj = x / cc, q = x - jj * cc;
+      const size_t g = (size_t)(j0 + jj) * C + q;
+      xs[jj * cc + q] = ga[g];
+      if (gb) xs[(LG_T + jj) * cc + q] = gb[g];
     }
-    const R* pa = ta + ((size_t)m * M + n) * J;
-    C2<R> acc = cmk<R>(0, 0), accb = cmk<R>(0, 0);
-    for (int jj = 0; jj < J; ++jj) cfma(acc, pa[jj], sa[jj * LG_COLS + tx]);
-    if (ima) acc = im_mul(acc, mm);
-    if (fb) {
-      const R* pb = tb + ((size_t)m * M + n) * J;
-      for (int jj = 0; jj < J; ++jj) cfma(accb, pb[jj], sbb[jj * LG_COLS + tx]);
-      if (imb) accb = im_mul(accb, mm);
-      acc = acc + accb * sb;
-    }
-    if (nfac) acc = acc * nfac[n];
-    if (accumulate) acc = acc + spec[o];
-    spec[o] = acc;
-  }
-}
-
-// four[b][m][j][c] = sum_n ta[m][n][j] ca na[n] sa + sb sum_n tb cb nb[n] sb_
-template <typename R>
-__global__ void __launch_bounds__(LG_COLS * LG_ROWS)
-k_leg_synth(int M, int J, int C, const C2<R>* __restrict__ sa, const R* __restrict__ ta,
-            int ima, const R* __restrict__ na, const C2<R>* __restrict__ sbp,
-            const R* __restrict__ tb, int imb, const R* __restrict__ nb, R sb,
-            C2<R>* __restrict__ four) {
-  extern __shared__ unsigned char smraw[];
-  C2<R>* xa = reinterpret_cast<C2<R>*>(smraw);   // [M][LG_COLS]
-  C2<R>* xb = xa + M * LG_COLS;
-  const int m = blockIdx.x, b = blockIdx.y, c0 = blockIdx.z * LG_COLS;
-  const int cc = min(LG_COLS, C - c0);
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * LG_COLS + tx;
-  const R mm = R(m);
-  for (int idx = tid; idx < M * LG_COLS; idx += LG_COLS * LG_ROWS) {
-    const int n = idx / LG_COLS, c = idx % LG_COLS;
-    C2<R> va = cmk<R>(0, 0), vb = cmk<R>(0, 0);
-    if (c < cc && n >= m) {
-      const size_t g = (((size_t)b * M + m) * M + n) * C + c0 + c;
-      va = sa[g];
-      if (ima) va = im_mul(va, mm);
-      if (na) va = va * na[n];
-      if (sbp) {
-        vb = sbp[g];
-        if (imb) vb = im_mul(vb, mm);
-        if (nb) vb = vb * nb[n];
-        vb = vb * sb;
+    for (int x = tid; x < nr * LG_T; x += LG_NT) {
+      const int r = x / LG_T, jj = x % LG_T;
+      if (jj < nj) {
+        ts[r * TS + jj] = ta[trow + (size_t)r * J + j0 + jj];
+        if (gb) ts[(RR + r) * TS + jj] = tb[trow + (size_t)r * J + j0 + jj];
       }
     }
-    xa[idx] = va;
-    xb[idx] = vb;
-  }
-  __syncthreads();
-  if (tx >= cc) return;
-  for (int jj = ty; jj < J; jj += LG_ROWS) {
-    C2<R> acc = cmk<R>(0, 0);
-    for (int n = m; n < M; ++n) {
-      cfma(acc, ta[((size_t)m * M + n) * J + jj], xa[n * LG_COLS + tx]);
-      if (sbp) cfma(acc, tb[((size_t)m * M + n) * J + jj], xb[n * LG_COLS + tx]);
+    __syncthreads();
+    const C2<R>* x = xs + c;
+    const R* t = ts + (row - r0) * TS;
+    if (!act) continue;
+    if (gb) {
+#pragma unroll 4
+      for (int jj = 0; jj < nj; ++jj) {
+        cfma(acc, t[jj], x[jj * cc]);
+        cfma(accb, t[RR * TS + jj], x[(LG_T + jj) * cc]);
+      }
+    } else {
+#pragma unroll 4
+      for (int jj = 0; jj < nj; ++jj) cfma(acc, t[jj], x[jj * cc]);
     }
-    four[(((size_t)b * M + m) * J + jj) * C + c0 + tx] = acc;
   }
+  if (!act) return;
+  const R mm = R(m);
+  if (ima) acc = im_mul(acc, mm);
+  if (fb) {
+    if (imb) accb = im_mul(accb, mm);
+    acc = acc + accb * sb;
+  }
+  if (nfac) acc = acc * nfac[n];
+  C2<R>* o = out + (size_t)n * C + c;
+  if (accumulate) acc = acc + *o;
+  *o = acc;
+}
+
+// (the factors of the staged coefficients are FP64 products too: large batches take
+// LG_NTMAX values a block to stage less often: 32 members 400 -> 313 us)
+// four[b][m][j][c] = sum_n ta[m][n][j] ca na[n] sa + sb sum_n tb cb nb[n] sb_
+template <typename R>
+__global__ void __launch_bounds__(LG_NTMAX)
+k_leg_synth(int M, int J, int C, int CC, int nch, const C2<R>* __restrict__ sa,
+            const R* __restrict__ ta, int ima, const R* __restrict__ na,
+            const C2<R>* __restrict__ sbp, const R* __restrict__ tb, int imb,
+            const R* __restrict__ nb, R sb, C2<R>* __restrict__ four) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C2<R>* xs = reinterpret_cast<C2<R>*>(smraw);           // [2][LG_T][cc]
+  const int m = blockIdx.x, b = blockIdx.y;
+  const int ch = blockIdx.z % nch, part = blockIdx.z / nch;
+  const int c0 = ch * CC, cc = min(CC, C - c0), NT = blockDim.x,
+            RR = leg_rows(cc, J, NT);
+  R* ts = reinterpret_cast<R*>(xs + 2 * LG_T * cc);      // [2][LG_T][RR]
+  const int tid = threadIdx.x, v0 = part * NT, v = v0 + tid, nval = J * cc;
+  if (v0 >= nval) return;
+  const bool act = v < nval;
+  const int jj = act ? v / cc : 0, c = act ? v - jj * cc : 0;
+  const int r0 = v0 / cc, nr = min(RR, J - r0);
+  const R mm = R(m);
+  C2<R> acc = cmk<R>(0, 0);
+  for (int n0 = m; n0 < M; n0 += LG_T) {
+    const int nn = min(LG_T, M - n0);
+    __syncthreads();
+    for (int x = tid; x < nn * cc; x += NT) {
+      const int y = x / cc, q = x - y * cc, n = n0 + y;
+      const size_t g = (((size_t)b * M + m) * M + n) * C + c0 + q;
+      C2<R> va = sa[g];
+      if (ima) va = im_mul(va, mm);
+      if (na) va = va * na[n];
+      xs[y * cc + q] = va;
+      if (sbp) {
+        C2<R> vb = sbp[g];
+        if (imb) vb = im_mul(vb, mm);
+        if (nb) vb = vb * nb[n];
+        xs[(LG_T + y) * cc + q] = vb * sb;
+      }
+    }
+    for (int x = tid; x < nn * nr; x += NT) {
+      const int y = x / nr, r = x - y * nr;
+      const size_t g = ((size_t)m * M + n0 + y) * J + r0 + r;
+      ts[y * RR + r] = ta[g];
+      if (sbp) ts[(LG_T + y) * RR + r] = tb[g];
+    }
+    __syncthreads();
+    const C2<R>* x = xs + c;
+    const R* t = ts + (jj - r0);
+    if (!act) continue;
+    if (sbp) {
+#pragma unroll 4
+      for (int y = 0; y < nn; ++y) {
+        cfma(acc, t[y * RR], x[y * cc]);
+        cfma(acc, t[(LG_T + y) * RR], x[(LG_T + y) * cc]);
+      }
+    } else {
+#pragma unroll 4
+      for (int y = 0; y < nn; ++y) cfma(acc, t[y * RR], x[y * cc]);
+    }
+  }
+  if (act) four[(((size_t)b * M + m) * J + jj) * C + c0 + c] = acc;
 }
 
 template <typename R, int I>
@@ -210,6 +295,12 @@ int fourier_dispatch(bool fwd, int B, int J, int I, int C, int nmax, const void*
   }
 }
 
+// The kernel's dynamic shared memory limit: always the same value, since other
+// threads and captured launches rely on it with sizes of their own.
+template <typename F> void leg_allow(F kern) {
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+
 template <typename R>
 static int leg_anal(int B, int nmax, int J, int C, const void* fa, const void* ta, int ima,
                     const void* fb, const void* tb, int imb, double sb, const void* nfac,
@@ -217,12 +308,13 @@ static int leg_anal(int B, int nmax, int J, int C, const void* fa, const void* t
   const int M = nmax + 1;
   if (B < 1 || M < 1 || J < 2 || C < 1 || !fa || !ta || !spec || (fb && !tb))
     return LBM_ERR_ARG;
-  const size_t smem = sizeof(C2<R>) * 2 * J * LG_COLS;
-  cudaFuncSetAttribute(k_leg_anal<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dim3 grid(M, B, (C + LG_COLS - 1) / LG_COLS), block(LG_COLS, LG_ROWS);
-  k_leg_anal<R><<<grid, block, smem, st>>>(M, J, C, (const C2<R>*)fa, (const R*)ta, ima,
-                                           (const C2<R>*)fb, (const R*)tb, imb, R(sb),
-                                           (const R*)nfac, acc, (C2<R>*)spec);
+  const int CC = leg_cols(C), nch = (C + CC - 1) / CC;
+  const dim3 grid(M, B, nch * ((M * CC + LG_NT - 1) / LG_NT));
+  const size_t smem = leg_smem<R>(C, CC, M, LG_NT);
+  leg_allow(k_leg_anal<R>);
+  k_leg_anal<R><<<grid, LG_NT, smem, st>>>(
+      M, J, C, CC, nch, (const C2<R>*)fa, (const R*)ta, ima, (const C2<R>*)fb, (const R*)tb, imb,
+      R(sb), (const R*)nfac, acc, (C2<R>*)spec);
   LBM_LAUNCH_CHECK();
   return LBM_OK;
 }
@@ -234,12 +326,15 @@ static int leg_synth(int B, int nmax, int J, int C, const void* sa, const void* 
   const int M = nmax + 1;
   if (B < 1 || M < 1 || J < 2 || C < 1 || !sa || !ta || !four || (sbp && !tb))
     return LBM_ERR_ARG;
-  const size_t smem = sizeof(C2<R>) * 2 * M * LG_COLS;
-  cudaFuncSetAttribute(k_leg_synth<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dim3 grid(M, B, (C + LG_COLS - 1) / LG_COLS), block(LG_COLS, LG_ROWS);
-  k_leg_synth<R><<<grid, block, smem, st>>>(M, J, C, (const C2<R>*)sa, (const R*)ta, ima,
-                                            (const R*)na, (const C2<R>*)sbp, (const R*)tb,
-                                            imb, (const R*)nb, R(sb), (C2<R>*)four);
+  const int CC = leg_cols(C), nch = (C + CC - 1) / CC;
+  const int big = (J * CC + LG_NTMAX - 1) / LG_NTMAX;
+  const int nt = (long)M * B * nch * big >= 8 * LG_SMS ? LG_NTMAX : LG_NT;
+  const dim3 grid(M, B, nch * ((J * CC + nt - 1) / nt));
+  const size_t smem = leg_smem<R>(C, CC, J, nt);
+  leg_allow(k_leg_synth<R>);
+  k_leg_synth<R><<<grid, nt, smem, st>>>(
+      M, J, C, CC, nch, (const C2<R>*)sa, (const R*)ta, ima, (const R*)na, (const C2<R>*)sbp,
+      (const R*)tb, imb, (const R*)nb, R(sb), (C2<R>*)four);
   LBM_LAUNCH_CHECK();
   return LBM_OK;
 }

@@ -321,3 +321,94 @@ def test_implicit_kernel_against_fp64_formula(torch, I, J, N, K, nmem, vdiff, pr
     for v, f in zip(views[:2], first):
         assert torch.equal(v, torch.view_as_real(f).reshape(-1))
     assert torch.equal(stp.sas, first[2])
+
+
+@pytest.mark.parametrize("B,J,N,C", [(1, 64, 42, 20), (1, 6, 3, 1), (2, 50, 31, 17), (1, 64, 42, 35),
+                                     (3, 34, 21, 40), (1, 128, 85, 65), (1, 64, 42, 1),
+                                     (40, 64, 42, 21), (1, 64, 42, 1000)])
+@pytest.mark.parametrize("two", [False, True])
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_legendre_api_against_fp64_sums(torch, B, J, N, C, two, dtype):
+    """The Legendre sums of the transform API over column chunks with
+    remainders, one column, row tiles that end early and both block sizes, on
+    tables without symmetry.  Bound per value: (terms + 8) u times the sum of
+    the products' magnitudes."""
+    import lbm_isca_gb300.ops      # noqa: F401  (registers the operators)
+    rt = getattr(torch, dtype)
+    ct = torch.complex64 if dtype == "float32" else torch.complex128
+    u, M = torch.finfo(rt).eps / 2, N + 1
+    g = torch.Generator(device="cuda").manual_seed(B + J + C)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda", dtype=torch.float64)   # noqa: E731
+    ta, tb = rnd(M, M, J).to(rt), rnd(M, M, J).to(rt)
+    fac = [rnd(M).to(rt) for _ in range(3)]
+    field = lambda *s: torch.view_as_complex(rnd(*s, 2)).to(ct)     # noqa: E731
+    m = torch.arange(M, device="cuda", dtype=torch.float64)[None, :, None, None]
+    tri = (torch.arange(M, device="cuda")[None, :] >= torch.arange(M, device="cuda")[:, None])
+    D = lambda x: x.to(torch.complex128 if x.is_complex() else torch.float64)   # noqa: E731
+
+    def mul(eq, T, X):
+        return torch.complex(torch.einsum(eq, D(T), D(X).real.contiguous()),
+                             torch.einsum(eq, D(T), D(X).imag.contiguous()))
+
+    def check(got, want, size, terms):
+        err = torch.view_as_real(D(got) - want).abs().amax(-1)
+        assert bool((err <= (terms + 8) * u * size + 1e-300).all())
+
+    fa, fb = field(B, M, J, C), field(B, M, J, C)
+    got = torch.ops.lbm_gb300.legendre_analysis(fa, ta, 1, fb if two else None,
+                                                tb if two else None, 0, -1.5, fac[0])
+    A = lambda T, X: mul("mnj,bmjc->bmnc", T, X)         # noqa: E731
+    Z = lambda T, X: torch.einsum("mnj,bmjc->bmnc", D(T).abs(), D(X).abs())   # noqa: E731
+    want, size = 1j * m * A(ta, fa), m * Z(ta, fa)
+    if two:
+        want, size = want - 1.5 * A(tb, fb), size + 1.5 * Z(tb, fb)
+    nf = D(fac[0])[None, None, :, None] * tri[None, :, :, None]
+    check(got, want * nf, size * nf.abs(), 2 * J)
+
+    sa, sb = field(B, M, M, C), field(B, M, M, C)
+    got = torch.ops.lbm_gb300.legendre_synthesis(sa, ta, 0, fac[1], sb if two else None,
+                                                 tb if two else None, 1, fac[2], 0.5)
+    tr = tri[None, :, :, None]
+    S = lambda T, X: mul("mnj,bmnc->bmjc", T, X)         # noqa: E731
+    Q = lambda T, X: torch.einsum("mnj,bmnc->bmjc", D(T).abs(), D(X).abs())   # noqa: E731
+    x = D(sa) * D(fac[1])[None, None, :, None] * tr
+    want, size = S(ta, x), Q(ta, x)
+    if two:
+        x = 0.5j * m * D(sb) * D(fac[2])[None, None, :, None] * tr
+        want, size = want + S(tb, x), size + Q(tb, x)
+    check(got, want, size, 2 * M)
+
+
+@pytest.mark.parametrize("K", [2, 7, 20, 64])
+@pytest.mark.parametrize("linear", [False, True])
+def test_tendency_kernel_against_oracle(torch, K, linear):
+    """Grid tendencies at level counts that divide a block's threads and that
+    do not, against the oracle (as at 20 levels: 1e-10 of the largest value)."""
+    import types
+    from lbm_isca_gb300 import LBM, Config, Spectral, VerticalGrid
+    from oracle import lbm_oracle as orc
+    from lbm_isca_gb300.state import State
+    I, J, N = 64, 32, 21
+    sigm = configs.equal_sigma_half_levels(K)
+    bs = configs.solid_body_basic_state(I, J, sigm)
+    mu, _ = configs.gaussian_latitudes(J)
+    bs.q = np.broadcast_to(0.01 * (1.0 - mu * mu)[:, None, None], bs.t.shape).copy()
+    cfg = dict(configs.plain_damping(K), strictly_linear=linear)
+    m = LBM(bs, Spectral(nlon=I, nlat=J, nmax=N, device="gb300"),
+            VerticalGrid(sigm=sigm, device="gb300"), Config(**cfg))
+    tr, lv = orc.SphericalTransform(I, J, N), orc.SigmaLevels(sigm)
+    om = orc.OracleModel(tr, lv, bs, orc.RunConfig(**cfg))
+    rng = np.random.default_rng(K)
+    u, v = tr.vordiv_to_uv(*tr.uv_to_vordiv(*rng.normal(size=(2, J, I, K))))
+    wave = lambda x: tr.wave_to_grid(tr.grid_to_wave(x))          # noqa: E731
+    f = types.SimpleNamespace(u=u, v=v, t=wave(rng.normal(size=(J, I, K))),
+                              q=wave(1e-3 * rng.normal(size=(J, I, K))),
+                              ps=0.5 * wave(rng.normal(size=(J, I))))
+    heat = configs.elliptic_heating(I, J, sigm)
+    got = m.dyn.tendencies(State(bs.ps, u=f.u, v=f.v, t=f.t, q=f.q, ps=f.ps, device="gb300"),
+                           frc_t=heat)
+    ref = orc.tendencies(tr, lv, om.bt, orc.GridState(np.asarray(bs.ps), f.u, f.v, f.t, f.q, f.ps),
+                         frc_t=heat, strictly_linear=linear)
+    for a, b in zip(got, ref):
+        a = a.detach().cpu().numpy()
+        assert np.abs(a - b).max() < 1e-10 * np.abs(b).max()
