@@ -9,20 +9,25 @@
 
 namespace lbm {
 
-// 32-thread blocks: one member's columns (8192 at T42) or coefficients
-// (3698) spread over all SMs instead of filling a few.
-constexpr int ADJ_THREADS = 32;
+// One thread per (column, level) and per (coefficient, level), ADJ_THREADS / K
+// columns a block, the column's exchanges in shared memory.  Both are bound by the
+// latency of a column's chain and the FP64 pipe: with one thread per column and
+// its level arrays in local memory, one member of T42 filled 256 and 116 warps.
+// At T42, 20 levels, one member, FP64: tendencies 239 -> 84 us, implicit update 146 -> 24.
+constexpr int ADJ_THREADS = 256;
 
-// One thread per grid column (member, latitude, longitude).
-template <typename R, int KM>
+template <typename R>
 __global__ void __launch_bounds__(ADJ_THREADS) k_tendency_grid_adj(lbm_tend_adj_args a) {
-  const int J = a.nlat, I = a.nlon, K = a.kmax;
-  const size_t col = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int J = a.nlat, I = a.nlon, K = a.kmax, CB = ADJ_THREADS / K;
+  __shared__ R sgt[ADJ_THREADS], ske[ADJ_THREADS], ssa[ADJ_THREADS], ssb[ADJ_THREADS];
+  __shared__ R spx[ADJ_THREADS], spy[ADJ_THREADS];
   const size_t ncol2 = (size_t)J * I;
-  if (col >= (size_t)a.nmem * ncol2) return;
-  const size_t ji = col % ncol2;
+  const int tid = threadIdx.x, cl = tid / K, k = tid - cl * K, cK = cl * K;
+  const size_t col = (size_t)blockIdx.x * CB + cl;
+  const bool act = cl < CB && col < (size_t)a.nmem * ncol2;
+  const size_t ji = act ? col % ncol2 : 0;
   auto P = [](const void* p) { return (const R*)p; };
-  const size_t b3 = ji * K, p3 = col * K;
+  const size_t b3 = ji * K, p3 = (act ? col : 0) * K;
   lbm_adj::ColConst<R> c;
   c.K = K;
   c.kappa = R(a.kappa);
@@ -50,50 +55,62 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_tendency_grid_adj(lbm_tend_adj_
   c.piyb = P(a.piyb)[ji];
   c.u0 = a.u0 ? P(a.u0) + p3 : nullptr;
   c.v0 = a.v0 ? P(a.v0) + p3 : nullptr;
-  R work[5 * (KM + 1)];
-  // the adjoints are accumulated level by level (K x K scatters of the
-  // hydrostatic and tmtx transposes, the vertical-advection transposes):
-  // into thread-local arrays, whose elements the hardware interleaves across
-  // the threads of a warp, and written to the level-strided outputs once
-  R lu[KM], lv[KM], lt[KM], lq[KM], lvor[KM], ldiv[KM];
-  lbm_adj::tendency_column_adjoint<R>(
-      c, P(a.a_fu) + p3, P(a.a_fv) + p3, P(a.a_ke) + p3, P(a.a_gt) + p3, P(a.a_xu) + p3,
-      P(a.a_xv) + p3, P(a.a_g) + p3, P(a.a_yu) + p3, P(a.a_yv) + p3, P(a.a_gt_pi)[col],
-      lu, lv, lt, lq, lvor, ldiv, (R*)a.a_pix + col, (R*)a.a_piy + col, work);
-  R *ou = (R*)a.a_u + p3, *ov = (R*)a.a_v + p3, *ot = (R*)a.a_t + p3, *oq = (R*)a.a_q + p3,
-    *ovor = (R*)a.a_vor + p3, *odiv = (R*)a.a_div + p3;
-  for (int k = 0; k < K; ++k) {
-    ou[k] = lu[k];
-    ov[k] = lv[k];
-    ot[k] = lt[k];
-    oq[k] = lq[k];
-    ovor[k] = lvor[k];
-    odiv[k] = ldiv[k];
+  const lbm_adj::TendAdjIn<R> y = {P(a.a_fu) + p3, P(a.a_fv) + p3, P(a.a_ke) + p3,
+                                   P(a.a_gt) + p3, P(a.a_xu) + p3, P(a.a_xv) + p3,
+                                   P(a.a_g) + p3,  P(a.a_yu) + p3, P(a.a_yv) + p3,
+                                   act ? P(a.a_gt_pi)[col] : R(0)};
+  if (act) {
+    sgt[tid] = y.gt[k];
+    ske[tid] = y.ke[k];
+    lbm_adj::tendency_adj_sums(c, y, k, ssa + tid, ssb + tid);
+  }
+  __syncthreads();
+  lbm_adj::TendAdjOut<R> o = {};
+  if (act) {
+    R cum = R(0);
+    for (int l = 1; l < K; ++l) cum += ssb[cK + l];
+    for (int l = 1; l <= k; ++l) cum += ssa[cK + l];
+    o = lbm_adj::tendency_adj_level(c, y, k, cum, sgt + cK, ske + cK);
+    spx[tid] = o.px;
+    spy[tid] = o.py;
+  }
+  __syncthreads();                     // outputs may take the place of inputs
+  if (act) {
+    ((R*)a.a_u)[p3 + k] = o.u;
+    ((R*)a.a_v)[p3 + k] = o.v;
+    ((R*)a.a_t)[p3 + k] = o.t;
+    ((R*)a.a_q)[p3 + k] = o.q;
+    ((R*)a.a_vor)[p3 + k] = o.vor;
+    ((R*)a.a_div)[p3 + k] = o.div;
+  }
+  // column sums: pi_x, then pi_y
+  for (int x = tid; x < 2 * CB; x += ADJ_THREADS) {
+    const int q = x % CB;
+    const size_t cq = (size_t)blockIdx.x * CB + q;
+    if (cq >= (size_t)a.nmem * ncol2) continue;
+    const R* sp = (x < CB ? spx : spy) + q * K;
+    R s = R(0);
+    for (int l = 0; l < K; ++l) s += sp[l];
+    ((R*)(x < CB ? a.a_pix : a.a_piy))[cq] = s;
   }
 }
 
-// One thread per (member, m, n, real/imaginary part).
-template <typename R, int KM>
+template <typename R>
 __global__ void __launch_bounds__(ADJ_THREADS) k_implicit_adj(lbm_implicit_adj_args a) {
-  const int K = a.kmax, M = a.nmax + 1;
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t total = (size_t)a.nmem * M * M * 2;
-  if (idx >= total) return;
-  const int comp = (int)(idx & 1);
-  const size_t coef = idx >> 1;                 // (e, m, n)
-  const int n = (int)(coef % M), m = (int)((coef / M) % M);
+  using V = C2<R>;
+  const int K = a.kmax, M = a.nmax + 1, CB = ADJ_THREADS / K;
+  __shared__ V sh[4][ADJ_THREADS];
+  const int tid = threadIdx.x, cl = tid / K, l = tid - cl * K, cK = cl * K;
+  const size_t coef = (size_t)blockIdx.x * CB + cl;             // (e, m, n)
+  const bool in = cl < CB && coef < (size_t)a.nmem * M * M;
+  const int n = in ? (int)(coef % M) : 0, m = in ? (int)((coef / M) % M) : 0;
+  const bool act = in && n >= m;
+  const V z = cmk<R>(0, 0);
+  const size_t o3 = (in ? coef : 0) * K + l, o2 = in ? coef : 0;
   auto P = [](const void* p) { return (const R*)p; };
-  const size_t o3 = coef * K * 2 + comp, o2 = coef * 2 + comp;
-  R* ap[5] = {(R*)a.ap_vor + o3, (R*)a.ap_div + o3, (R*)a.ap_t + o3, (R*)a.ap_q + o3,
-              (R*)a.ap_pi + o2};
-  R* aw[5] = {(R*)a.aw_vor + o3, (R*)a.aw_div + o3, (R*)a.aw_t + o3, (R*)a.aw_q + o3,
-              (R*)a.aw_pi + o2};
-  if (n < m) {           // outside the triangle the update writes zeros
-    for (int f = 0; f < 4; ++f)
-      for (int k = 0; k < K; ++k) ap[f][2 * k] = aw[f][2 * k] = R(0);
-    *ap[4] = *aw[4] = R(0);
-    return;
-  }
+  const void* an[4] = {a.an_vor, a.an_div, a.an_t, a.an_q};
+  void* ap[4] = {a.ap_vor, a.ap_div, a.ap_t, a.ap_q};
+  void* aw[4] = {a.aw_vor, a.aw_div, a.aw_t, a.aw_q};
   lbm_adj::ImplConst<R> c;
   c.K = K;
   c.dt = R(a.dt);
@@ -112,33 +129,58 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_implicit_adj(lbm_implicit_adj_a
   c.vd[2] = P(a.vd_t);
   c.vd[3] = P(a.vd_q);
   c.vd_skip_vordiv = n < 2;
-  R work[4 * KM];
-  lbm_adj::implicit_coef_adjoint<R>(c, 2, P(a.an_vor) + o3, P(a.an_div) + o3, P(a.an_t) + o3,
-                                    P(a.an_q) + o3, P(a.an_pi)[o2], ap[0], ap[1], ap[2], ap[3],
-                                    ap[4], aw[0], aw[1], aw[2], aw[3], aw[4], work);
+  const V anpi = act ? ((const V*)a.an_pi)[o2] : z;
+  const V awpi = anpi * (R(2) * c.dt);
+#pragma unroll
+  for (int f = 0; f < 4; ++f) sh[f][tid] = act ? ((const V*)an[f])[o3] : z;
+  __syncthreads();
+  lbm_adj::ImplAdjLevel<V> o = {};
+  if (act) {
+    V v[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) v[f] = lbm_adj::impl_adj_vdiff(c, f, sh[f] + cK, l, z);
+    lbm_adj::impl_adj_point(c, l, v, o);
+  }
+  __syncthreads();
+  sh[0][tid] = o.aw[2];
+  __syncthreads();
+  if (act) lbm_adj::impl_adj_dbar(c, l, sh[0] + cK, awpi, z, o);
+  sh[1][tid] = o.x;
+  __syncthreads();
+  V part = z;
+  if (act) part = lbm_adj::impl_adj_rhs(c, l, sh[1] + cK, z, o);
+  sh[2][tid] = o.x;
+  sh[3][tid] = part;
+  __syncthreads();
+  if (act) lbm_adj::impl_adj_wdx(c, l, sh[2] + cK, z, o);
+  if (!in) return;
+  // outside the triangle the update writes zeros
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    ((V*)ap[f])[o3] = o.ap[f];
+    ((V*)aw[f])[o3] = o.aw[f];
+  }
+  if (l == 0) {
+    V s = z;
+    for (int k = 0; k < K; ++k) s = s + sh[3][cK + k];
+    ((V*)a.ap_pi)[o2] = anpi + s;
+    ((V*)a.aw_pi)[o2] = awpi + s * c.dt;
+  }
 }
 
 template <typename R>
 static int tend_adj(const lbm_tend_adj_args* a, cudaStream_t st) {
-  const size_t cols = (size_t)a->nmem * a->nlat * a->nlon;
-  const unsigned blocks = (unsigned)((cols + ADJ_THREADS - 1) / ADJ_THREADS);
-  if (a->kmax <= 32)
-    k_tendency_grid_adj<R, 32><<<blocks, ADJ_THREADS, 0, st>>>(*a);
-  else
-    k_tendency_grid_adj<R, 64><<<blocks, ADJ_THREADS, 0, st>>>(*a);
+  const size_t cols = (size_t)a->nmem * a->nlat * a->nlon, CB = ADJ_THREADS / a->kmax;
+  k_tendency_grid_adj<R><<<(unsigned)((cols + CB - 1) / CB), ADJ_THREADS, 0, st>>>(*a);
   LBM_LAUNCH_CHECK();
   return LBM_OK;
 }
 
 template <typename R>
 static int impl_adj(const lbm_implicit_adj_args* a, cudaStream_t st) {
-  const size_t M = (size_t)a->nmax + 1;
-  const size_t total = (size_t)a->nmem * M * M * 2;
-  const unsigned blocks = (unsigned)((total + ADJ_THREADS - 1) / ADJ_THREADS);
-  if (a->kmax <= 32)
-    k_implicit_adj<R, 32><<<blocks, ADJ_THREADS, 0, st>>>(*a);
-  else
-    k_implicit_adj<R, 64><<<blocks, ADJ_THREADS, 0, st>>>(*a);
+  const size_t M = (size_t)a->nmax + 1, total = (size_t)a->nmem * M * M;
+  const size_t CB = ADJ_THREADS / a->kmax;
+  k_implicit_adj<R><<<(unsigned)((total + CB - 1) / CB), ADJ_THREADS, 0, st>>>(*a);
   LBM_LAUNCH_CHECK();
   return LBM_OK;
 }

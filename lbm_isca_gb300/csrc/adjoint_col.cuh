@@ -21,35 +21,21 @@
 
 namespace lbm_adj {
 
-// Transpose of the f-argument of the vertical advection operator
+// Transposes of the vertical advection operator at one level,
 //   VA(f; s)[k] = (fhi - flo - f[k] (s[k+1] - s[k])) / dsig[k],
 //   flo = s[k] (f[k] + f[k-1]) / 2 for k >= 1, fhi = s[k+1] (f[k+1] + f[k]) / 2
-//   for k + 1 <= K - 1 (reference dynamics.py:117-143): fbar += dVA/df^T y.
+//   for k + 1 <= K - 1 (reference dynamics.py:117-143), z = y / dsig.
+// Of the f-argument: level k of fbar = dVA/df^T y, from z at k - 1, k, k + 1.
 template <typename R>
-LBM_COL_HD void va_f_adj(int k, int K, R y, const R* s, const R* dsig, R* fbar) {
-  const R z = y / dsig[k];
-  if (k + 1 <= K - 1) {
-    const R h = R(0.5) * s[k + 1] * z;
-    fbar[k + 1] += h;
-    fbar[k] += h;
-  }
-  if (k >= 1) {
-    const R h = R(0.5) * s[k] * z;
-    fbar[k] -= h;
-    fbar[k - 1] -= h;
-  }
-  fbar[k] -= z * (s[k + 1] - s[k]);
+LBM_COL_HD R va_f_adj(int k, int K, R zm, R z, R zp, R s0, R s1) {
+  const R lo = k >= 1 ? R(0.5) * s0 * (zm - z) : R(0);
+  const R hi = k + 1 <= K - 1 ? R(0.5) * s1 * (z - zp) : R(0);
+  return lo + hi - z * (s1 - s0);
 }
 
-// Transpose of the s-argument (s has K + 1 entries).
+// Of the s-argument: half level k (1 <= k <= K - 1) of sbar = dVA/ds^T y.
 template <typename R>
-LBM_COL_HD void va_s_adj(int k, int K, R y, const R* f, const R* dsig, R* sbar) {
-  const R z = y / dsig[k];
-  if (k + 1 <= K - 1) sbar[k + 1] += R(0.5) * (f[k + 1] + f[k]) * z;
-  if (k >= 1) sbar[k] -= R(0.5) * (f[k] + f[k - 1]) * z;
-  sbar[k + 1] -= z * f[k];
-  sbar[k] += z * f[k];
-}
+LBM_COL_HD R va_s_adj(R f, R fm, R z, R zm) { return R(0.5) * (f - fm) * (z + zm); }
 
 // Vertical constants and one column of the basic state.
 template <typename R>
@@ -62,113 +48,112 @@ struct ColConst {
   const R *u0, *v0;   // linearisation trajectory of the kinetic energy, or null
 };
 
-// Adjoint of the grid-point tendency of one column.  Inputs: adjoints of
-// fu fv ke gt xu xv g yu yv (each [K]) and of gt_pi.  Outputs (overwritten):
-// adjoints of u v t q vor div ([K]) and of pi_x, pi_y.  Scratch: 5 (K + 1)
-// values in `work`.
+// Adjoints of the outputs of one column (each [K]; gt_pi: one value).
+template <typename R>
+struct TendAdjIn {
+  const R *fu, *fv, *ke, *gt, *xu, *xv, *g, *yu, *yv;
+  R gtpi;
+};
+
+// Level k of the adjoint of sigma-dot and of the column sums: sd'[k] =
+// sigm[k] S[0] - S[k] for 1 <= k <= K-1 (zero at both ends), x5'[k-1] takes w3
+// S[k].  sa: the adjoint of S[k], k >= 1; sb: this level's part of that of S[0].
+template <typename R>
+LBM_COL_HD void tendency_adj_sums(const ColConst<R>& c, const TendAdjIn<R>& y, int k, R* sa,
+                                  R* sb) {
+  *sa = *sb = R(0);
+  if (k == 0) return;
+  const R r = R(1) / c.dsig[k], rm = R(1) / c.dsig[k - 1];
+  const R asd = va_s_adj(c.tb[k], c.tb[k - 1], y.gt[k] * r, y.gt[k - 1] * rm) +
+                va_s_adj(c.ub[k], c.ub[k - 1], y.fu[k] * r, y.fu[k - 1] * rm) +
+                va_s_adj(c.vb[k], c.vb[k - 1], y.fv[k] * r, y.fv[k - 1] * rm) +
+                va_s_adj(c.qb[k], c.qb[k - 1], y.g[k] * r, y.g[k - 1] * rm);
+  *sa = -c.w3[k - 1] * c.kappa * c.tvb[k - 1] * y.gt[k - 1] - asd;
+  *sb = c.sigm[k] * asd;
+}
+
+// Adjoints of the inputs at level k: u v t q vor div and the level's parts of
+// those of pi_x, pi_y.
+template <typename R>
+struct TendAdjOut { R u, v, t, q, vor, div, px, py; };
+
+// cum: sum of the adjoints of S[0] .. S[k] (S[k] = sum_{l >= k} dsig_l (div' +
+// padv')_l); gt, ke: the column's values again, in fast memory.
+template <typename R>
+LBM_COL_HD TendAdjOut<R> tendency_adj_level(const ColConst<R>& c, const TendAdjIn<R>& y, int k,
+                                            R cum, const R* gt, const R* ke) {
+  const int K = c.K;
+  TendAdjOut<R> o;
+  const R tdev = c.tb[k] - c.tref[k], tvdev = c.tvb[k] - c.tref[k];
+  const R rcpg = c.rair * c.cpg[k];
+  const R g = gt[k], fu = y.fu[k], fv = y.fv[k], e = ke[k], ag = y.g[k];
+  const R s0 = c.sdb[k], s1 = c.sdb[k + 1];
+  const R r = R(1) / c.dsig[k], rm = k >= 1 ? R(1) / c.dsig[k - 1] : R(0),
+          rp = k + 1 <= K - 1 ? R(1) / c.dsig[k + 1] : R(0);
+  const int km = k >= 1 ? k - 1 : 0, kp = k + 1 <= K - 1 ? k + 1 : k;
+  auto vaf = [&](const R* a) {
+    return va_f_adj(k, K, a[km] * rm, a[k] * r, a[kp] * rp, s0, s1);
+  };
+  // gt: + sum_l tmtx[k][l] div'_l;  ke: sum_l ww[k][l] (tv'_l - t'_l)
+  R tm = R(0), he = R(0);
+  for (int l = 0; l < K; ++l) {
+    tm += c.tmtx[l * K + k] * gt[l];
+    he += c.ww[l * K + k] * ke[l];
+  }
+  // gt = -kappa (tv' x5b + tvb x5') + t' divb + tdev div' + VA(t'; sdb) + VA(tb; sd')
+  // fu = v' absv + vb vor' - rcpg (tv' pixb + tvdev pi_x) + VA(u'; sdb) + VA(ub; sd')
+  // fv = -u' absv - ub vor' - rcpg (tv' piyb + tvdev pi_y) + VA(v'; sdb) + VA(vb; sd')
+  const R atv = he - c.kappa * c.x5b[k] * g - rcpg * (c.pixb * fu + c.piyb * fv);
+  const R ax5 = -c.kappa * c.tvb[k] * g;
+  // x5' = alpha div' + wP padv' + w3 S[k+1];  gt_pi = -sum_k dsig padv'
+  o.div = tdev * g + tm + c.qb[k] * ag + c.alpha[k] * ax5 + c.dsig[k] * cum;
+  const R apadv = c.wP[k] * ax5 + c.dsig[k] * (cum - y.gtpi);
+  // tv' = t' (1 + eps qb) + eps tb q';  xu = u' tdev + ub t', xv = v' tdev + vb t'
+  o.t = c.divb[k] * g + vaf(y.gt) + c.ub[k] * y.xu[k] + c.vb[k] * y.xv[k] - he +
+        (R(1) + c.eps * c.qb[k]) * atv;
+  // g = q' divb + qb div' + VA(q'; sdb) + VA(qb; sd');  yu = u' qb + ub q', yv = v' qb + vb q'
+  o.q = c.ub[k] * y.yu[k] + c.vb[k] * y.yv[k] + c.divb[k] * ag + vaf(y.g) +
+        c.eps * c.tb[k] * atv;
+  // ke: u' (ub + u0) + v' (vb + v0);  padv' = u' pixb + ub pi_x + v' piyb + vb pi_y
+  o.u = tdev * y.xu[k] + vaf(y.fu) - c.absv[k] * fv + (c.ub[k] + (c.u0 ? c.u0[k] : R(0))) * e +
+        c.qb[k] * y.yu[k] + c.pixb * apadv;
+  o.v = tdev * y.xv[k] + vaf(y.fv) + c.absv[k] * fu + (c.vb[k] + (c.v0 ? c.v0[k] : R(0))) * e +
+        c.qb[k] * y.yv[k] + c.piyb * apadv;
+  o.vor = c.vb[k] * fu - c.ub[k] * fv;
+  o.px = c.ub[k] * apadv - rcpg * tvdev * fu;
+  o.py = c.vb[k] * apadv - rcpg * tvdev * fv;
+  return o;
+}
+
+// Adjoint of the grid-point tendency of one column, level after level.  Inputs:
+// adjoints of fu fv ke gt xu xv g yu yv (each [K]) and of gt_pi.  Outputs
+// (overwritten): adjoints of u v t q vor div ([K]) and of pi_x, pi_y.  Scratch:
+// 5 (K + 1) values in `work`.
 template <typename R>
 LBM_COL_HD void tendency_column_adjoint(const ColConst<R>& c, const R* afu, const R* afv,
                                         const R* ake, const R* agt, const R* axu,
                                         const R* axv, const R* ag, const R* ayu,
                                         const R* ayv, R agtpi, R* au, R* av, R* at, R* aq,
                                         R* avor, R* adiv, R* apix, R* apiy, R* work) {
-  const int K = c.K;
-  R* atv = work;                 // adjoint of tv' [K]
-  R* ax5 = atv + (K + 1);        // adjoint of the omega factor x5' [K]
-  R* apadv = ax5 + (K + 1);      // adjoint of v'.grad(ln ps) terms [K]
-  R* aS = apadv + (K + 1);       // adjoint of the column sums S [K+1]
-  R* asd = aS + (K + 1);         // adjoint of sigma-dot [K+1]
-  for (int k = 0; k <= K; ++k) {
-    atv[k] = ax5[k] = apadv[k] = aS[k] = asd[k] = R(0);
+  const TendAdjIn<R> y = {afu, afv, ake, agt, axu, axv, ag, ayu, ayv, agtpi};
+  R cum = R(0), sb;
+  for (int k = 0; k < c.K; ++k) {
+    tendency_adj_sums(c, y, k, work + k, &sb);
+    cum += sb;
   }
-  for (int k = 0; k < K; ++k) au[k] = av[k] = at[k] = aq[k] = avor[k] = adiv[k] = R(0);
-  R px = R(0), py = R(0);
-  for (int k = 0; k < K; ++k) {
-    const R tdev = c.tb[k] - c.tref[k], tvdev = c.tvb[k] - c.tref[k];
-    const R rcpg = c.rair * c.cpg[k];
-    // gt = -kappa (tv' x5b + tvb x5') + t' divb + tdev div' + VA(t'; sdb)
-    //      + VA(tb; sd') + sum_l tmtx[k][l] div'_l
-    const R g = agt[k];
-    atv[k] -= c.kappa * c.x5b[k] * g;
-    ax5[k] -= c.kappa * c.tvb[k] * g;
-    at[k] += c.divb[k] * g;
-    adiv[k] += tdev * g;
-    va_f_adj(k, K, g, c.sdb, c.dsig, at);
-    va_s_adj(k, K, g, c.tb, c.dsig, asd);
-    for (int l = 0; l < K; ++l) adiv[l] += c.tmtx[k * K + l] * g;
-    // xu = u' tdev + ub t', xv = v' tdev + vb t'
-    au[k] += tdev * axu[k];
-    at[k] += c.ub[k] * axu[k];
-    av[k] += tdev * axv[k];
-    at[k] += c.vb[k] * axv[k];
-    // fu = v' absv + vb vor' - rcpg (tv' pixb + tvdev pi_x) + VA(u'; sdb) + VA(ub; sd')
-    R f = afu[k];
-    av[k] += c.absv[k] * f;
-    avor[k] += c.vb[k] * f;
-    atv[k] -= rcpg * c.pixb * f;
-    px -= rcpg * tvdev * f;
-    va_f_adj(k, K, f, c.sdb, c.dsig, au);
-    va_s_adj(k, K, f, c.ub, c.dsig, asd);
-    // fv = -u' absv - ub vor' - rcpg (tv' piyb + tvdev pi_y) + VA(v'; sdb) + VA(vb; sd')
-    f = afv[k];
-    au[k] -= c.absv[k] * f;
-    avor[k] -= c.ub[k] * f;
-    atv[k] -= rcpg * c.piyb * f;
-    py -= rcpg * tvdev * f;
-    va_f_adj(k, K, f, c.sdb, c.dsig, av);
-    va_s_adj(k, K, f, c.vb, c.dsig, asd);
-    // ke = sum_l ww[k][l] (tv'_l - t'_l) + u' (ub + u0) + v' (vb + v0)
-    const R e = ake[k];
-    for (int l = 0; l < K; ++l) {
-      atv[l] += c.ww[k * K + l] * e;
-      at[l] -= c.ww[k * K + l] * e;
-    }
-    au[k] += (c.ub[k] + (c.u0 ? c.u0[k] : R(0))) * e;
-    av[k] += (c.vb[k] + (c.v0 ? c.v0[k] : R(0))) * e;
-    // yu = u' qb + ub q', yv = v' qb + vb q'
-    au[k] += c.qb[k] * ayu[k];
-    aq[k] += c.ub[k] * ayu[k];
-    av[k] += c.qb[k] * ayv[k];
-    aq[k] += c.vb[k] * ayv[k];
-    // g = q' divb + qb div' + VA(q'; sdb) + VA(qb; sd')
-    f = ag[k];
-    aq[k] += c.divb[k] * f;
-    adiv[k] += c.qb[k] * f;
-    va_f_adj(k, K, f, c.sdb, c.dsig, aq);
-    va_s_adj(k, K, f, c.qb, c.dsig, asd);
-    // gt_pi = -sum_k dsig padv'
-    apadv[k] -= c.dsig[k] * agtpi;
+  *apix = *apiy = R(0);
+  for (int k = 0; k < c.K; ++k) {
+    cum += work[k];
+    const TendAdjOut<R> o = tendency_adj_level(c, y, k, cum, agt, ake);
+    au[k] = o.u;
+    av[k] = o.v;
+    at[k] = o.t;
+    aq[k] = o.q;
+    avor[k] = o.vor;
+    adiv[k] = o.div;
+    *apix += o.px;
+    *apiy += o.py;
   }
-  for (int k = 0; k < K; ++k) {
-    // tv' = t' (1 + eps qb) + eps tb q'
-    at[k] += (R(1) + c.eps * c.qb[k]) * atv[k];
-    aq[k] += c.eps * c.tb[k] * atv[k];
-    // x5' = alpha div' + wP padv' + w3 S[k+1]
-    adiv[k] += c.alpha[k] * ax5[k];
-    apadv[k] += c.wP[k] * ax5[k];
-    aS[k + 1] += c.w3[k] * ax5[k];
-  }
-  // sd'[k] = sigm[k] S[0] - S[k] for 1 <= k <= K-1 (zero at both ends)
-  for (int k = 1; k < K; ++k) {
-    aS[0] += c.sigm[k] * asd[k];
-    aS[k] -= asd[k];
-  }
-  // S[k] = sum_{l >= k} dsig_l (div' + padv')_l ; S[K] = 0
-  R cum = R(0);
-  for (int l = 0; l < K; ++l) {
-    cum += aS[l];
-    adiv[l] += c.dsig[l] * cum;
-    apadv[l] += c.dsig[l] * cum;
-  }
-  // padv' = u' pixb + ub pi_x + v' piyb + vb pi_y
-  for (int k = 0; k < K; ++k) {
-    au[k] += c.pixb * apadv[k];
-    av[k] += c.piyb * apadv[k];
-    px += c.ub[k] * apadv[k];
-    py += c.vb[k] * apadv[k];
-  }
-  *apix = px;
-  *apiy = py;
 }
 
 // Operators of the implicit update for one total wavenumber n.
@@ -182,10 +167,77 @@ struct ImplConst {
   bool vd_skip_vordiv;                        // n < 2: no vertical diffusion of vor, div
 };
 
-// Adjoint of the implicit update of one coefficient, one real component
-// (stride `st` between levels).  Inputs: adjoints of the new level
-// an_* [K] and an_pi.  Outputs (overwritten): adjoints of the previous
-// level ap_* and of the explicit tendencies aw_*.  Scratch: 4 K values.
+// Element l of A^T x, for real or complex x.
+template <typename R, typename V>
+LBM_COL_HD V mat_t(const R* A, const V* x, int l, int K, V acc) {
+  for (int k = 0; k < K; ++k) acc = acc + x[k] * A[k * K + l];
+  return acc;
+}
+
+// Adjoint of the implicit update of one coefficient at level l, in four parts with
+// the column's values of the part before between them (V: real, or complex).
+template <typename V>
+struct ImplAdjLevel { V ap[4], aw[4], x; };   // vor div t q of the previous level, of the
+                                              // tendencies; the value the next part needs
+
+// x = VD^T an (no diffusion of vor, div at n < 2), field f.
+template <typename R, typename V>
+LBM_COL_HD V impl_adj_vdiff(const ImplConst<R>& c, int f, const V* an, int l, V zero) {
+  const bool use = c.vd[f] && !(f < 2 && c.vd_skip_vordiv);
+  return use ? mat_t(c.vd[f], an, l, c.K, zero) : an[l];
+}
+
+// The pointwise updates: vor/q_new = (p + 2 dt w) / (1 + 2 dt kv|kq), d_new = 2 dbar - p_div,
+// t_new = (p_t + 2 dt (w_t - tmtx dbar)) / ft.  Leaves the adjoint of dbar in x.
+template <typename R, typename V>
+LBM_COL_HD void impl_adj_point(const ImplConst<R>& c, int l, const V* v, ImplAdjLevel<V>& o) {
+  const R dt2 = R(2) * c.dt;
+  const R rv = R(1) / (R(1) + dt2 * c.kv[l]), rq = R(1) / (R(1) + dt2 * c.kq[l]);
+  const R rt = R(1) / (R(1) + dt2 * c.ktt[l]);
+  o.ap[0] = v[0] * rv;
+  o.aw[0] = v[0] * (dt2 * rv);
+  o.ap[1] = v[1] * R(-1);
+  o.ap[2] = v[2] * rt;
+  o.aw[2] = v[2] * (dt2 * rt);
+  o.ap[3] = v[3] * rq;
+  o.aw[3] = v[3] * (dt2 * rq);
+  o.x = v[1] * R(2);
+}
+
+// pi_new = p_pi + 2 dt (w_pi - sum dsig dbar); awt: the aw[2] of the column.
+template <typename R, typename V>
+LBM_COL_HD void impl_adj_dbar(const ImplConst<R>& c, int l, const V* awt, V awpi, V zero,
+                              ImplAdjLevel<V>& o) {
+  o.x = o.x + mat_t(c.tmtx, awt, l, c.K, zero) * R(-1) + awpi * (-c.dsig[l]);
+}
+
+// dbar = Minv rhs, rhs = p_div (1 + dt kd) ft + dt (w_div ft - lap wdphiy), wdphiy =
+// WW wdx + gg ft (p_pi + dt w_pi).  Leaves the adjoint of wdphiy in x; returns
+// this level's part of that of p_pi.
+template <typename R, typename V>
+LBM_COL_HD V impl_adj_rhs(const ImplConst<R>& c, int l, const V* dbar, V zero,
+                          ImplAdjLevel<V>& o) {
+  const R ft = R(1) + R(2) * c.dt * c.ktt[l];
+  const V rhs = mat_t(c.minv, dbar, l, c.K, zero);
+  o.ap[1] = o.ap[1] + rhs * ((R(1) + c.dt * c.kd[l]) * ft);
+  o.aw[1] = rhs * (c.dt * ft);
+  o.x = rhs * (-c.dt * c.lap);
+  return o.x * (c.gg[l] * ft);
+}
+
+// wdx = p_t (1 + dt ktt) + dt w_t
+template <typename R, typename V>
+LBM_COL_HD void impl_adj_wdx(const ImplConst<R>& c, int l, const V* phy, V zero,
+                             ImplAdjLevel<V>& o) {
+  const V s = mat_t(c.ww, phy, l, c.K, zero);
+  o.ap[2] = o.ap[2] + s * (R(1) + c.dt * c.ktt[l]);
+  o.aw[2] = o.aw[2] + s * c.dt;
+}
+
+// The four parts for one coefficient and one real component (stride `st`
+// between levels).  Inputs: adjoints of the new level an_* [K] and an_pi.
+// Outputs (overwritten): adjoints of the previous level ap_* and of the explicit
+// tendencies aw_*.  Scratch: 4 K values.
 template <typename R>
 LBM_COL_HD void implicit_coef_adjoint(const ImplConst<R>& c, int st, const R* an_vor,
                                       const R* an_div, const R* an_t, const R* an_q, R an_pi,
@@ -193,78 +245,50 @@ LBM_COL_HD void implicit_coef_adjoint(const ImplConst<R>& c, int st, const R* an
                                       R* aw_vor, R* aw_div, R* aw_t, R* aw_q, R* aw_pi,
                                       R* work) {
   const int K = c.K;
-  const R dt = c.dt, dt2 = R(2) * dt;
-  R* x = work;            // adjoint of a field before its vertical diffusion
-  R* dbar = work + K;     // adjoint of the solved divergence
-  R* rhs = work + 2 * K;  // adjoint of the right-hand side
-  R* phy = work + 3 * K;  // adjoint of the geopotential term wdphiy
   const R* an[4] = {an_vor, an_div, an_t, an_q};
   R* ap[4] = {ap_vor, ap_div, ap_t, ap_q};
   R* aw[4] = {aw_vor, aw_div, aw_t, aw_q};
+  R *col = work, *x = work + K, *y = work + 2 * K, *cp = work + 3 * K;
+  auto get = [&](int l) {
+    ImplAdjLevel<R> o;
+    for (int f = 0; f < 4; ++f) { o.ap[f] = ap[f][l * st]; o.aw[f] = aw[f][l * st]; }
+    o.x = x[l];
+    return o;
+  };
+  auto put = [&](int l, const ImplAdjLevel<R>& o, R* next) {
+    for (int f = 0; f < 4; ++f) { ap[f][l * st] = o.ap[f]; aw[f][l * st] = o.aw[f]; }
+    next[l] = o.x;
+  };
   for (int f = 0; f < 4; ++f) {
-    // x = VD^T an  (no diffusion of vor, div at n < 2)
-    const R* vd = c.vd[f];
-    const bool use = vd && !(f < 2 && c.vd_skip_vordiv);
-    for (int l = 0; l < K; ++l) {
-      R s = R(0);
-      if (use) {
-        for (int k = 0; k < K; ++k) s += vd[k * K + l] * an[f][k * st];
-      } else {
-        s = an[f][l * st];
-      }
-      x[l] = s;
-    }
-    for (int k = 0; k < K; ++k) {
-      const R v = x[k];
-      if (f == 0 || f == 3) {
-        // vor/q_new = (p + 2 dt w) / (1 + 2 dt kv|kq)
-        const R r = R(1) / (R(1) + dt2 * (f == 0 ? c.kv[k] : c.kq[k]));
-        ap[f][k * st] = v * r;
-        aw[f][k * st] = dt2 * v * r;
-      } else if (f == 1) {
-        // d_new = 2 dbar - p_div
-        dbar[k] = R(2) * v;
-        ap[f][k * st] = -v;
-      } else {
-        // t_new = (p_t + 2 dt (w_t - tmtx dbar)) / ft
-        const R ft = R(1) + dt2 * c.ktt[k];
-        ap[f][k * st] = v / ft;
-        aw[f][k * st] = dt2 * v / ft;
-      }
-    }
+    for (int k = 0; k < K; ++k) cp[k] = an[f][k * st];
+    for (int l = 0; l < K; ++l) ap[f][l * st] = impl_adj_vdiff(c, f, cp, l, R(0));
   }
-  // pi_new = p_pi + 2 dt (w_pi - sum dsig dbar)
+  for (int l = 0; l < K; ++l) {
+    ImplAdjLevel<R> o = {};
+    const R v[4] = {ap[0][l * st], ap[1][l * st], ap[2][l * st], ap[3][l * st]};
+    impl_adj_point(c, l, v, o);
+    put(l, o, x);
+    col[l] = o.aw[2];
+  }
   *ap_pi = an_pi;
-  *aw_pi = dt2 * an_pi;
+  *aw_pi = R(2) * c.dt * an_pi;
   for (int l = 0; l < K; ++l) {
-    R s = R(0);
-    for (int k = 0; k < K; ++k) s -= c.tmtx[k * K + l] * aw_t[k * st];
-    dbar[l] += s - c.dsig[l] * (*aw_pi);
+    ImplAdjLevel<R> o = get(l);
+    impl_adj_dbar(c, l, col, *aw_pi, R(0), o);
+    put(l, o, y);
   }
-  // dbar = Minv rhs
-  for (int l = 0; l < K; ++l) {
-    R s = R(0);
-    for (int k = 0; k < K; ++k) s += c.minv[k * K + l] * dbar[k];
-    rhs[l] = s;
-  }
-  // rhs = p_div (1 + dt kd) ft + dt (w_div ft - lap wdphiy)
   R apix = R(0);
-  for (int k = 0; k < K; ++k) {
-    const R ft = R(1) + dt2 * c.ktt[k];
-    ap_div[k * st] += (R(1) + dt * c.kd[k]) * ft * rhs[k];
-    aw_div[k * st] = dt * ft * rhs[k];
-    phy[k] = -dt * c.lap * rhs[k];
-    // wdphiy = WW wdx + gg ft (p_pi + dt w_pi)
-    apix += c.gg[k] * ft * phy[k];
+  for (int l = 0; l < K; ++l) {
+    ImplAdjLevel<R> o = get(l);
+    apix += impl_adj_rhs(c, l, y, R(0), o);
+    put(l, o, x);
   }
   *ap_pi += apix;
-  *aw_pi += dt * apix;
-  // wdx = p_t (1 + dt ktt) + dt w_t
+  *aw_pi += c.dt * apix;
   for (int l = 0; l < K; ++l) {
-    R s = R(0);
-    for (int k = 0; k < K; ++k) s += c.ww[k * K + l] * phy[k];
-    ap_t[l * st] += (R(1) + dt * c.ktt[l]) * s;
-    aw_t[l * st] += dt * s;
+    ImplAdjLevel<R> o = get(l);
+    impl_adj_wdx(c, l, x, R(0), o);
+    put(l, o, y);
   }
 }
 

@@ -412,3 +412,32 @@ def test_tendency_kernel_against_oracle(torch, K, linear):
     for a, b in zip(got, ref):
         a = a.detach().cpu().numpy()
         assert np.abs(a - b).max() < 1e-10 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("K", [2, 7, 33, 64])
+def test_adjoint_kernels_are_the_transposes(torch, K):
+    """<A x, y> = <x, A^T y> for the grid tendencies (linearised) and the
+    implicit update with vertical diffusion, at level counts that divide a
+    block's threads and that do not.  Both sides are sums of products rounded a
+    few hundred times: 1e-13 of |A x| |y|."""
+    from lbm_isca_gb300.adjoint import TimeStep, spec_dot, state_dot
+    from test_adjoint import _Rand, _model
+    m, _ = _model(K, vdifv=1.0e3, vdifd=1.0e3, vdift=1.0e3, vdifq=2.0e3)
+    st, r = TimeStep(m), _Rand(torch, K, K=K)
+    norm = lambda xs: float(sum(spec_dot(x, x) for x in xs)) ** 0.5      # noqa: E731
+
+    def check(ax, y, rhs):
+        lhs = float(sum(spec_dot(a, b) for a, b in zip(ax, y)))
+        assert abs(lhs - float(rhs)) < 1e-13 * norm(ax) * norm(y)
+
+    ga, dx = r.state(st), r.state(st)
+    aw = [r.spec(), r.spec(), r.spec(), r.spec(False), r.spec()]
+    check(st.tangent_tendencies(ga, dx), aw, state_dot(dx, st.adjoint_tendencies(ga, aw)))
+    keys = ("vor", "div", "t", "pi", "q")
+    p, y = ({k: r.spec(k != "pi") for k in keys} for _ in range(2))
+    w = [r.spec(k != "pi") for k in keys]
+    new = m.integ.step(1200.0, p, w)
+    ap, aw2 = st._implicit_adjoint(1200.0, y)
+    check([new[k] for k in keys], [y[k] for k in keys],
+          sum(spec_dot(p[k], ap[k]) for k in keys)
+          + sum(spec_dot(wi, aw2[k]) for wi, k in zip(w, keys)))
