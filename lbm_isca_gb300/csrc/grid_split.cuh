@@ -181,6 +181,8 @@ __global__ void __launch_bounds__(IDFT_NT) k_idft(SD<float> d, const float2* __r
 }
 
 // ---------------------------------------------------------------------------
+constexpr int ALG_SEGMAX = 16;      // segments of a column at most
+
 // One thread per column, BT columns of one latitude per block (grid
 // (J I / BT, E)).  FP32: the kernel waits on global loads; the minimum resident
 // blocks per SM keep 92 / 80 / 80 registers at I = 64 / 128 / 256 -- at 128 that
@@ -189,16 +191,24 @@ __global__ void __launch_bounds__(IDFT_NT) k_idft(SD<float> d, const float2* __r
 // division: the reciprocal layer thickness is formed once per block; 27 us a member
 // at T42L20), bound by
 // the FP64 pipe; 32 columns per block spread one member over every SM.
-template <typename R, int I, int BT, int MINB>
-__global__ void __launch_bounds__(BT, MINB) k_alg(SD<R> d, int ps_mode) {
+//
+// SEG (few columns): a warp per segment of LS levels of 32 columns.  The values
+// that the column scans add up are left in shared memory by the segment that
+// owns the level, and every segment adds up those below it in the level's order
+// (the same sums).
+template <typename R, int I, int BT, int MINB, bool SEG>
+__global__ void __launch_bounds__(SEG ? ALG_SEGMAX * BT : BT, MINB)
+    k_alg(SD<R> d, int ps_mode, int LS) {
   constexpr int NB = I / BT;
   const int j = blockIdx.x / NB, e = blockIdx.y;
-  const int c = (blockIdx.x % NB) * BT + threadIdx.x;
+  const int lane = SEG ? threadIdx.x % BT : threadIdx.x;
+  const int c = (blockIdx.x % NB) * BT + lane;
   const int J = d.J, K = d.K;
+  const int ka = SEG ? (int)(threadIdx.x / BT) * LS : 0, ke_ = SEG ? min(ka + LS, K) : K;
   __shared__ R vert[LBM_VERT_COUNT * 65];
   __shared__ R rds[64];                              // 1 / dsig
-  for (int x = threadIdx.x; x < LBM_VERT_COUNT * (K + 1); x += BT) vert[x] = d.vert[x];
-  for (int x = threadIdx.x; x < K; x += BT) rds[x] = R(1) / vrow(d, LBM_VERT_DSIG, x);
+  for (int x = threadIdx.x; x < LBM_VERT_COUNT * (K + 1); x += blockDim.x) vert[x] = d.vert[x];
+  for (int x = threadIdx.x; x < K; x += blockDim.x) rds[x] = R(1) / vrow(d, LBM_VERT_DSIG, x);
   __syncthreads();
   const int VS = K + 1;
   auto V = [&](int row, int k) { return vert[row * VS + k]; };
@@ -216,8 +226,8 @@ __global__ void __launch_bounds__(BT, MINB) k_alg(SD<R> d, int ps_mode) {
   const R uh = g6[3 * I], vh = g6[4 * I], dh = g6[5 * I];
   const R sx = pixb * uh + piyb * vh + pix * usum + piy * vsum;   // sum dsig v.grad(pi)
   const R stot = dh + sx;
-  g9[0] = -sx;                                   // gt_pi
-  {
+  if (!SEG || ka == 0) {
+    g9[0] = -sx;                                 // gt_pi
     const size_t gp = (size_t)e * J * I + g2;
     const R pscur = psbar * expm1(pi);
     R pb = d.psb[gp];
@@ -245,12 +255,46 @@ __global__ void __launch_bounds__(BT, MINB) k_alg(SD<R> d, int ps_mode) {
   R prefd = R(0), prefp = R(0), pref3 = R(0);
   // level window: m = k-1, 0 = k, p = k+1 (u, v, T, q); vorticity and
   // divergence of level k only
-  R u0 = gl[SF_U * I], v0 = gl[SF_V * I], t0 = gl[SF_T * I], q0 = gl[SF_Q * I];
-  R vo0 = gl[SF_VOR * I], dv0 = gl[SF_DIV * I];
   R um = R(0), vm = R(0), tm_ = R(0), qm = R(0);       // level k - 1
   R hum = R(0), hvm = R(0), htm = R(0), hqm = R(0);    // half differences at k - 1
+  if constexpr (SEG) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    R* scan = reinterpret_cast<R*>(smraw) + lane;      // [K][3][BT]: dv, v.grad(pi), Tv' - T'
+    for (int k = ka; k < ke_; ++k) {
+      const R* gk = gl + (size_t)k * SF_N * I;
+      const R* bq = bk + (size_t)k * I;
+      const R u0 = gk[SF_U * I], v0 = gk[SF_V * I], t0 = gk[SF_T * I], q0 = gk[SF_Q * I];
+      const R ub = __ldg(bq + B_U * b3f), vb = __ldg(bq + B_V * b3f);
+      const R tb = __ldg(bq + B_T * b3f), qb = __ldg(bq + B_Q * b3f);
+      scan[(3 * k + 0) * BT] = gk[SF_DIV * I];
+      scan[(3 * k + 1) * BT] = u0 * pixb + ub * pix + v0 * piyb + vb * piy;
+      scan[(3 * k + 2) * BT] = eps * (t0 * qb + tb * q0);
+    }
+    __syncthreads();
+    for (int k = 0; k < ka; ++k) {
+      const R dv0 = scan[(3 * k + 0) * BT], pa = scan[(3 * k + 1) * BT];
+      const R xv = scan[(3 * k + 2) * BT], dsk = V(LBM_VERT_DSIG, k);
+      sdlo = sdlo + dsk * (dv0 + pa - stot);
+      prefd += dsk * dv0;
+      prefp += dsk * pa;
+      pref3 += V(LBM_VERT_RDLOG3, k) * xv;
+    }
+    bk += (size_t)ka * I;
+    bsk += (size_t)ka * I;
+    gl += (size_t)ka * SF_N * I;
+    go += (size_t)ka * 9 * I;
+    if (ka > 0 && ka < K) {
+      const R* gm = gl - SF_N * I;
+      um = gm[SF_U * I]; vm = gm[SF_V * I]; tm_ = gm[SF_T * I]; qm = gm[SF_Q * I];
+      hum = __ldg(bk - I + B_HDU * b3f); hvm = __ldg(bk - I + B_HDV * b3f);
+      htm = __ldg(bk - I + B_HDT * b3f); hqm = __ldg(bk - I + B_HDQ * b3f);
+    }
+    if (ka >= K) return;
+  }
+  R u0 = gl[SF_U * I], v0 = gl[SF_V * I], t0 = gl[SF_T * I], q0 = gl[SF_Q * I];
+  R vo0 = gl[SF_VOR * I], dv0 = gl[SF_DIV * I];
   R sb0 = __ldg(bsk);
-  for (int k = 0; k < K; ++k) {
+  for (int k = ka; k < ke_; ++k) {
     const bool hasm = k >= 1, hasp = k + 1 <= K - 1;
     R up = u0, vp = v0, tp = t0, qp = q0, vop = R(0), dvp = R(0);
     if (hasp) {

@@ -429,6 +429,18 @@ namespace lbm {
 
 // ---- launch configuration ------------------------------------------------------
 // Resident k_alg blocks of I threads (see the kernel).
+// Levels per segment of k_alg, 0 for whole columns: segments while the columns are
+// less than a warp per SM partition (one member of T42: 256 of 608).  Two
+// levels in FP32, bound by latency (T42L20, one member, us: 22 whole, 9.0, 10.6, 11.6
+// and 17 with 2, 3, 5, 10 levels); five in FP64, where the sums below a segment
+// cost more of the FP64 pipe (83 whole, 59, 50, 47, 52).  At seven members whole
+// columns win (19 against 21 to 35).
+template <typename R> int alg_seg(int E, int J, int I, int K) {
+  const long warps = (long)E * J * (I / 32);
+  if (warps > 4 * LF_SMS || K < 2) return 0;
+  const int ls = sizeof(R) == 4 ? 2 : 5, least = (K + ALG_SEGMAX - 1) / ALG_SEGMAX;
+  return ls > least ? ls : least;
+}
 template <int I> constexpr int alg_minb() { return I == 64 ? 10 : (I == 128 ? 6 : 3); }
 
 template <typename R, int I> constexpr int grid_kb() { return (sizeof(R) == 8 && I == 256) ? 2 : 4; }
@@ -506,6 +518,22 @@ inline int persistent_grid(const void* fn, int nt, size_t smem, int units) {
   return ctas < units ? ctas : units;
 }
 
+template <typename R, int I, int BT, int MINB>
+void launch_alg(const SD<R>& d, int ps_mode, cudaStream_t st, bool attrs) {
+  const int LS = alg_seg<R>(d.E, d.J, I, d.K);
+  if (!LS) {
+    if (!attrs) k_alg<R, I, BT, MINB, false><<<dim3(d.J * (I / BT), d.E), BT, 0, st>>>(d, ps_mode, 0);
+    return;
+  }
+  const int smem = 3 * 32 * (int)sizeof(R) * d.K;
+  if (attrs)
+    cudaFuncSetAttribute(k_alg<R, I, 32, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         3 * 32 * (int)sizeof(R) * 64);
+  else
+    k_alg<R, I, 32, 1, true><<<dim3(d.J * (I / 32), d.E), 32 * ((d.K + LS - 1) / LS), smem, st>>>(
+        d, ps_mode, LS);
+}
+
 template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl& c,
                                              cudaStream_t st, int only = -1) {
   constexpr int KB = grid_kb<R, I>(), NT = grid_nt<R, I>();
@@ -517,7 +545,7 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
     if (only < 0 || only == 0 || only == 4)
       k_idft<I><<<dim3(d.J, d.E), IDFT_NT, idft_smem(I, d.M), st>>>(d, d.dft);
     if (only < 0 || only == 0 || only == 5)
-      k_alg<R, I, I, alg_minb<I>()><<<dim3(d.J, d.E), I, 0, st>>>(d, c.ps_mode);
+      launch_alg<R, I, I, alg_minb<I>()>(d, c.ps_mode, st, false);
     if ((only < 0 || only == 0 || only == 6) && d.legendre && !(d.tc_off & 4) &&
         ftc_supported(I, d.K, d.N)) {
       const FtcPlan pl = ftc_plan(d.E, d.J, I, d.K, d.N);
@@ -542,7 +570,7 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
       using G = GridFft<I>;
       k_ifft<R, I><<<dim3(d.J, 1 + (d.K + G::LI - 1) / G::LI, d.E), G::NTI,
                      G::template ifft_smem<R>(d.M), st>>>(d);
-      k_alg<R, I, 32, 1><<<dim3(d.J * (I / 32), d.E), 32, 0, st>>>(d, c.ps_mode);
+      launch_alg<R, I, 32, 1>(d, c.ps_mode, st, false);
       k_ffft<R, I><<<dim3(d.J, 1 + (d.K + G::LF - 1) / G::LF, d.E), G::NTF,
                      G::template ffft_smem<R>(d.M), st>>>(d);
     } else {
@@ -576,6 +604,7 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
 
 template <typename R, int I> void set_attrs(const SD<R>& d) {
   constexpr int KB = grid_kb<R, I>(), NT = grid_nt<R, I>();
+  launch_alg<R, I, sizeof(R) == 4 ? I : 32, sizeof(R) == 4 ? alg_minb<I>() : 1>(d, 0, 0, true);
   if constexpr (sizeof(R) == 4) {
     cudaFuncSetAttribute(k_idft<I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)idft_smem(I, d.M));

@@ -441,3 +441,28 @@ def test_adjoint_kernels_are_the_transposes(torch, K):
     check([new[k] for k in keys], [y[k] for k in keys],
           sum(spec_dot(p[k], ap[k]) for k in keys)
           + sum(spec_dot(wi, aw2[k]) for wi, k in zip(w, keys)))
+
+
+@pytest.mark.parametrize("grid,K", [("T21", 2), ("T21", 21), ("T21", 64), ("T42", 20),
+                                    ("T42", 7)])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("ps_mode", [0, 2])
+def test_column_segments_equal_whole_columns(torch, grid, K, precision, ps_mode):
+    """k_alg of one member (columns cut into level segments) against the same
+    member in an ensemble large enough for whole columns: the same bits in FP32,
+    rounding of the column sums (1e-13 of the largest value) in FP64."""
+    one = _stepper(torch, grid, K, 1, precision)
+    many = _stepper(torch, grid, K, 20, precision)
+    for name in ("sf", "sfs", "psa", "psb"):
+        getattr(many, name).copy_(getattr(one, name).expand_as(getattr(many, name)))
+    for s in (one, many):
+        s.grid9.zero_()
+        _launch(torch, s, 0, ps_mode=ps_mode)
+    for name in ("grid9", "psa", "psb"):
+        a = getattr(one, name)[0]
+        b = getattr(many, name).reshape(20, *a.shape)[19]
+        assert float(a.abs().max()) > 0
+        if precision == "fp32":
+            assert torch.equal(a, b)
+        else:
+            assert _rel(a, b) < 1e-13
