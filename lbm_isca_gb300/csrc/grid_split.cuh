@@ -401,21 +401,31 @@ __global__ void __launch_bounds__(SEG ? ALG_SEGMAX * BT : BT, MINB)
 // and the table likewise into T0..T3 = cos, sin of m = 2p and of m = 2p + 1.
 // Plane c gives the sums S_c[row][p] = sum_i P_c[i][row] T_c[i][p]; each lane
 // owns one c and an 8-row by 8-pair tile (64 accumulators) and reads per point
-// two float4 of its rows and two of its pairs.  The quarter warps of a half
-// warp hold different planes, so every 16-byte load is one shared-memory
-// wavefront per half warp (conflict-free by the plane and row strides).  The
-// sums go through shared memory to an output pass that combines rows (a3 =
-// wg X(gt) - wd i m X(xu), ...) and writes af/afs with coalesced stores.
+// two float4 of its rows and two of its pairs (conflict-free by the plane and row
+// strides).  The sums go through shared memory to an output pass that combines
+// rows (a3 = wg X(gt) - wd i m X(xu), ...) and writes af/afs with coalesced stores.
 //
 // CTAs are persistent: each walks the units with a grid stride, loads the
-// table once, and streams the next unit's rows into shared memory by
-// cp.async while it computes the current one.
+// table once, and prefetches the next unit's rows into L2 while it computes the
+// current one.  Neither the FMAs (120 of 516 us at T42L20, 128 members) nor DRAM
+// (137) bound it but the phases of two or three CTAs per SM that do not overlap:
+// without the fold 436 of 637, without the products 456, without the combining
+// 544.  The fold takes its sixteen loads from one row pointer, and the sums are
+// staged without bank conflicts: us at T42, 7 and 128 members and T85L40, 16
+// members: 40 -> 35, 613 -> 516, 992 -> 817.  Packed FMAs (552), and two or three
+// quads of loads in flight (518, 639), were slower.
 struct FdftPlan {
   int lc, nrg, npg, warps, nt;           // levels, row groups, pair groups, warps, threads
   int rp, ps, npp, ts;                   // strides (floats): plane point, plane, table point,
                                          //   table plane
+  int os;                                // stride (complex) of the staged sums' wavenumbers
   int tab, pl, b0, total;                // float offsets of the shared-memory blocks, size
 };
+
+// Place of wavenumber m's staged sums.  In a half warp the sums of one store
+// differ by 16 wavenumbers (pair group), 8 (quarter) and a level (7 values): an
+// odd stride and five values more every 16 wavenumbers spread them over the banks.
+LBM_HD int fdft_place(int m, int os) { return m * os + 5 * (m >> 4); }
 
 LBM_HD FdftPlan fdft_layout(int I, int M, int lc) {
   const int Q = I / 4, NP = (M + 1) / 2, nrow = 9 * lc + 2;
@@ -431,8 +441,9 @@ LBM_HD FdftPlan fdft_layout(int I, int M, int lc) {
   p.ts = Q * p.npp + 4;
   auto al4 = [](int x) { return (x + 3) & ~3; };
   // the staged outputs [M][7 lc] float2 alias the planes
+  p.os = (7 * lc) | 1;
   int planes = 4 * p.ps;
-  if (14 * M * lc > planes) planes = 14 * M * lc;
+  if (2 * fdft_place(M, p.os) > planes) planes = 2 * fdft_place(M, p.os);
   int o = 0;
   p.tab = o; o = al4(o + 4 * p.ts);
   p.pl = o; o = al4(o + planes);
@@ -473,7 +484,7 @@ LBM_HD FdftPlan fdft_plan(int I, int M, int K) {
 }
 
 template <int I>
-__global__ void __launch_bounds__(256) k_fdft(SD<float> d, const float2* __restrict__ dft,
+__global__ void __launch_bounds__(256, I == 256 ? 1 : 2) k_fdft(SD<float> d, const float2* __restrict__ dft,
                                               FdftPlan pl) {
   constexpr int Q = I / 4;
   const int J = d.J, K = d.K, M = d.M, NR9 = fdft_rows(K);
@@ -509,9 +520,11 @@ __global__ void __launch_bounds__(256) k_fdft(SD<float> d, const float2* __restr
     const float* g9 = d.grid9 + (size_t)col * NR9 * I;
     const float* lev = g9 + (size_t)(2 + 9 * k0) * I;
     __syncthreads();                         // the previous unit's sums are read
+    const float gw = d.jfac[JF_GW * J + j], gwdc = d.jfac[JF_GWDELC * J + j];
+    const float wg = gw / float(I), wd = gwdc / float(I);
     // fold: a lane takes one point of four consecutive plane rows (a warp:
-    // 32 points, or two row quads at I = 64) and stores each plane's four
-    // rows as one float4; the lanes of point 0 keep (x0, x_{I/2}, u_Q, v_Q).
+    // 32 points, or two row quads at I = 64) and stores each plane's four rows as
+    // one float4; one thread per row keeps (x0, x_{I/2}, u_Q, v_Q).
     // Plane rows: level l's gt xu g yu fu fv ke xv at 8 l .. 8 l + 7, then the
     // yv rows of the levels, then (level 0) the two surface rows.
     {
@@ -519,51 +532,52 @@ __global__ void __launch_bounds__(256) k_fdft(SD<float> d, const float2* __restr
       const int nrq = (nrow + 3) >> 2;
       const int nit = ((nrq + SUB - 1) / SUB) * NIW;
       auto rowp = [&](int pr) -> const float* {
-        if (pr < 8 * lc) return lev + (size_t)(9 * (pr >> 3) + (pr & 7)) * I;
-        if (pr < 9 * lc) return lev + (size_t)(9 * (pr - 8 * lc) + 8) * I;
-        return g9 + (size_t)(pr - 9 * lc) * I;
+        if (pr < 8 * lc) return lev + (9 * (pr >> 3) + (pr & 7)) * I;
+        if (pr < 9 * lc) return lev + (9 * (pr - 8 * lc) + 8) * I;
+        return g9 + (pr - 9 * lc) * I;
       };
       for (int it = warp; it < nit; it += nwarp) {
         const int rq = (it / NIW) * SUB + lane / PPW;
         const int i = (it % NIW) * PPW + (lane & (PPW - 1));
-        if (rq < nrq) {
-          float xv[4][4];
+        if (rq >= nrq || i == 0) continue;
+        float xv[4][4], pv[4][4];              // all sixteen loads first
+        if (rq < 2 * lc) {                     // four consecutive rows of a level
+          const float* row = lev + (9 * (rq >> 1) + 4 * (rq & 1)) * I;
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
-            const int r = 4 * rq + t;
-            if (r < nrow) {
-              const float* row = rowp(r);
-              xv[t][0] = __ldg(row + i);
-              xv[t][1] = __ldg(row + ((I - i) & (I - 1)));
-              xv[t][2] = __ldg(row + (I / 2 - i));
-              xv[t][3] = __ldg(row + (I / 2 + i));
-            } else {
-              xv[t][0] = xv[t][1] = xv[t][2] = xv[t][3] = 0.f;
-            }
+            xv[t][0] = __ldg(row + t * I + i);
+            xv[t][1] = __ldg(row + t * I + I - i);
+            xv[t][2] = __ldg(row + t * I + I / 2 - i);
+            xv[t][3] = __ldg(row + t * I + I / 2 + i);
           }
-          float pv[4][4];
+        } else {                               // rows past the unit's: copies, not used
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
-            const float xa = xv[t][0], xb = xv[t][1], xc = xv[t][2], xd = xv[t][3];
-            const float uu = xa + xb, w = xa - xb, uh = xc + xd, vh = xc - xd;
-            pv[0][t] = uu + uh;
-            pv[1][t] = w - vh;
-            pv[2][t] = uu - uh;
-            pv[3][t] = w + vh;
-            const int r = 4 * rq + t;
-            if (i == 0 && r < nrow) {
-              const float* row = rowp(r);
-              const float xq = __ldg(row + Q), x3q = __ldg(row + 3 * Q);
-              b0s[r] = make_float4(xa, xc, xq + x3q, xq - x3q);
-            }
-          }
-          if (i != 0) {
-            float* o = pln + i * RP + 4 * rq;
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-              *reinterpret_cast<float4*>(o + c * PS) = make_float4(pv[c][0], pv[c][1], pv[c][2], pv[c][3]);
+            const float* row = rowp(min(4 * rq + t, nrow - 1));
+            xv[t][0] = __ldg(row + i);
+            xv[t][1] = __ldg(row + I - i);
+            xv[t][2] = __ldg(row + I / 2 - i);
+            xv[t][3] = __ldg(row + I / 2 + i);
           }
         }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const float xa = xv[t][0], xb = xv[t][1], xc = xv[t][2], xd = xv[t][3];
+          const float uu = xa + xb, w = xa - xb, uh = xc + xd, vh = xc - xd;
+          pv[0][t] = uu + uh;
+          pv[1][t] = w - vh;
+          pv[2][t] = uu - uh;
+          pv[3][t] = w + vh;
+        }
+        float* o = pln + i * RP + 4 * rq;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          *reinterpret_cast<float4*>(o + c * PS) = make_float4(pv[c][0], pv[c][1], pv[c][2], pv[c][3]);
+      }
+      for (int r = tid; r < nrow; r += nt) {
+        const float* row = rowp(r);
+        const float xq = __ldg(row + Q), x3q = __ldg(row + 3 * Q);
+        b0s[r] = make_float4(__ldg(row), __ldg(row + I / 2), xq + x3q, xq - x3q);
       }
     }
     __syncthreads();
@@ -622,9 +636,7 @@ __global__ void __launch_bounds__(256) k_fdft(SD<float> d, const float2* __restr
     // quarter pairs 0-3 of its group, the odd quarter pairs 4-7.  A level's
     // group gives its six fields (a3 = wg X(gt) - wd i m X(xu), a5 from g,
     // yu; fu fv ke xv); the trailing groups give yv and the surface rows.
-    const float gw = d.jfac[JF_GW * J + j], gwdc = d.jfac[JF_GWDELC * J + j];
-    const float wg = gw / float(I), wd = gwdc / float(I);
-    float2* fo = reinterpret_cast<float2*>(pln);     // [M][7 lc]: item m lc + l at 7 (m lc + l)
+    float2* fo = reinterpret_cast<float2*>(pln);     // [M][7 lc] at fdft_place(m)
     const bool ev = (c & 1) == 0;
     const int par = c >> 1;                          // 0: even m, 1: odd m
     const int NP = (M + 1) >> 1;
@@ -647,7 +659,7 @@ __global__ void __launch_bounds__(256) k_fdft(SD<float> d, const float2* __restr
         if (p >= NP || m >= M) continue;
         // X_h = (re[h], -im[h])
         if (rg < lc) {
-          float2* o = fo + AF_N * (m * lc + rg);
+          float2* o = fo + fdft_place(m, pl.os) + AF_N * rg;
           const float wdm = wd * float(m);
           if (rp < 2) {
             // rows (gt, xu) or (g, yu): wg X0 - wd i m X1
@@ -665,7 +677,7 @@ __global__ void __launch_bounds__(256) k_fdft(SD<float> d, const float2* __restr
           for (int h = 0; h < 2; ++h) {
             const int pr = 8 * rg + 2 * rp + h;
             if (pr < 9 * lc) {
-              fo[AF_N * (m * lc + (pr - 8 * lc)) + AF_YV] = make_float2(wd * re[h][q], wd * -im[h][q]);
+              fo[fdft_place(m, pl.os) + AF_N * (pr - 8 * lc) + AF_YV] = make_float2(wd * re[h][q], wd * -im[h][q]);
             } else if (surf && pr < 9 * lc + 2) {
               float2* os = reinterpret_cast<float2*>(d.afs);
               os[(((size_t)e * M + m) * J + j) * 2 + (pr - 9 * lc)] =
@@ -675,17 +687,18 @@ __global__ void __launch_bounds__(256) k_fdft(SD<float> d, const float2* __restr
         }
       }
     }
-    const int nitem = M * lc;
     __syncthreads();
     {
-      // staged rows -> af, consecutive threads on consecutive addresses
+      // staged rows -> af, a warp per wavenumber, consecutive lanes on
+      // consecutive addresses
       const int RS = AF_N * lc;
-      const unsigned mg = (unsigned)((0x100000000ull + RS - 1) / RS);   // y / RS, y < 2^16
       float2* afu = reinterpret_cast<float2*>(d.af) + (((size_t)e * M * J + j) * K + k0) * AF_N;
       const size_t mstride = (size_t)J * K * AF_N;
-      for (int y = tid; y < AF_N * nitem; y += nt) {
-        const int m = __umulhi((unsigned)y, mg);
-        afu[m * mstride + (y - m * RS)] = fo[y];
+      for (int m = warp; m < M; m += nwarp) {
+        const float2* sp = fo + fdft_place(m, pl.os);
+        float2* op = afu + m * mstride;
+#pragma unroll 4
+        for (int x = lane; x < RS; x += 32) op[x] = sp[x];
       }
     }
   }

@@ -466,3 +466,39 @@ def test_column_segments_equal_whole_columns(torch, grid, K, precision, ps_mode)
             assert torch.equal(a, b)
         else:
             assert _rel(a, b) < 1e-13
+
+
+@pytest.mark.parametrize("I,J,N,K,nmem", [(64, 32, 21, 1, 1), (64, 32, 21, 20, 2), (64, 6, 3, 7, 9),
+                                          (128, 64, 42, 17, 3), (128, 64, 63, 3, 1),
+                                          (128, 64, 42, 64, 1), (256, 128, 85, 9, 2),
+                                          (256, 128, 127, 5, 1)])
+def test_longitude_analysis_against_fp64_sums(torch, I, J, N, K, nmem):
+    """k_fdft against FP64 transforms of the same rows: level chunks with
+    remainders, one level, the most wavenumbers.  Bound per value: I + 16
+    operations on terms that sum to the row's magnitudes (times m for the
+    rows combined with a derivative)."""
+    stp = _grid_stepper(torch, I, J, N, K, nmem, "fp32")
+    u = 2.0 ** -24
+    g = torch.Generator(device="cuda").manual_seed(I + K)
+    stp.grid9.copy_(torch.randn(stp.grid9.shape, generator=g, device="cuda", dtype=torch.float64))
+    stp.af.zero_()
+    stp.afs.zero_()
+    _launch(torch, stp, 6)
+    x = stp.grid9.double()                               # [E][J][2 + 9K][I]
+    X = torch.fft.rfft(x, dim=-1)[..., :stp.M]
+    A = x.abs().sum(-1, keepdim=True).expand_as(X)
+    jf = stp.jfac.double().reshape(4, J)
+    wg, wd = (jf[k][None, :, None, None] / I for k in (0, 1))    # gw, gw del cos
+    m = torch.arange(stp.M, device="cuda", dtype=torch.float64)
+    rows = [X[:, :, 2 + f::9] for f in range(9)]         # gt xu g yu fu fv ke xv yv
+    mag = [A[:, :, 2 + f::9] for f in range(9)]
+    want = [wd * rows[4], wd * rows[5], wg * rows[6], wg * rows[0] - wd * 1j * m * rows[1],
+            wd * rows[7], wg * rows[2] - wd * 1j * m * rows[3], wd * rows[8]]
+    size = [wd * mag[4], wd * mag[5], wg * mag[6], wg * mag[0] + wd * m * mag[1],
+            wd * mag[7], wg * mag[2] + wd * m * mag[3], wd * mag[8]]
+    for f in range(7):
+        got = stp.af[..., f].to(torch.complex128).permute(0, 2, 3, 1)      # [E][J][K][M]
+        assert bool(((got - want[f]).abs() <= (I + 16) * u * size[f]).all()), f
+    for f in range(2):
+        got = stp.afs[..., f].to(torch.complex128).permute(0, 2, 1)
+        assert bool(((got - (wg * X)[:, :, f]).abs() <= (I + 16) * u * (wg * A)[:, :, f]).all())
