@@ -25,6 +25,10 @@ constexpr int IDFT_NT = 128;    // threads of the longitude synthesis block
 constexpr int IDFT_RC = 48;      // rows per staged chunk (two buffers fit five CTAs per SM)
 constexpr int IDFT_RG = 8;       // rows per thread item
 
+// One chunk of rows per block instead of a column's chunks in turn, while the
+// columns leave SMs idle.  us at T42L20, one member: 16.0 -> 9.7.
+inline bool idft_chunks(int E, int J) { return E * J < 2 * LF_SMS; }
+
 LBM_HD int idft_rows(int K) { return 6 + 6 * K; }
 LBM_HD int fdft_rows(int K) { return 2 + 9 * K; }
 
@@ -35,8 +39,37 @@ LBM_HD size_t idft_smem(int I, int M) {
 }
 
 // ---------------------------------------------------------------------------
-template <int I>
-__global__ void __launch_bounds__(IDFT_NT) k_idft(SD<float> d, const float2* __restrict__ dft) {
+// (cos, sin) sums of (Re, Im) x (cos, sin) pairs as they lie in memory: one packed
+// FMA, or two scalar ones.  The packed form needs up to 148 registers: capped at
+// 128 (four CTAs per SM) it is faster at I = 64 and 256 (us: T21 48 members 36 -> 32,
+// T85 16 members 568 -> 503), where the table leaves room for few CTAs or the grid
+// is small; at I = 128 five CTAs of the scalar form win (253 against 262 at 128
+// members).
+template <bool PAIR> struct IdftSum;
+template <> struct IdftSum<true> {
+  unsigned long long v = 0ull;
+  LBM_D void fma(unsigned long long x, unsigned long long t) { v = Cacc<float>::fma2(x, t, v); }
+  LBM_D float2 get() const {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+  }
+};
+template <> struct IdftSum<false> {
+  float2 v = {0.f, 0.f};
+  LBM_D void fma(unsigned long long x, unsigned long long t) {
+    float2 a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(x));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(b.x), "=f"(b.y) : "l"(t));
+    v.x = fmaf(a.x, b.x, v.x);
+    v.y = fmaf(a.y, b.y, v.y);
+  }
+  LBM_D float2 get() const { return v; }
+};
+
+template <int I, bool CHUNK>
+__global__ void __launch_bounds__(IDFT_NT, I == 128 ? 5 : 4) k_idft(SD<float> d, const float2* __restrict__ dft) {
+  constexpr bool PAIR = I != 128;
   constexpr int Q = I / 4, NT = IDFT_NT, RC = IDFT_RC, RG = IDFT_RG;
   const int j = blockIdx.x, e = blockIdx.y;
   const int J = d.J, K = d.K, M = d.M;
@@ -88,11 +121,12 @@ __global__ void __launch_bounds__(IDFT_NT) k_idft(SD<float> d, const float2* __r
     return (f == SF_U || f == SF_V) ? rcos : 1.f;
   };
 
-  stage(0, 0);
+  const int vs0 = CHUNK ? (int)blockIdx.z * RC : 0;
+  stage(vs0, 0);
   int buf = 0;
-  for (int v0 = 0; v0 < NR; v0 += RC) {
+  for (int v0 = vs0; v0 < NR; v0 += RC) {
     const int nr = min(RC, NR - v0);
-    if (v0 + RC < NR) stage(v0 + RC, buf ^ 1);
+    if (!CHUNK && v0 + RC < NR) stage(v0 + RC, buf ^ 1);
     else cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
@@ -105,44 +139,31 @@ __global__ void __launch_bounds__(IDFT_NT) k_idft(SD<float> d, const float2* __r
       const int i0 = it % QH + 1, g = it / QH;
       const int r0 = g * RG;
       if (r0 >= nr) continue;
-      float ce[2][RG], co[2][RG], se[2][RG], so[2][RG];
+      IdftSum<PAIR> ae[2][RG], ao[2][RG];      // even and odd m
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int r = 0; r < RG; ++r) ce[h][r] = co[h][r] = se[h][r] = so[h][r] = 0.f;
-      const float2* tb0 = tab + i0;
-      const float2* tb1 = tab + i0 + QH;
+        for (int r = 0; r < RG; ++r) ae[h][r] = ao[h][r] = IdftSum<PAIR>();
+      const unsigned long long* tb0 = reinterpret_cast<const unsigned long long*>(tab) + i0;
+      const unsigned long long* tb1 = tb0 + QH;
+      auto add = [&](int m, IdftSum<PAIR> (&acc)[2][RG]) {
+        const unsigned long long t0 = tb0[m * (Q + 1)], t1 = tb1[m * (Q + 1)];
+        const ulonglong2* x = reinterpret_cast<const ulonglong2*>(F + m * RC + r0);
+#pragma unroll
+        for (int t = 0; t < RG / 2; ++t) {
+          const ulonglong2 b = x[t];
+          acc[0][2 * t].fma(b.x, t0);
+          acc[0][2 * t + 1].fma(b.y, t0);
+          acc[1][2 * t].fma(b.x, t1);
+          acc[1][2 * t + 1].fma(b.y, t1);
+        }
+      };
       int m = 1;
       for (; m + 1 < M; m += 2) {              // (odd, even) pairs of m >= 1
-        const float2 to0 = tb0[m * (Q + 1)], te0 = tb0[(m + 1) * (Q + 1)];
-        const float2 to1 = tb1[m * (Q + 1)], te1 = tb1[(m + 1) * (Q + 1)];
-        const float4* xo = reinterpret_cast<const float4*>(F + m * RC + r0);
-        const float4* xe = reinterpret_cast<const float4*>(F + (m + 1) * RC + r0);
-#pragma unroll
-        for (int t = 0; t < RG / 2; ++t) {
-          const float4 b = xo[t], a = xe[t];
-          co[0][2 * t] = fmaf(b.x, to0.x, co[0][2 * t]);       so[0][2 * t] = fmaf(b.y, to0.y, so[0][2 * t]);
-          co[0][2 * t + 1] = fmaf(b.z, to0.x, co[0][2 * t + 1]); so[0][2 * t + 1] = fmaf(b.w, to0.y, so[0][2 * t + 1]);
-          ce[0][2 * t] = fmaf(a.x, te0.x, ce[0][2 * t]);       se[0][2 * t] = fmaf(a.y, te0.y, se[0][2 * t]);
-          ce[0][2 * t + 1] = fmaf(a.z, te0.x, ce[0][2 * t + 1]); se[0][2 * t + 1] = fmaf(a.w, te0.y, se[0][2 * t + 1]);
-          co[1][2 * t] = fmaf(b.x, to1.x, co[1][2 * t]);       so[1][2 * t] = fmaf(b.y, to1.y, so[1][2 * t]);
-          co[1][2 * t + 1] = fmaf(b.z, to1.x, co[1][2 * t + 1]); so[1][2 * t + 1] = fmaf(b.w, to1.y, so[1][2 * t + 1]);
-          ce[1][2 * t] = fmaf(a.x, te1.x, ce[1][2 * t]);       se[1][2 * t] = fmaf(a.y, te1.y, se[1][2 * t]);
-          ce[1][2 * t + 1] = fmaf(a.z, te1.x, ce[1][2 * t + 1]); se[1][2 * t + 1] = fmaf(a.w, te1.y, se[1][2 * t + 1]);
-        }
+        add(m, ao);
+        add(m + 1, ae);
       }
-      if (m < M) {                              // last (odd) m
-        const float2 to0 = tb0[m * (Q + 1)], to1 = tb1[m * (Q + 1)];
-        const float4* xo = reinterpret_cast<const float4*>(F + m * RC + r0);
-#pragma unroll
-        for (int t = 0; t < RG / 2; ++t) {
-          const float4 b = xo[t];
-          co[0][2 * t] = fmaf(b.x, to0.x, co[0][2 * t]);       so[0][2 * t] = fmaf(b.y, to0.y, so[0][2 * t]);
-          co[0][2 * t + 1] = fmaf(b.z, to0.x, co[0][2 * t + 1]); so[0][2 * t + 1] = fmaf(b.w, to0.y, so[0][2 * t + 1]);
-          co[1][2 * t] = fmaf(b.x, to1.x, co[1][2 * t]);       so[1][2 * t] = fmaf(b.y, to1.y, so[1][2 * t]);
-          co[1][2 * t + 1] = fmaf(b.z, to1.x, co[1][2 * t + 1]); so[1][2 * t + 1] = fmaf(b.w, to1.y, so[1][2 * t + 1]);
-        }
-      }
+      if (m < M) add(m, ao);                   // last (odd) m
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int i = i0 + h * QH;
@@ -151,8 +172,9 @@ __global__ void __launch_bounds__(IDFT_NT) k_idft(SD<float> d, const float2* __r
           if (r0 + r >= nr) break;
           const int v = v0 + r0 + r;
           const float sc = rscale(v);
-          const float c0 = F[r0 + r].x + 2.f * ce[h][r], c1 = 2.f * co[h][r];
-          const float s0 = 2.f * se[h][r], s1 = 2.f * so[h][r];
+          const float2 e = ae[h][r].get(), o = ao[h][r].get();
+          const float c0 = F[r0 + r].x + 2.f * e.x, c1 = 2.f * o.x;
+          const float s0 = 2.f * e.y, s1 = 2.f * o.y;
           const float p = c0 + c1, mn = c0 - c1, s = s0 + s1, dd = s0 - s1;
           float* row = g6 + (size_t)v * I;
           row[i] = (p - s) * sc;
@@ -162,19 +184,25 @@ __global__ void __launch_bounds__(IDFT_NT) k_idft(SD<float> d, const float2* __r
         }
       }
     }
-    // i = 0 and i = I/2: one row per thread (consecutive rows, no bank conflicts)
-    for (int r = tid; r < nr; r += NT) {
+    // i = 0 and i = I/2: one row per thread (consecutive rows, no bank conflicts), on
+    // the warps that have fewer of the items above
+    constexpr int EDGE = !PAIR ? 0 : (QH * NGR % NT) / 32 * 32;
+    for (int r = tid - EDGE; r < nr; r += NT - EDGE) {
+      if (r < 0) break;
       float se_ = 0.f, so_ = 0.f;
-      for (int m = 1; m < M; ++m) {
-        const float a = F[m * RC + r].x;
-        if (m & 1) so_ += a;
-        else se_ += a;
+      int m = 1;
+#pragma unroll 4
+      for (; m + 1 < M; m += 2) {
+        so_ += F[m * RC + r].x;
+        se_ += F[(m + 1) * RC + r].x;
       }
+      if (m < M) so_ += F[m * RC + r].x;
       const int v = v0 + r;
       const float sc = rscale(v), x0 = F[r].x;
       g6[(size_t)v * I] = (x0 + 2.f * (se_ + so_)) * sc;
       g6[(size_t)v * I + I / 2] = (x0 + 2.f * (se_ - so_)) * sc;
     }
+    if (CHUNK) return;
     buf ^= 1;
     __syncthreads();
   }

@@ -518,6 +518,13 @@ inline int persistent_grid(const void* fn, int nt, size_t smem, int units) {
   return ctas < units ? ctas : units;
 }
 
+template <int I> void launch_idft(const SD<float>& d, cudaStream_t st) {
+  const size_t smem = idft_smem(I, d.M);
+  const int nz = (idft_rows(d.K) + IDFT_RC - 1) / IDFT_RC;
+  if (idft_chunks(d.E, d.J)) k_idft<I, true><<<dim3(d.J, d.E, nz), IDFT_NT, smem, st>>>(d, d.dft);
+  else k_idft<I, false><<<dim3(d.J, d.E), IDFT_NT, smem, st>>>(d, d.dft);
+}
+
 template <typename R, int I, int BT, int MINB>
 void launch_alg(const SD<R>& d, int ps_mode, cudaStream_t st, bool attrs) {
   const int LS = alg_seg<R>(d.E, d.J, I, d.K);
@@ -543,7 +550,7 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
     // grid-point part as three launches: longitude synthesis, column
     // algebra, longitude analysis (kernel ids 4, 5, 6; 0 = all three)
     if (only < 0 || only == 0 || only == 4)
-      k_idft<I><<<dim3(d.J, d.E), IDFT_NT, idft_smem(I, d.M), st>>>(d, d.dft);
+      launch_idft<I>(d, st);
     if (only < 0 || only == 0 || only == 5)
       launch_alg<R, I, I, alg_minb<I>()>(d, c.ps_mode, st, false);
     if ((only < 0 || only == 0 || only == 6) && d.legendre && !(d.tc_off & 4) &&
@@ -606,7 +613,9 @@ template <typename R, int I> void set_attrs(const SD<R>& d) {
   constexpr int KB = grid_kb<R, I>(), NT = grid_nt<R, I>();
   launch_alg<R, I, sizeof(R) == 4 ? I : 32, sizeof(R) == 4 ? alg_minb<I>() : 1>(d, 0, 0, true);
   if constexpr (sizeof(R) == 4) {
-    cudaFuncSetAttribute(k_idft<I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_idft<I, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)idft_smem(I, d.M));
+    cudaFuncSetAttribute(k_idft<I, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)idft_smem(I, d.M));
     const FdftPlan pl = fdft_plan(I, d.M, d.K);
     const size_t smem = sizeof(float) * (size_t)pl.total;

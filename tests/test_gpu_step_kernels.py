@@ -502,3 +502,34 @@ def test_longitude_analysis_against_fp64_sums(torch, I, J, N, K, nmem):
     for f in range(2):
         got = stp.afs[..., f].to(torch.complex128).permute(0, 2, 1)
         assert bool(((got - (wg * X)[:, :, f]).abs() <= (I + 16) * u * (wg * A)[:, :, f]).all())
+
+
+@pytest.mark.parametrize("I,J,N,K,nmem", [(64, 32, 21, 1, 1), (64, 32, 21, 20, 12), (64, 6, 31, 7, 1),
+                                          (128, 64, 42, 17, 5), (128, 64, 42, 20, 4),
+                                          (128, 64, 63, 3, 1), (256, 128, 85, 9, 2),
+                                          (256, 128, 127, 5, 3)])
+def test_longitude_synthesis_against_fp64_sums(torch, I, J, N, K, nmem):
+    """k_idft, a chunk of rows per block and whole columns, against FP64
+    transforms of the same coefficients.  Bound per value: 2 M + 16 operations
+    on terms that sum to the row's magnitudes."""
+    stp = _grid_stepper(torch, I, J, N, K, nmem, "fp32")
+    u, M = 2.0 ** -24, stp.M
+    _noise(torch, stp.sf, 1)
+    _noise(torch, stp.sfs, 2)
+    stp.grid6.zero_()
+    _launch(torch, stp, 4)
+    rcos = stp.jfac.double().reshape(4, J)[2][None, :, None, None]
+    S = stp.sfs.to(torch.complex128).permute(0, 2, 3, 1)       # [E][J][5][M]
+    F = stp.sf.to(torch.complex128).permute(0, 2, 3, 4, 1)     # [E][J][K][6][M]
+    m = torch.arange(M, device="cuda", dtype=torch.float64)
+    rows = [S[:, :, :1], 1j * m * S[:, :, :1] * rcos, S[:, :, 1:4] * rcos, S[:, :, 4:5]]
+    # surface fields: pi, H pi (pi_y), U-, V-, D-sum
+    lev = F.clone()
+    lev[:, :, :, :2] *= rcos[..., None]
+    X = torch.cat(rows + [lev.reshape(nmem, J, 6 * K, M)], 2)
+    want = torch.fft.irfft(X, n=I, dim=-1) * I
+    two = torch.full((M,), 2.0, device="cuda", dtype=torch.float64)
+    two[0] = 1.0
+    size = (X.abs() * two).sum(-1, keepdim=True)
+    err = (stp.grid6.double() - want).abs()
+    assert bool((err <= (2 * M + 16) * u * size).all()), float((err / size).max() / u)
