@@ -168,6 +168,7 @@ class EnsembleStepper:
         self.pn = torch.as_tensor(nn, device=dev)
         R = lambda x: x.to(device=dev, dtype=rd).contiguous()   # noqa: E731
         JH = J // 2
+        self.pmn = self.pm * self.M + self.pn      # flat index of the rectangle
         self.symp = R(sp.pnm[self.pm, self.pn, :JH])
         self.symh = R(sp.hnm[self.pm, self.pn, :JH])
         self.tw = R(sp._tw64)
@@ -297,34 +298,51 @@ class EnsembleStepper:
             self._drop_graphs()
             return
         Ef = self.E if per_member else 1
-        f3 = torch.zeros((Ef, 4, self.NS, self.K), device=self.dev, dtype=self.cd)
-        fs = torch.zeros((Ef, self.NS), device=self.dev, dtype=self.cd)
-        for i, x in enumerate((frc_vor, frc_div, frc_t, frc_q)):
-            if x is not None:           # (B, M, M, K), B = 1 or E
-                p = self.pack(x).reshape(-1, self.NS, self.K)
-                f3[:, i] = p.expand(Ef, self.NS, self.K)
-        if frc_pi is not None:          # (B, M, M)
-            p = self.pack(frc_pi).reshape(-1, self.NS)
-            fs[:] = p.expand(Ef, self.NS)
-        new_ptrs = self.frc3 is None
-        if self.frc3 is not None and self.frc3.shape == f3.shape:
-            # in place, ordered after the steps already queued on the stepper's
-            # stream (they may still read the old forcing)
-            self.stream.wait_stream(torch.cuda.current_stream(self.dev))
-            with torch.cuda.stream(self.stream):
-                self.frc3.copy_(f3)
-                self.frcs.copy_(fs)
-            f3.record_stream(self.stream)
-            fs.record_stream(self.stream)
-        else:
+        fields = (frc_vor, frc_div, frc_t, frc_q, frc_pi)
+        # gathered on the caller's stream: it may change its arrays once we return
+        packed = [None if x is None else self._gather(x, x is not frc_pi) for x in fields]
+        cur = torch.cuda.current_stream(self.dev)
+        new_ptrs = self.frc3 is None or self.frc3.shape[0] != Ef
+        if new_ptrs:
+            f3 = torch.zeros((Ef, 4, self.NS, self.K), device=self.dev, dtype=self.cd)
+            fs = torch.zeros((Ef, self.NS), device=self.dev, dtype=self.cd)
+            self._put_forcing(f3, fs, packed, ())
             # new buffers: the stepper's stream must see them written
-            self.stream.wait_stream(torch.cuda.current_stream(self.dev))
+            self.stream.wait_stream(cur)
             self.frc3, self.frcs = f3, fs
-            new_ptrs = True
+        else:
+            # in place, ordered after the steps already queued on the stepper's
+            # stream (they may still read the old forcing); a field without
+            # forcing is zeroed once
+            self.stream.wait_stream(cur)
+            with torch.cuda.stream(self.stream):
+                self._put_forcing(self.frc3, self.frcs, packed, self._forced)
+            for p in packed:
+                if p is not None:
+                    p.record_stream(self.stream)
+        self._forced = tuple(i for i, p in enumerate(packed) if p is not None)
         self.frc_shared = 0 if per_member else 1
         if new_ptrs:
             self._desc = None
             self._drop_graphs()
+
+    def _gather(self, x, has_k):
+        """(..., M, M[, K]) rectangle -> (B, NS[, K]) packed, precision of x."""
+        x = x.to(self.dev)
+        tail = (self.K,) if has_k else ()
+        if x.shape[-2 - len(tail):] != (self.M, self.M) + tail or not x.is_contiguous():
+            return self.pack(x).reshape(-1, self.NS, *tail)
+        return x.reshape(-1, self.M * self.M, *tail).index_select(1, self.pmn)
+
+    def _put_forcing(self, f3, fs, packed, forced):
+        """Packed fields into the forcing buffers, zeros into those of `forced`
+        (indices of the fields set before) that have none now."""
+        for i, p in enumerate(packed):
+            out = fs if i == 4 else f3[:, i]
+            if p is not None:
+                out.copy_(p.expand(out.shape))
+            elif i in forced:
+                out.zero_()
 
     # ------------------------------------------------------------------
     def pack(self, x):

@@ -533,3 +533,35 @@ def test_longitude_synthesis_against_fp64_sums(torch, I, J, N, K, nmem):
     size = (X.abs() * two).sum(-1, keepdim=True)
     err = (stp.grid6.double() - want).abs()
     assert bool((err <= (2 * M + 16) * u * size).all()), float((err / size).max() / u)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_forcings_set_in_turn_equal_fresh_ones(torch, precision):
+    """A stepper whose forcings change (fields added, dropped, shared by the
+    members, not contiguous, real) holds what a new stepper is given: the same values."""
+    K, E = 5, 3
+    one = _grid_stepper(torch, 64, 32, 21, K, E, precision)
+    M = one.M
+    g = torch.Generator().manual_seed(2)
+    f = lambda *s: torch.randn(s, generator=g, dtype=torch.float64).cuda()      # noqa: E731
+    c = lambda *s: torch.complex(f(*s), f(*s))                                  # noqa: E731
+    for kw in (dict(frc_t=c(E, M, M, K)), dict(frc_t=c(M, M, K), frc_pi=c(E, M, M)),
+               dict(frc_vor=c(E, M, M, K)), dict(frc_q=c(E, M, K, M).transpose(-1, -2)),
+               dict(frc_div=f(1, M, M, K), frc_pi=c(1, M, M).cpu())):
+        one.set_forcing(per_member=True, **kw)
+        fresh = _grid_stepper(torch, 64, 32, 21, K, E, precision)
+        fresh.set_forcing(per_member=True, **kw)
+        torch.cuda.synchronize()
+        assert torch.equal(one.frc3, fresh.frc3) and torch.equal(one.frcs, fresh.frcs)
+        for i, n in enumerate(("vor", "div", "t", "q")):
+            want = kw.get("frc_" + n)
+            if want is None:
+                assert not bool(one.frc3[:, i].any())
+            else:
+                want = want.reshape(-1, M, M, K)[:, one.pm, one.pn].to(one.cd)
+                assert torch.equal(one.frc3[:, i], want.expand(E, -1, -1))
+        if kw.get("frc_pi") is None:
+            assert not bool(one.frcs.any())
+        else:
+            want = kw["frc_pi"].cuda()[..., one.pm, one.pn].reshape(-1, one.NS).to(one.cd)
+            assert torch.equal(one.frcs, want.expand(E, -1))
