@@ -346,54 +346,62 @@ __global__ void __launch_bounds__(FTC_THREADS, 1)
 }
 
 // Surface rows (gt_pi, pi(t - dt)) of the longitude analysis on the FMA
-// pipes, rounded to nearest: one block per (latitude, FSURF_EB members), one
+// pipes, rounded to nearest: one block per (latitude, EB members), one
 // thread per lane L = 2m + c; W[L][i] read from an FP32 cos table (the sine
 // as cos(theta + pi / 2)), the members' rows staged [row][i][member] so that
-// a table value feeds 2 x FSURF_EB FMAs.  Writes afs = gw / I X, as k_fdft.
-constexpr int FSURF_EB = 8;
+// a table value feeds 2 EB FMAs.  Writes afs = gw / I X, as k_fdft.  Bound by the
+// latency of its loads: four points at a time; eight members a block, two while
+// those blocks would be fewer than two per SM.  us at T42, before -> after: 8 members
+// 17 -> 8.8, 512 members 87 either way; T21, 48 members 10 -> 6.5.
+inline int fsurf_eb(int E, int J) { return J * ((E + 7) / 8) < 2 * LF_SMS ? 2 : 8; }
+inline size_t fsurf_smem(int I, int EB) { return sizeof(float) * (size_t)I * (1 + 2 * EB); }
 
-inline size_t fsurf_smem(int I) { return sizeof(float) * (size_t)I * (1 + 2 * FSURF_EB); }
-
+template <int EB>
 __global__ void __launch_bounds__(128) k_fdft_surf(SD<float> d, const float* __restrict__ cs) {
   extern __shared__ float4 sh_fsurf[];
   float* tw = reinterpret_cast<float*>(sh_fsurf);
   const int I = d.I, J = d.J, M = d.M, E = d.E, R = 2 + 9 * d.K;
-  float* rows = tw + I;                                  // [2][I][FSURF_EB]
-  const int j = blockIdx.x, e0 = blockIdx.y * FSURF_EB;
+  float* rows = tw + I;                                  // [2][I][EB]
+  const int j = blockIdx.x, e0 = blockIdx.y * EB;
   for (int t = threadIdx.x; t < I; t += blockDim.x) tw[t] = cs[t];
-  for (int x = threadIdx.x; x < 2 * I * FSURF_EB; x += blockDim.x) {
+#pragma unroll 4
+  for (int x = threadIdx.x; x < 2 * I * EB; x += blockDim.x) {
     const int eb = x / (2 * I), rem = x - eb * 2 * I, r = rem / I, i = rem - r * I;
     const int e = e0 + eb;
-    rows[(r * I + i) * FSURF_EB + eb] =
+    rows[(r * I + i) * EB + eb] =
         e < E ? d.grid9[(((size_t)e * J + j) * R + r) * I + i] : 0.f;
   }
   __syncthreads();
   const int L = threadIdx.x, m = L >> 1, c = L & 1;
   if (m >= M) return;
   const int off = c ? I / 4 : 0;                         // -sin(t) = cos(t + pi / 2)
-  float acc[2][FSURF_EB];
+  float acc[2][EB];
 #pragma unroll
   for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int b = 0; b < FSURF_EB; ++b) acc[h][b] = 0.f;
+    for (int b = 0; b < EB; ++b) acc[h][b] = 0.f;
+#pragma unroll 4
   for (int i = 0; i < I; ++i) {
     const float w = tw[(m * i + off) & (I - 1)];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const float4* p = reinterpret_cast<const float4*>(rows + (size_t)(h * I + i) * FSURF_EB);
+      const float* p = rows + (size_t)(h * I + i) * EB;
+      __align__(16) float v[EB];
+      if constexpr (EB % 4 == 0) {
 #pragma unroll
-      for (int q = 0; q < FSURF_EB / 4; ++q) {
-        const float4 v = p[q];
-        acc[h][4 * q] = fmaf(w, v.x, acc[h][4 * q]);
-        acc[h][4 * q + 1] = fmaf(w, v.y, acc[h][4 * q + 1]);
-        acc[h][4 * q + 2] = fmaf(w, v.z, acc[h][4 * q + 2]);
-        acc[h][4 * q + 3] = fmaf(w, v.w, acc[h][4 * q + 3]);
+        for (int q = 0; q < EB; q += 4)
+          *reinterpret_cast<float4*>(v + q) = *reinterpret_cast<const float4*>(p + q);
+      } else {
+        static_assert(EB == 2, "");
+        *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(p);
       }
+#pragma unroll
+      for (int b = 0; b < EB; ++b) acc[h][b] = fmaf(w, v[b], acc[h][b]);
     }
   }
   const float wg = d.jfac[JF_GW * J + j] / float(I);
 #pragma unroll
-  for (int b = 0; b < FSURF_EB; ++b) {
+  for (int b = 0; b < EB; ++b) {
     const int e = e0 + b;
     if (e < E) {
       float* os = reinterpret_cast<float*>(d.afs) + ((((size_t)e * M + m) * J + j) * 2) * 2 + c;

@@ -560,8 +560,11 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
                   FTC_THREADS, pl.smem, st>>>(d, d.tc_dft, pl, d.legendre);
       // the surface rows on the FMA pipes; their FP32 cos table follows the
       // tensor-core image
-      k_fdft_surf<<<dim3(d.J, (d.E + FSURF_EB - 1) / FSURF_EB), 128, fsurf_smem(I), st>>>(
-          d, reinterpret_cast<const float*>(d.tc_dft + pl.tab_bytes));
+      const float* cs = reinterpret_cast<const float*>(d.tc_dft + pl.tab_bytes);
+      const int EB = fsurf_eb(d.E, d.J);
+      const dim3 g(d.J, (d.E + EB - 1) / EB);
+      if (EB == 2) k_fdft_surf<2><<<g, 128, fsurf_smem(I, 2), st>>>(d, cs);
+      else k_fdft_surf<8><<<g, 128, fsurf_smem(I, 8), st>>>(d, cs);
     } else if (only < 0 || only == 0 || only == 6) {
       const FdftPlan pl = fdft_plan(I, d.M, d.K);
       const size_t smem = sizeof(float) * (size_t)pl.total;

@@ -565,3 +565,26 @@ def test_forcings_set_in_turn_equal_fresh_ones(torch, precision):
         else:
             want = kw["frc_pi"].cuda()[..., one.pm, one.pn].reshape(-1, one.NS).to(one.cd)
             assert torch.equal(one.frcs, want.expand(E, -1))
+
+
+@pytest.mark.parametrize("K,nmem", [(8, 1), (20, 3), (20, 75)])
+def test_surface_rows_of_few_and_many_members(torch, K, nmem):
+    """k_fdft_surf with two members a block against eight: the same bits for a
+    member, and FP64 transforms within I + 16 roundings of the row's magnitudes."""
+    few = _grid_stepper(torch, 64, 32, 21, K, nmem, "bf16x3")
+    many = _grid_stepper(torch, 64, 32, 21, K, 83, "bf16x3")
+    assert few.legendre and few.tc_dft is not None
+    g = torch.Generator(device="cuda").manual_seed(K)
+    few.grid9.copy_(torch.randn(few.grid9.shape, generator=g, device="cuda"))
+    many.grid9.zero_()
+    many.grid9[-nmem:].copy_(few.grid9)
+    for s in (few, many):
+        s.afs.zero_()
+        _launch(torch, s, 6)
+    assert torch.equal(few.afs, many.afs[-nmem:])
+    x = few.grid9[:, :, :2].double()
+    wg = few.jfac.double().reshape(4, 32)[0][None, :, None, None] / 64
+    want = wg * torch.fft.rfft(x, dim=-1)[..., :few.M]
+    got = few.afs.to(torch.complex128).permute(0, 2, 3, 1)
+    size = wg * x.abs().sum(-1, keepdim=True)
+    assert bool(((got - want).abs() <= (64 + 16) * 2.0 ** -24 * 2 * size).all())
