@@ -11,7 +11,7 @@
 // k_grid), and 40-70 KB of shared memory keep two to four blocks per SM
 // resident where k_grid's level ring takes 185 KB.
 // Measured per step at T42L20 (grid part: these two and k_alg): 1 member
-// 675 -> 181 us (k_ifft 38, k_alg 82, k_ffft 60), 32 members 9.27 -> 2.95 ms
+// 675 -> 145 us (k_ifft 38, k_alg 47, k_ffft 60), 32 members 9.27 -> 2.95 ms
 // (0.80, 0.89, 1.26).
 #pragma once
 

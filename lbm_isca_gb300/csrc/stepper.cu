@@ -575,8 +575,8 @@ template <typename R, int I> int launch_step(const SD<R>& d, const lbm_step_ctl&
   } else if (only < 0 || only == 0) {
     if (d.grid6 && d.grid9) {
       // workspace for the grid rows: the grid part as three launches with
-      // enough blocks for one member (1 member of T42L20 675 -> 181 us, 32
-      // members 9.27 -> 2.93 ms)
+      // enough blocks for one member (1 member of T42L20 675 -> 145 us, 32
+      // members 9.27 -> 2.95 ms)
       using G = GridFft<I>;
       k_ifft<R, I><<<dim3(d.J, 1 + (d.K + G::LI - 1) / G::LI, d.E), G::NTI,
                      G::template ifft_smem<R>(d.M), st>>>(d);

@@ -579,11 +579,11 @@ class EnsembleStepper:
 
     def check_finite(self):
         """False when a member produced a non-finite value (bit 0 of err);
-        raises if a tensor-core kernel gave up a bounded wait (bit 1)."""
+        raises if a kernel gave up a bounded wait (bit 1)."""
         self.stream.synchronize()
         e = int(self.err.item())
         if e & 2:
-            raise RuntimeError("lbm_gb300: a tensor-core kernel timed out waiting for its "
+            raise RuntimeError("lbm_gb300: a kernel timed out waiting for its "
                                "pipeline (results of this run are invalid)")
         return (e & 1) == 0
 
