@@ -433,8 +433,9 @@ namespace lbm {
 // less than a warp per SM partition (one member of T42: 256 of 608).  Two
 // levels in FP32, bound by latency (T42L20, one member, us: 22 whole, 9.0, 10.6, 11.6
 // and 17 with 2, 3, 5, 10 levels); five in FP64, where the sums below a segment
-// cost more of the FP64 pipe (83 whole, 59, 50, 47, 52).  At seven members whole
-// columns win (19 against 21 to 35).
+// cost more of the FP64 pipe (83 whole, 59, 50, 47, 52).  At 512 warps FP32 19.7 ->
+// 15, FP64 84 either way; at 768 whole columns are as fast or faster (20.2 against
+// 20.4, 106 against 140).
 template <typename R> int alg_seg(int E, int J, int I, int K) {
   const long warps = (long)E * J * (I / 32);
   if (warps > 4 * LF_SMS || K < 2) return 0;
