@@ -331,7 +331,7 @@ class EnsembleStepper:
         x = x.to(self.dev)
         tail = (self.K,) if has_k else ()
         if x.shape[-2 - len(tail):] != (self.M, self.M) + tail or not x.is_contiguous():
-            return self.pack(x).reshape(-1, self.NS, *tail)
+            return self.pack(x, has_k).reshape(-1, self.NS, *tail)
         return x.reshape(-1, self.M * self.M, *tail).index_select(1, self.pmn)
 
     def _put_forcing(self, f3, fs, packed, forced):
@@ -345,12 +345,16 @@ class EnsembleStepper:
                 out.zero_()
 
     # ------------------------------------------------------------------
-    def pack(self, x):
-        """(..., M, M[, K]) rectangle -> (..., NS[, K]) packed, working precision."""
+    def pack(self, x, has_k=None):
+        """(..., M, M[, K]) rectangle -> (..., NS[, K]) packed, working precision.
+        has_k: whether x has a level axis; None takes it from the shape, which
+        does not tell (..., M, M) from (M, M, K) where K = M."""
         x = x.to(self.dev)
-        if x.shape[-2:] == (self.M, self.M):
-            return x[..., self.pm, self.pn].to(self.cd)
-        return x[..., self.pm, self.pn, :].to(self.cd)
+        if has_k is None:
+            has_k = x.shape[-2:] != (self.M, self.M)
+        if has_k:
+            return x[..., self.pm, self.pn, :].to(self.cd)
+        return x[..., self.pm, self.pn].to(self.cd)
 
     def unpack(self, p, has_k=True):
         lead = p.shape[:-2] if has_k else p.shape[:-1]
@@ -366,9 +370,9 @@ class EnsembleStepper:
         """Load the current level (spectral dict incl. pi), the previous level
         (spectral vor/div/t/q) and both grid ps' fields; member axis first."""
         for i, k in enumerate(("vor", "div", "t", "q")):
-            self.sa3[:, i] = self.pack(a_spec[k]).reshape(self.E, self.NS, self.K)
-            self.sb3[:, i] = self.pack(b_spec[k]).reshape(self.E, self.NS, self.K)
-        self.sas[:, 0] = self.pack(a_spec["pi"]).reshape(self.E, self.NS)
+            self.sa3[:, i] = self.pack(a_spec[k], True).reshape(self.E, self.NS, self.K)
+            self.sb3[:, i] = self.pack(b_spec[k], True).reshape(self.E, self.NS, self.K)
+        self.sas[:, 0] = self.pack(a_spec["pi"], False).reshape(self.E, self.NS)
         self.psa.copy_(psa.reshape(self.E, self.J, self.I))
         self.psb.copy_(psb.reshape(self.E, self.J, self.I))
         self.pending_ps_mode = 0

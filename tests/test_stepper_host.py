@@ -1,0 +1,62 @@
+"""Host side of the ensemble stepper on CPU tensors: packing of rectangles."""
+
+import contextlib
+import types
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture
+def host_stepper(monkeypatch):
+    """Makes EnsembleStepper objects that hold what packing and forcing need, on
+    the CPU, with torch's stream calls replaced by nothing."""
+    from lbm_isca_gb300.stepper import EnsembleStepper
+    null = types.SimpleNamespace(wait_stream=lambda other: None)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: null)
+    monkeypatch.setattr(torch.cuda, "default_stream", lambda *a: null)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+
+    def make(N, K, E):
+        s = object.__new__(EnsembleStepper)
+        s.dev, s.cd = torch.device("cpu"), torch.complex128
+        s.M, s.K, s.E, s.NS = N + 1, K, E, (N + 1) * (N + 2) // 2
+        s.pm, s.pn = torch.triu_indices(s.M, s.M)
+        s.pmn = s.pm * s.M + s.pn
+        s.stream, s.frc3, s.frcs, s._graphs, s._desc = null, None, None, {}, None
+        return s
+    monkeypatch.setattr(torch.Tensor, "record_stream", lambda self, s: None)
+    return make
+
+
+def _spec(g, *shape):
+    return torch.view_as_complex(torch.randn(*shape, 2, generator=g, dtype=torch.float64))
+
+
+def test_as_many_levels_as_wavenumbers(host_stepper):
+    """K = nmax + 1: a field's level axis is not taken for n, in the state and
+    in a forcing that is not contiguous."""
+    N, K, E = 4, 5, 3
+    s, g = host_stepper(N, K, E), torch.Generator().manual_seed(1)
+    x, pi = _spec(g, E, s.M, s.M, K), _spec(g, E, s.M, s.M)
+    want, want_pi = x[:, s.pm, s.pn, :], pi[:, s.pm, s.pn]
+    turned = x.permute(3, 2, 1, 0).contiguous().permute(3, 2, 1, 0)
+    assert torch.equal(s._gather(turned, True), want)
+    assert torch.equal(s._gather(x, True), want) and torch.equal(s._gather(pi, False), want_pi)
+    assert torch.equal(s.pack(pi), want_pi)
+
+    s.I = s.J = 2
+    s.sa3 = torch.zeros((E, 4, s.NS, K), dtype=s.cd)
+    s.sb3, s.sas = torch.zeros_like(s.sa3), torch.zeros((E, 4, s.NS), dtype=s.cd)
+    s.psa = s.psb = torch.zeros((E, 2, 2), dtype=torch.float64)
+    s.err, s.err_member = torch.zeros(1), torch.zeros(E)
+    s.op_args = lambda: ()
+    ops = types.SimpleNamespace(stepper_colsum=lambda: None, stepper_prime=lambda: None)
+    with pytest.MonkeyPatch.context() as mp:
+        mp.setattr(torch.ops, "lbm_gb300", ops, raising=False)
+        s.load({k: x for k in ("vor", "div", "t", "q")} | {"pi": pi},
+               {k: x for k in ("vor", "div", "t", "q")}, s.psa, s.psb)
+    for f in range(4):
+        assert torch.equal(s.sa3[:, f], want) and torch.equal(s.sb3[:, f], want)
+    assert torch.equal(s.sas[:, 0], want_pi)
