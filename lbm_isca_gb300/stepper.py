@@ -301,6 +301,10 @@ class EnsembleStepper:
         fields = (frc_vor, frc_div, frc_t, frc_q, frc_pi)
         # gathered on the caller's stream: it may change its arrays once we return
         packed = [None if x is None else self._gather(x, x is not frc_pi) for x in fields]
+        # to the buffers' sizes, which refuses a wrong one before the first write:
+        # a refused call leaves the forcing as it was
+        sizes = [(Ef, self.NS, self.K)] * 4 + [(Ef, self.NS)]
+        packed = [p if p is None else p.expand(n) for p, n in zip(packed, sizes)]
         cur = torch.cuda.current_stream(self.dev)
         new_ptrs = self.frc3 is None or self.frc3.shape[0] != Ef
         if new_ptrs:
@@ -335,12 +339,12 @@ class EnsembleStepper:
         return x.reshape(-1, self.M * self.M, *tail).index_select(1, self.pmn)
 
     def _put_forcing(self, f3, fs, packed, forced):
-        """Packed fields into the forcing buffers, zeros into those of `forced`
+        """Packed fields (of their sizes) into the forcing buffers, zeros into those of `forced`
         (indices of the fields set before) that have none now."""
         for i, p in enumerate(packed):
             out = fs if i == 4 else f3[:, i]
             if p is not None:
-                out.copy_(p.expand(out.shape))
+                out.copy_(p)
             elif i in forced:
                 out.zero_()
 

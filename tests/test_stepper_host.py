@@ -1,4 +1,5 @@
-"""Host side of the ensemble stepper on CPU tensors: packing of rectangles."""
+"""Host side of the ensemble stepper on CPU tensors: packing of rectangles,
+forcings."""
 
 import contextlib
 import types
@@ -60,3 +61,23 @@ def test_as_many_levels_as_wavenumbers(host_stepper):
     for f in range(4):
         assert torch.equal(s.sa3[:, f], want) and torch.equal(s.sb3[:, f], want)
     assert torch.equal(s.sas[:, 0], want_pi)
+
+
+@pytest.mark.parametrize("bad", [dict(frc_t=(3, True)), dict(frc_pi=(3, False)),
+                                 dict(frc_vor=(2, True), frc_q=(3, True))])
+def test_refused_forcing_leaves_the_old_one(host_stepper, bad):
+    """A call with a field of a wrong number of members raises and changes
+    nothing: neither the forcing in force nor what later calls leave."""
+    N, K, E = 4, 3, 2
+    s, g = host_stepper(N, K, E), torch.Generator().manual_seed(2)
+    first = _spec(g, E, s.M, s.M, K)
+    s.set_forcing(frc_t=first, per_member=True)
+    f3, fs = s.frc3.clone(), s.frcs.clone()
+    fields = dict(frc_vor=_spec(g, E, s.M, s.M, K), frc_pi=_spec(g, E, s.M, s.M))
+    fields.update({k: _spec(g, n, s.M, s.M, *([K] if has_k else [])) for k, (n, has_k) in
+                   bad.items()})
+    with pytest.raises(RuntimeError):
+        s.set_forcing(per_member=True, **fields)
+    assert torch.equal(s.frc3, f3) and torch.equal(s.frcs, fs)
+    s.set_forcing(frc_t=first, per_member=True)
+    assert torch.equal(s.frc3, f3) and torch.equal(s.frcs, fs)
