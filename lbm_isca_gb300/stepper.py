@@ -268,6 +268,7 @@ class EnsembleStepper:
         dts = [float(x) for x in dts]
         if dts == self._dts:
             return
+        self._retire(self.minv, self.vdm)
         K, M = self.K, self.M
         mins, vds = [], []
         for dt in dts:
@@ -288,10 +289,18 @@ class EnsembleStepper:
     def set_index(self, dt):
         return self._dts.index(float(dt))
 
+    def _retire(self, *buffers):
+        """Before buffers are dropped that steps still queued on the stepper's
+        stream may read: their memory is not reused ahead of those."""
+        for t in buffers:
+            if t is not None:
+                t.record_stream(self.stream)
+
     def set_forcing(self, frc_vor=None, frc_div=None, frc_t=None, frc_pi=None, frc_q=None,
                     per_member=False):
         """Spectral forcings, rectangle layout ((E,) M, M, K) / ((E,) M, M)."""
         if all(x is None for x in (frc_vor, frc_div, frc_t, frc_pi, frc_q)):
+            self._retire(self.frc3, self.frcs)
             self.frc3 = self.frcs = None
             self.frc_shared = 1
             self._desc = None
@@ -313,6 +322,7 @@ class EnsembleStepper:
             self._put_forcing(f3, fs, packed, ())
             # new buffers: the stepper's stream must see them written
             self.stream.wait_stream(cur)
+            self._retire(self.frc3, self.frcs)
             self.frc3, self.frcs = f3, fs
         else:
             # in place, ordered after the steps already queued on the stepper's

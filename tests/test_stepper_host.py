@@ -81,3 +81,28 @@ def test_refused_forcing_leaves_the_old_one(host_stepper, bad):
     assert torch.equal(s.frc3, f3) and torch.equal(s.frcs, fs)
     s.set_forcing(frc_t=first, per_member=True)
     assert torch.equal(s.frc3, f3) and torch.equal(s.frcs, fs)
+
+
+def test_replaced_buffers_outlive_the_queued_steps(host_stepper, monkeypatch):
+    """Forcing and operator buffers belong to the caller's stream, queued steps
+    read them on the stepper's: each set is recorded there before it is dropped."""
+    N, K, E = 4, 3, 2
+    s, g = host_stepper(N, K, E), torch.Generator().manual_seed(3)
+    kept = []
+    monkeypatch.setattr(torch.Tensor, "record_stream",
+                        lambda t, st: kept.append((t.data_ptr(), st)))
+    shared, per = _spec(g, s.M, s.M, K), _spec(g, E, s.M, s.M, K)
+    s.set_forcing(frc_t=shared)
+    for change in (lambda: s.set_forcing(frc_t=per, per_member=True), s.set_forcing):
+        old = [t.data_ptr() for t in (s.frc3, s.frcs)]
+        change()
+        assert {(p, s.stream) for p in old} <= set(kept)
+
+    one = torch.eye(K, dtype=torch.float64)
+    s.rd, s._dts, s.minv, s.vdm = torch.float64, [], None, None
+    s.semi = types.SimpleNamespace(matrices=lambda dt: (None, one.expand(s.M, K, K), None))
+    s.vdiff = types.SimpleNamespace(operators=lambda dt: dict.fromkeys(("vor", "div", "t", "q")))
+    s.set_timesteps([600.0])
+    old = [t.data_ptr() for t in (s.minv, s.vdm)]
+    s.set_timesteps([1200.0])
+    assert {(p, s.stream) for p in old} <= set(kept)
