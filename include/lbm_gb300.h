@@ -296,6 +296,9 @@ int lbm_implicit_step_adjoint(int prec, const lbm_implicit_adj_args* a, void* st
  *        cos(2 pi t / nlon), t = 0..nlon-1, the table of the two surface
  *        rows, which stay on the FMA pipes
  * sf, af and grid9 must be 16-byte aligned (LBM_ERR_ARG otherwise).
+ * Grids whose tables exceed a block's shared memory (227 KB) are refused by
+ * prime, run, launch and capture (LBM_ERR_ARG); which ones does not depend on
+ * nmem.
  * ==========================================================================*/
 enum {
   LBM_VERT_DSIG = 0, LBM_VERT_SIGM, LBM_VERT_ALPHA, LBM_VERT_W3, LBM_VERT_WP,

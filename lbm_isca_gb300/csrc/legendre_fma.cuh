@@ -667,13 +667,16 @@ template <typename R> void launch_anal(const SD<R>& d, cudaStream_t st, bool att
 struct SynthPlan {
   int NJG, NJQ, QC, nch, nt, eb;      // latitude groups, quads of them, level quads per block,
                                       //   chunks, threads, members per block
-  int jhp, bufs, oil, ox;             // table row stride, state buffers, byte offsets of the
-                                      //   inverse Laplacian factors and of the state
+  int jhp, ntab, bufs, oil, ox;       // table row stride, tables, state buffers, byte offsets
+                                      //   of the inverse Laplacian factors and of the state
   unsigned smem;
 };
 template <typename R> struct SynthCfg;
 // FP64 folds the inverse Laplacian factor into the tables (P, P il, H il) instead
-// of scaling each coefficient: four of twenty FP64 operations per row less.
+// of scaling each coefficient: four of twenty FP64 operations per row less.  Where
+// the third table leaves no room for a level quad of one member ((nmax + 2)
+// (nlat / 2 + 11) above 9,685) there are two, as in FP32: by the grid alone, so that
+// a member's results do not depend on the ensemble.
 template <> struct SynthCfg<float> { static constexpr int JG = 4, NW = 10, NTAB = 2; };
 template <> struct SynthCfg<double> { static constexpr int JG = 1, NW = 8, NTAB = 3; };
 
@@ -694,19 +697,28 @@ template <typename R> SynthPlan synth_plan(int E, int J, int K, int N) {
   int want = (2 * LF_SMS + NP * E - 1) / (NP * E);
   if (want > nq) want = nq;
   if (nch < want) nch = want;
-  const size_t tabs = sizeof(R) * SynthCfg<R>::NTAB * NR * (size_t)p.jhp;
+  auto layout = [&](int ntab, int qc_, int bufs) {
+    const int kc = 4 * qc_ < K ? 4 * qc_ : K;
+    p.ntab = ntab;
+    p.bufs = bufs;
+    p.oil = (int)((sizeof(R) * ntab * NR * (size_t)p.jhp + 15) & ~size_t(15));
+    p.ox = (int)((p.oil + sizeof(R) * NR + 15) & ~size_t(15));
+    size_t x = bufs * C * NR * 4 * (size_t)kc;
+    if (x < C * NR * 4) x = C * NR * 4;                      // the surface fields
+    p.smem = (unsigned)(p.ox + x);
+    return p.smem;
+  };
+  const int ntab = layout(SynthCfg<R>::NTAB, 1, 1) <= 227 * 1024 ? SynthCfg<R>::NTAB : 2;
   for (;; ++nch) {
     p.QC = (nq + nch - 1) / nch;
     p.nch = (nq + p.QC - 1) / p.QC;
     p.eb = members_per_block(E, NP * p.nch);
-    p.bufs = p.eb > 1 ? 2 : 1;
-    const int kc = 4 * p.QC < K ? 4 * p.QC : K;
-    p.oil = (int)((tabs + 15) & ~size_t(15));
-    p.ox = (int)((p.oil + sizeof(R) * NR + 15) & ~size_t(15));
-    size_t x = p.bufs * C * NR * 4 * (size_t)kc;
-    if (x < C * NR * 4) x = C * NR * 4;                      // the surface fields
-    p.smem = (unsigned)(p.ox + x);
-    if (p.smem <= 113 * 1024 || p.QC == 1) break;
+    if (layout(ntab, p.QC, p.eb > 1 ? 2 : 1) <= 113 * 1024 || p.QC == 1) break;
+  }
+  // one member a block where two buffers do not fit
+  if (p.smem > 227 * 1024) {
+    p.eb = 1;
+    layout(ntab, p.QC, 1);
   }
   const int w = p.NJQ * p.QC;
   p.nt = 32 * (w < NW ? w : NW);
@@ -715,21 +727,21 @@ template <typename R> SynthPlan synth_plan(int E, int J, int K, int N) {
   return p;
 }
 
-// Tables of the pair's rows, [NR][JHp], zero past the equator: P and H, or for the
-// level fields in FP64 P, P il and H il.
-template <typename R, bool SURF>
+// Tables of the pair's rows, [NR][JHp], zero past the equator: P and H, or P, P il
+// and H il.
+template <typename R, int NTAB>
 LBM_D void synth_tables(const SD<R>& d, const PairRows<R>& pr, R* tp, int JHp) {
   const int JH = d.J / 2, off1 = spec_offset(pr.m1, d.N), off2 = spec_offset(pr.m2, d.N);
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, TT = (d.N + 2) * JHp;
 #pragma unroll 2
   for (int r = threadIdx.x >> 5; r < pr.NR; r += nw) {
     const size_t o = (size_t)(r < pr.L1 ? off1 + r : off2 + (r - pr.L1)) * JH;
-    const R il = sizeof(R) == 8 && !SURF ? d.invlap[pr.n_of(r)] : R(1);
+    const R il = NTAB == 3 ? d.invlap[pr.n_of(r)] : R(1);
     for (int jh = lane; jh < JHp; jh += 32) {
       const R P = jh < JH ? d.symp[o + jh] : R(0), H = jh < JH ? d.symh[o + jh] : R(0);
       R* t = tp + r * JHp + jh;
       t[0] = P;
-      if constexpr (sizeof(R) == 8 && !SURF) {
+      if constexpr (NTAB == 3) {
         t[TT] = P * il;
         t[2 * TT] = H * il;
       } else {
@@ -804,7 +816,7 @@ __global__ void __launch_bounds__(128) k_synth_surf(SD<float> d, SynthPlan pl, i
   const PairRows<float> pr(blockIdx.x, d.N);
   const int e0 = blockIdx.y * eb;
   float* tp = reinterpret_cast<float*>(smraw);
-  synth_tables<float, true>(d, pr, tp, pl.jhp);
+  synth_tables<float, 2>(d, pr, tp, pl.jhp);
   synth_surface(d, blockIdx.x, e0, min(d.E, e0 + eb), tp, tp + (d.N + 2) * pl.jhp, pl.jhp,
                 reinterpret_cast<C2<float>*>(smraw + pl.ox));
 }
@@ -827,6 +839,7 @@ LBM_D unsigned long long scale_c(unsigned long long x, unsigned long long il) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(il));
   return r;
 }
+LBM_D C2<double> scale_c(C2<double> x, double il) { return x * il; }
 
 // Block (m-pair, eb members, chunk of QC level quads); chunk index 0 is the
 // surface block.  A member's rows are staged as they lie in the state
@@ -837,7 +850,7 @@ LBM_D unsigned long long scale_c(unsigned long long x, unsigned long long il) {
 // us at T42L20 against one thread item for both parities before: FP32 11 (21), 159
 // (208), 573 (784) at 1, 128, 512 members; T85L40, 16 members 225 (383); FP64 41
 // (98), 682 (641) at 1, 32 members.
-template <typename R, int MINB>
+template <typename R, int MINB, int NTAB>
 __global__ void __launch_bounds__(32 * SynthCfg<R>::NW, MINB) k_synth(SD<R> d, SynthPlan pl) {
   constexpr int JG = SynthCfg<R>::JG;
   using V = typename Cval<R>::T;
@@ -849,11 +862,11 @@ __global__ void __launch_bounds__(32 * SynthCfg<R>::NW, MINB) k_synth(SD<R> d, S
   R* tp = reinterpret_cast<R*>(smraw);                       // [NTAB][NR][JHp]
   C2<R>* buf = reinterpret_cast<C2<R>*>(smraw + pl.ox);      // [bufs][NR][4][kn]
   if (blockIdx.z == 0) {                                     // first, so that no tail is left
-    synth_tables<R, true>(d, pr, tp, JHp);
+    synth_tables<R, 2>(d, pr, tp, JHp);
     synth_surface(d, p, e0, e1, tp, tp + TT, JHp, buf);
     return;
   }
-  R* ils = reinterpret_cast<R*>(smraw + pl.oil);             // inverse Laplacian of row r (FP32)
+  R* ils = reinterpret_cast<R*>(smraw + pl.oil);             // inverse Laplacian of row r
   const int k0 = ((int)blockIdx.z - 1) * 4 * pl.QC, kn = min(4 * pl.QC, K - k0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const int off1 = spec_offset(pr.m1, N), off2 = spec_offset(pr.m2, N);
@@ -880,7 +893,7 @@ __global__ void __launch_bounds__(32 * SynthCfg<R>::NW, MINB) k_synth(SD<R> d, S
     cp_async_commit();
   };
   issue(e0, buf);
-  synth_tables<R, false>(d, pr, tp, JHp);
+  synth_tables<R, NTAB>(d, pr, tp, JHp);
   for (int r = tid; r < pr.NR; r += blockDim.x) ils[r] = d.invlap[pr.n_of(r)];
   const int par = lane >> 4, nm = pr.L2 ? 2 : 1, nq = (kn + 3) / 4;
   const R sg = par ? R(-1) : R(1);
@@ -919,7 +932,18 @@ __global__ void __launch_bounds__(32 * SynthCfg<R>::NW, MINB) k_synth(SD<R> d, S
           ld1(s + kn, dv);
           ld1(s + 2 * kn, tt);
           ld1(s + 3 * kn, qq);
-          if constexpr (JG == 4) {
+          if constexpr (NTAB == 2 && JG == 1) {
+            const R P = pp[0], H = pp[TT], il = ils[r];
+            const V psi = scale_c(vo, il), chi = scale_c(dv, il);
+            acc[0][0].fma(P, chi);
+            acc[0][1].fma(H, psi);
+            acc[0][2].fma(P, psi);
+            acc[0][3].fma(H, chi);
+            acc[0][4].fma(P, vo);
+            acc[0][5].fma(P, dv);
+            acc[0][6].fma(P, tt);
+            acc[0][7].fma(P, qq);
+          } else if constexpr (NTAB == 2) {
             const auto il = Cacc<R>::fac(ils[r]);
             const V psi = scale_c(vo, il), chi = scale_c(dv, il);
             const float4 u = *reinterpret_cast<const float4*>(pp);

@@ -470,10 +470,18 @@ template <typename R> void launch_synth(const SD<R>& d, cudaStream_t st, bool at
       return;
     }
   }
-  if (attrs)
-    cudaFuncSetAttribute(k_synth<R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp.smem);
-  else
-    k_synth<R, 2><<<dim3(NP, (d.E + sp.eb - 1) / sp.eb, sp.nch + 1), sp.nt, sp.smem, st>>>(d, sp);
+  auto go = [&](auto kern) {
+    if (attrs)
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp.smem);
+    else
+      kern<<<dim3(NP, (d.E + sp.eb - 1) / sp.eb, sp.nch + 1), sp.nt, sp.smem, st>>>(d, sp);
+  };
+  if constexpr (sizeof(R) == 4) {
+    go(k_synth<R, 2, 2>);
+  } else {
+    if (sp.ntab == 3) go(k_synth<R, 2, 3>);
+    else go(k_synth<R, 2, 2>);
+  }
 }
 // Implicit update: 8- / 16-byte accesses where every complex array is so aligned.
 template <typename R> void launch_implicit(const SD<R>& d, R dt, int set, int ra_mode,
@@ -728,10 +736,24 @@ template <typename R> int launch_one(const lbm_stepper_desc* desc, const lbm_ste
   }
 }
 
+// Whether the plans of the Legendre kernels in use and of the implicit update fit a
+// block's shared memory (those of the other kernels: validate).
+template <typename R> bool plans_fit(const SD<R>& d) {
+  const size_t most = 227 * 1024;
+  const bool tc_anal = d.legendre && !(d.tc_off & 1), tc_synth = d.legendre && !(d.tc_off & 2);
+  const SynthPlan sp = synth_plan<R>(d.E, d.J, d.K, d.N);
+  const size_t anal = tc_anal ? anal_surf_smem(d.J, d.N)
+                              : anal_plan<R>(d.E, d.J, d.K, d.N).smem;
+  const size_t synth = tc_synth ? sp.ox + sizeof(C2<R>) * 4 * (d.N + 2) : sp.smem;
+  return anal <= most && synth <= most &&
+         impl_smem<R>(d.K, impl_plan(d.E, d.K, d.N).CC) <= most;
+}
+
 template <typename R> int prepare_attrs(const lbm_stepper_desc* desc) {
   const SD<R> d = make_sd<R>(*desc);
   int rc = validate(d);
   if (rc) return rc;
+  if (!plans_fit(d)) return LBM_ERR_ARG;
   switch (d.I) {
     case 64: set_attrs<R, 64>(d); break;
     case 128: set_attrs<R, 128>(d); break;
