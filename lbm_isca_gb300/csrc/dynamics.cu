@@ -249,8 +249,7 @@ int lbm_tendency_grid(int prec, const lbm_tend_grid_args* a, void* stream) {
   const int CB = TG_THREADS / a->kmax;
   const unsigned blocks = (unsigned)((cols + CB - 1) / CB);
   auto go = [&](auto kern, size_t smem) {
-    // one limit for all level counts: other threads and captured launches rely on it
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (smem > 48 * 1024) allow_smem(kern);   // (any kernel may have 48 KB)
     kern<<<blocks, TG_THREADS, smem, (cudaStream_t)stream>>>(*a);
   };
   if (prec == LBM_F64)

@@ -100,6 +100,16 @@ LBM_HD int nspec(int N) { return (N + 1) * (N + 2) / 2; }
 
 template <typename R> LBM_D R ld(const R* p) { return __ldg(p); }
 
+// Raises a kernel's dynamic shared memory limit to all that a block can have beside
+// the kernel's `fixed` bytes of static arrays.  The limit is one per kernel and
+// device: set to a launch's own size, it would be lowered by the next caller under
+// the launches of other plans, of other threads and of graphs being recorded
+// (which set no limits).
+constexpr int SMEM_BLOCK = 227 * 1024;
+template <typename F> inline void allow_smem(F kern, int fixed = 0) {
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BLOCK - fixed);
+}
+
 }  // namespace lbm
 
 // Launch-error check shared by the C-ABI entry points.

@@ -645,7 +645,7 @@ template <typename R> void launch_anal(const SD<R>& d, cudaStream_t st, bool att
   const int grid = pl.units < LF_SMS ? pl.units : LF_SMS;
   auto go = [&](auto kern) {
     if (attrs)
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+      allow_smem(kern);
     else
       kern<<<grid, 32 * (pl.CW + pl.HW + AN_FW), pl.smem, st>>>(d, pl);
   };

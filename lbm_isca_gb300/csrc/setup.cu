@@ -227,9 +227,7 @@ int lbm_batched_inverse(int batch, int n, const double* a, double* ainv, int* in
                         void* stream) {
   if (batch < 1 || n < 1 || n > 64 || !a || !ainv || !info) return LBM_ERR_ARG;
   const size_t smem = (size_t)n * 2 * n * sizeof(double);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_gauss_jordan, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+  if (smem > 48 * 1024) allow_smem(k_gauss_jordan, 1024);   // (static: the pivot)
   k_gauss_jordan<<<batch, 64, smem, (cudaStream_t)stream>>>(n, a, ainv, info);
   LBM_LAUNCH_CHECK();
   return LBM_OK;

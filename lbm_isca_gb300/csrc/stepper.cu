@@ -460,7 +460,7 @@ template <typename R> void launch_synth(const SD<R>& d, cudaStream_t st, bool at
       const StcPlan pl = stc_plan(d.E, d.J, d.K, d.N, d.tc_g);
       const int sm = sp.ox + (int)sizeof(C2<R>) * 4 * (d.N + 2);
       if (attrs) {
-        cudaFuncSetAttribute(k_synth_surf, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        allow_smem(k_synth_surf);
         return;
       }
       k_synth_tc<<<persistent_grid((const void*)k_synth_tc, STC_THREADS, pl.smem, pl.nunits),
@@ -472,7 +472,7 @@ template <typename R> void launch_synth(const SD<R>& d, cudaStream_t st, bool at
   }
   auto go = [&](auto kern) {
     if (attrs)
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp.smem);
+      allow_smem(kern);
     else
       kern<<<dim3(NP, (d.E + sp.eb - 1) / sp.eb, sp.nch + 1), sp.nt, sp.smem, st>>>(d, sp);
   };
@@ -492,7 +492,7 @@ template <typename R> void launch_implicit(const SD<R>& d, R dt, int set, int ra
                         (uintptr_t)d.frc3;
   auto go = [&](auto kern) {
     if (attrs)
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      allow_smem(kern);
     else
       kern<<<dim3((d.M + 1) / 2, d.E, pl.nch), pl.nt, smem, st>>>(d, dt, set, ra_mode, pl.CC);
   };
@@ -625,37 +625,31 @@ template <typename R, int I> void set_attrs(const SD<R>& d) {
   constexpr int KB = grid_kb<R, I>(), NT = grid_nt<R, I>();
   launch_alg<R, I, sizeof(R) == 4 ? I : 32, sizeof(R) == 4 ? alg_minb<I>() : 1>(d, 0, 0, true);
   if constexpr (sizeof(R) == 4) {
-    cudaFuncSetAttribute(k_idft<I, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)idft_smem(I, d.M));
-    cudaFuncSetAttribute(k_idft<I, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)idft_smem(I, d.M));
+    allow_smem(k_idft<I, false>);
+    allow_smem(k_idft<I, true>);
     const FdftPlan pl = fdft_plan(I, d.M, d.K);
     const size_t smem = sizeof(float) * (size_t)pl.total;
     if (smem <= 227 * 1024) {
-      cudaFuncSetAttribute(k_fdft<I>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      allow_smem(k_fdft<I>);
       persistent_grid((const void*)k_fdft<I>, pl.nt, smem, 1);
     }
     if (d.legendre && ftc_supported(I, d.K, d.N)) {
       const FtcPlan fp = ftc_plan(d.E, d.J, I, d.K, d.N);
-      cudaFuncSetAttribute(k_fdft_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp.smem);
+      allow_smem(k_fdft_tc);
       persistent_grid((const void*)k_fdft_tc, FTC_THREADS, fp.smem, 1);
     }
   } else {
-    cudaFuncSetAttribute(k_grid<R, I, KB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)GridSmem<R, I, KB, NT>::bytes(d.M));
-    cudaFuncSetAttribute(k_ifft<R, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)GridFft<I>::template ifft_smem<R>(d.M));
-    cudaFuncSetAttribute(k_ffft<R, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)GridFft<I>::template ffft_smem<R>(d.M));
+    allow_smem(k_grid<R, I, KB, NT>);
+    allow_smem(k_ifft<R, I>);
+    allow_smem(k_ffft<R, I>);
   }
   launch_anal<R>(d, nullptr, true);
   launch_synth<R>(d, nullptr, true);
   if constexpr (sizeof(R) == 4) {
     if (d.legendre) {
       const AtcPlan pl = atc_plan(d.E, d.J, d.K, d.N, d.tc_g);
-      cudaFuncSetAttribute(k_anal_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
-      cudaFuncSetAttribute(k_anal_surf, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)anal_surf_smem(d.J, d.N));
+      allow_smem(k_anal_tc);
+      allow_smem(k_anal_surf);
       persistent_grid((const void*)k_anal_tc, ATC_THREADS, pl.smem, 1);
     }
   }
@@ -663,7 +657,7 @@ template <typename R, int I> void set_attrs(const SD<R>& d) {
   if constexpr (sizeof(R) == 4) {
     if (d.legendre) {
       const StcPlan pl = stc_plan(d.E, d.J, d.K, d.N, d.tc_g);
-      cudaFuncSetAttribute(k_synth_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+      allow_smem(k_synth_tc);
       persistent_grid((const void*)k_synth_tc, STC_THREADS, pl.smem, 1);
     }
   }

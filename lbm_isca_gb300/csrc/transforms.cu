@@ -268,13 +268,11 @@ int launch_fourier(bool fwd, int B, int J, int C, int M, const void* in, const v
                       sizeof(R) * FT_COLS * (I + 1);
   dim3 grid(J, B, (C + FT_COLS - 1) / FT_COLS);
   if (fwd) {
-    cudaFuncSetAttribute(k_fourier_fwd<R, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+    allow_smem(k_fourier_fwd<R, I>);
     k_fourier_fwd<R, I><<<grid, FT_THREADS, smem, st>>>(
         J, C, M, (const R*)in, (const R*)js, (const C2<R>*)tw, (C2<R>*)out);
   } else {
-    cudaFuncSetAttribute(k_fourier_inv<R, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+    allow_smem(k_fourier_inv<R, I>);
     k_fourier_inv<R, I><<<grid, FT_THREADS, smem, st>>>(
         J, C, M, (const C2<R>*)in, (const R*)js, (const C2<R>*)tw, (R*)out);
   }
@@ -295,12 +293,6 @@ int fourier_dispatch(bool fwd, int B, int J, int I, int C, int nmax, const void*
   }
 }
 
-// The kernel's dynamic shared memory limit: always the same value, since other
-// threads and captured launches rely on it with sizes of their own.
-template <typename F> void leg_allow(F kern) {
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-}
-
 template <typename R>
 static int leg_anal(int B, int nmax, int J, int C, const void* fa, const void* ta, int ima,
                     const void* fb, const void* tb, int imb, double sb, const void* nfac,
@@ -311,7 +303,7 @@ static int leg_anal(int B, int nmax, int J, int C, const void* fa, const void* t
   const int CC = leg_cols(C), nch = (C + CC - 1) / CC;
   const dim3 grid(M, B, nch * ((M * CC + LG_NT - 1) / LG_NT));
   const size_t smem = leg_smem<R>(C, CC, M, LG_NT);
-  leg_allow(k_leg_anal<R>);
+  allow_smem(k_leg_anal<R>);
   k_leg_anal<R><<<grid, LG_NT, smem, st>>>(
       M, J, C, CC, nch, (const C2<R>*)fa, (const R*)ta, ima, (const C2<R>*)fb, (const R*)tb, imb,
       R(sb), (const R*)nfac, acc, (C2<R>*)spec);
@@ -331,7 +323,7 @@ static int leg_synth(int B, int nmax, int J, int C, const void* sa, const void* 
   const int nt = (long)M * B * nch * big >= 8 * LG_SMS ? LG_NTMAX : LG_NT;
   const dim3 grid(M, B, nch * ((J * CC + nt - 1) / nt));
   const size_t smem = leg_smem<R>(C, CC, J, nt);
-  leg_allow(k_leg_synth<R>);
+  allow_smem(k_leg_synth<R>);
   k_leg_synth<R><<<grid, nt, smem, st>>>(
       M, J, C, CC, nch, (const C2<R>*)sa, (const R*)ta, ima, (const R*)na, (const C2<R>*)sbp,
       (const R*)tb, imb, (const R*)nb, R(sb), (C2<R>*)four);

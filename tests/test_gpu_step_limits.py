@@ -1,10 +1,12 @@
 """The fused step where its plans and buffers meet a limit: grids that fill a
-block's shared memory."""
+block's shared memory, steppers of different sizes side by side."""
 
 import ctypes as C
+import threading
 
 import pytest
 
+from lbm_isca_gb300 import configs
 from test_gpu_step_kernels import (_grid_stepper,
                                    test_legendre_kernels_against_fp64_sums as _legendre_sums)
 
@@ -40,3 +42,82 @@ def test_a_grid_beyond_shared_memory_is_refused(torch, precision, nlat):
     ctl = stp._ctl([(stp._dts[0], False, 0)])
     assert lib().lbm_stepper_prime(C.byref(d), s) == LBM_ERR_ARG
     assert lib().lbm_stepper_run(C.byref(d), ctl, 1, s) == LBM_ERR_ARG
+
+
+SIDE_BY_SIDE = [  # grid, levels, members of two groups; each kernel's launches need the
+                  # more shared memory in the first group of one of them
+    [("T42", 20, 128), ("T42", 20, 8)], [("T42", 20, 32), ("T42", 20, 1)],
+    [("T42", 20, 1), ("T42", 20, 32)], [("T42", 20, 32), ("T21", 20, 48)],
+    [("T42", 20, 128), ("T85", 40, 1)]]
+GRIDS = {"T21": (64, 32, 21), "T42": (128, 64, 42), "T85": (256, 128, 85)}
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64", "bf16split"])
+@pytest.mark.parametrize("sizes", SIDE_BY_SIDE)
+def test_groups_of_any_order_and_size(torch, sizes, precision):
+    """One graph records the steps of all groups: no group's launches depend on
+    the plans of the others.  Each group equals itself alone."""
+    from lbm_isca_gb300.grouped import GroupedEnsemble
+    groups = []
+    for name, K, E in sizes:
+        I, J, N = GRIDS[name]
+        sigm = configs.equal_sigma_half_levels(K)
+        heats, _ = configs.ensemble_heating(I, J, sigm, E, seed=5)
+        groups.append(dict(nlon=I, nlat=J, nmax=N, sigm=sigm, heats=heats,
+                           basic_state=configs.solid_body_basic_state(I, J, sigm),
+                           config=configs.plain_damping(K)))
+    together = GroupedEnsemble(groups, precision=precision, tune=False).run(4)
+    assert together.check_finite()
+    for g, state in zip(groups, together.spectral_states()):
+        alone = GroupedEnsemble([g], precision=precision, tune=False).run(4)
+        assert float(state["t"].abs().max()) > 0
+        for k, x in alone.spectral_states()[0].items():
+            assert torch.equal(x, state[k]), k
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_steppers_on_two_threads(torch, precision):
+    """Two host threads step ensembles of different sizes, launch by launch:
+    the same state as one after the other."""
+    steps = [(600.0, False)] * 150
+    pair = [_grid_stepper(torch, 128, 64, 42, 20, E, precision) for E in (32, 1)]
+    g = torch.Generator().manual_seed(4)
+    heat = torch.zeros((43, 43, 20), dtype=torch.complex128)
+    heat[:6, 5:9] = torch.view_as_complex(
+        torch.randn((6, 4, 20, 2), generator=g, dtype=torch.float64)) * 1e-6
+    heat[0] = heat[0].real.clone()
+    for s in pair:
+        s.set_forcing(frc_t=heat.cuda())
+
+    def start():
+        for s in pair:
+            s.load_zero()
+        torch.cuda.synchronize()
+
+    def state():
+        torch.cuda.synchronize()
+        return [s.sa3.clone() for s in pair]
+
+    start()
+    for s in pair:
+        s.run(steps, use_graph=False)
+    want = state()
+    for x in want:
+        assert bool(torch.isfinite(torch.view_as_real(x)).all()) and float(x.abs().max()) > 0
+    start()
+    errors = []
+
+    def work(s):
+        try:
+            s.run(steps, use_graph=False)
+        except Exception as exc:
+            errors.append(exc)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in pair]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for a, b in zip(state(), want):
+        assert torch.equal(a, b)
