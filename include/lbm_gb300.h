@@ -295,7 +295,10 @@ int lbm_implicit_step_adjoint(int prec, const lbm_implicit_adj_args* a, void* st
  *        for m > nmax), in the layout of tc_anal; then nlon FP32 values
  *        cos(2 pi t / nlon), t = 0..nlon-1, the table of the two surface
  *        rows, which stay on the FMA pipes
- * sf, af and grid9 must be 16-byte aligned (LBM_ERR_ARG otherwise).
+ * sf and af must be 16-byte aligned; in FP32 mode also grid9, and sa3 where the
+ * synthesis is on the tensor cores, while sfs, dft and (longitude analysis on
+ * the FMA pipes) afs need 8 bytes; every other array its real type's alignment
+ * (LBM_ERR_ARG otherwise).
  * Grids whose tables exceed a block's shared memory (227 KB) are refused by
  * prime, run, launch and capture (LBM_ERR_ARG); which ones does not depend on
  * nmem.

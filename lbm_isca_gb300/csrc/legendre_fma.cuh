@@ -573,6 +573,8 @@ __global__ void __launch_bounds__(AN_NT, 1) k_anal(SD<R> d, AnalPlan pl) {
       v.ssrc = ((mm ? pr.m2 : pr.m1) * J) * 2 + f;
     };
     Unit ui(u0, nch, E), uf(u0, nch, E);
+    // (afs may lie off its element's alignment, which cp.async does not take)
+    const bool nats = ((uintptr_t)d.afs & (sizeof(C2<R>) - 1)) == 0;
     Mine vi, vf;
     vi.key = vf.key = -1;
     int ji = 0, jf = 0, si = 0, sf = 0;
@@ -600,8 +602,15 @@ __global__ void __launch_bounds__(AN_NT, 1) k_anal(SD<R> d, AnalPlan pl) {
           }
         if (vi.sj < left) {
           const C2<R>* a = d.afs + (size_t)ui.e * M * J * 2 + vi.ssrc;
-          cp_async_c2(dst + vi.so, a + 2 * (ji + vi.sj));
-          cp_async_c2(dst + vi.so + rst, a + 2 * (J - 1 - ji - vi.sj));
+          const C2<R>*n1 = a + 2 * (ji + vi.sj), *s1 = a + 2 * (J - 1 - ji - vi.sj);
+          C2<R>* o = dst + vi.so;
+          if (nats) {
+            cp_async_c2(o, n1);
+            cp_async_c2(o + rst, s1);
+          } else {
+            o[0] = *n1;
+            o[rst] = *s1;
+          }
         }
         ji += JC;
         if (ji >= JH) { ji = 0; ui.next(nch, E); }

@@ -675,9 +675,16 @@ template <typename R> int validate(const SD<R>& d) {
   for (int f = 0; f < 4; ++f)
     if (d.vd_on[f] && !d.vdiff) return LBM_ERR_ARG;
   if (sizeof(R) == 4 && (!d.dft || !d.grid6 || !d.grid9)) return LBM_ERR_ARG;
-  // 16-byte copies and bulk prefetches read sf, af and grid9
-  auto a16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-  if (!a16(d.sf) || !a16(d.af) || (sizeof(R) == 4 && !a16(d.grid9))) return LBM_ERR_ARG;
+  // 16-byte copies and bulk prefetches read sf, af and grid9, the tensor-core
+  // synthesis sa3; FP32 pairs in one access: sfs, dft and (k_fdft) afs
+  auto off = [](const void* p, int n) { return ((uintptr_t)p & (n - 1)) != 0; };
+  if (off(d.sf, 16) || off(d.af, 16) || (sizeof(R) == 4 && off(d.grid9, 16))) return LBM_ERR_ARG;
+  if (sizeof(R) == 4) {
+    const bool tc_dft = d.legendre && !(d.tc_off & 4) && ftc_supported(d.I, d.K, d.N);
+    if (off(d.sfs, 8) || off(d.dft, 8) || (!tc_dft && off(d.afs, 8)) ||
+        (d.legendre && !(d.tc_off & 2) && off(d.sa3, 16)))
+      return LBM_ERR_ARG;
+  }
   if (d.legendre) {
     // tensor-core analysis: FP32 state, 16-latitude steps, 16-byte af rows,
     // at most 256 table rows, the plan within shared memory

@@ -1,5 +1,6 @@
 """The fused step where its plans and buffers meet a limit: grids that fill a
-block's shared memory, steppers of different sizes side by side."""
+block's shared memory, steppers of different sizes side by side, arrays off their
+elements' alignment."""
 
 import ctypes as C
 import threading
@@ -7,7 +8,7 @@ import threading
 import pytest
 
 from lbm_isca_gb300 import configs
-from test_gpu_step_kernels import (_grid_stepper,
+from test_gpu_step_kernels import (_grid_stepper, _launch, _noise,
                                    test_legendre_kernels_against_fp64_sums as _legendre_sums)
 
 pytestmark = pytest.mark.gpu
@@ -121,3 +122,46 @@ def test_steppers_on_two_threads(torch, precision):
     assert not errors
     for a, b in zip(state(), want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("I,J,N,K,nmem", [(64, 32, 21, 7, 1), (128, 64, 42, 20, 9),
+                                          (128, 50, 31, 2, 3)])
+@pytest.mark.parametrize("precision", ["fp64", "bf16x3"])
+def test_surface_rows_off_their_alignment(torch, I, J, N, K, nmem, precision):
+    """afs on the alignment of its real type only: k_anal reads the same values."""
+    from lbm_isca_gb300._lib import StepperDesc
+    if precision == "bf16x3" and (K % 2 or J % 16):
+        pytest.skip("no tensor-core form")
+    stp = _grid_stepper(torch, I, J, N, K, nmem, precision)
+    _noise(torch, stp.af, 1)
+    _noise(torch, stp.afs, 2)
+    _launch(torch, stp, 1)
+    want = stp.tend.clone(), stp.tends.clone()
+    assert float(want[1].abs().max()) > 0
+    r = torch.view_as_real(stp.afs).reshape(-1)
+    buf = torch.empty(r.numel() + 1, device="cuda", dtype=r.dtype)
+    buf[1:] = r
+    stp.tend.zero_()
+    stp.tends.zero_()
+    d = StepperDesc.from_buffer_copy(stp.desc())
+    d.afs = buf[1:].data_ptr()
+    _launch(torch, stp, 1, desc=d)
+    assert torch.equal(stp.tend, want[0]) and torch.equal(stp.tends, want[1])
+
+
+@pytest.mark.parametrize("precision,tc_off,name,bytes_off", [
+    ("fp64", 0, "sf", 8), ("fp64", 0, "af", 8), ("fp32", 0, "grid9", 8), ("fp32", 0, "sfs", 4),
+    ("fp32", 0, "dft", 4), ("fp32", 0, "afs", 4), ("bf16x3", 7, "afs", 4),
+    ("bf16split", 0, "sa3", 8)])
+def test_alignment_that_kernels_need_is_checked(torch, precision, tc_off, name, bytes_off):
+    """LBM_ERR_ARG before any launch."""
+    from lbm_isca_gb300._lib import LBM_ERR_ARG, StepperDesc, lib
+    stp = _grid_stepper(torch, 64, 32, 21, 4, 1, precision)
+    d = StepperDesc.from_buffer_copy(stp.desc())
+    if stp.legendre:
+        d.tc_off = tc_off
+    setattr(d, name, getattr(d, name) + bytes_off)
+    s = C.c_void_p(stp.stream.cuda_stream)
+    ctl = stp._ctl([(stp._dts[0], False, 0)])
+    assert lib().lbm_stepper_prime(C.byref(d), s) == LBM_ERR_ARG
+    assert lib().lbm_stepper_run(C.byref(d), ctl, 1, s) == LBM_ERR_ARG
