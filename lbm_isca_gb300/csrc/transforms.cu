@@ -320,7 +320,11 @@ static int leg_synth(int B, int nmax, int J, int C, const void* sa, const void* 
     return LBM_ERR_ARG;
   const int CC = leg_cols(C), nch = (C + CC - 1) / CC;
   const int big = (J * CC + LG_NTMAX - 1) / LG_NTMAX;
-  const int nt = (long)M * B * nch * big >= 8 * LG_SMS ? LG_NTMAX : LG_NT;
+  // (one column of many latitudes in FP64: LG_NTMAX rows of table exceed a block)
+  const int nt = (long)M * B * nch * big >= 8 * LG_SMS &&
+                         leg_smem<R>(C, CC, J, LG_NTMAX) <= SMEM_BLOCK
+                     ? LG_NTMAX
+                     : LG_NT;
   const dim3 grid(M, B, nch * ((J * CC + nt - 1) / nt));
   const size_t smem = leg_smem<R>(C, CC, J, nt);
   allow_smem(k_leg_synth<R>);
