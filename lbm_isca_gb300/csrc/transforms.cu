@@ -125,7 +125,7 @@ template <typename R> size_t leg_smem(int C, int CC, int nrow, int nt) {
 // spec[b][m][n][c] (+)= nfac[n] (ca sum_j ta f_a + sb cb sum_j tb f_b)
 template <typename R>
 __global__ void __launch_bounds__(LG_NT)
-k_leg_anal(int M, int J, int C, int CC, int nch, const C2<R>* __restrict__ fa,
+k_leg_anal(int M, int J, int C, int CC, int nch, int z0, const C2<R>* __restrict__ fa,
            const R* __restrict__ ta, int ima, const C2<R>* __restrict__ fb,
            const R* __restrict__ tb, int imb, R sb, const R* __restrict__ nfac, int accumulate,
            C2<R>* __restrict__ spec) {
@@ -133,7 +133,7 @@ k_leg_anal(int M, int J, int C, int CC, int nch, const C2<R>* __restrict__ fa,
   constexpr int TS = LG_T + 1;
   C2<R>* xs = reinterpret_cast<C2<R>*>(smraw);           // [2][LG_T][cc]
   const int m = blockIdx.x, b = blockIdx.y;
-  const int ch = blockIdx.z % nch, part = blockIdx.z / nch;
+  const int z = z0 + (int)blockIdx.z, ch = z % nch, part = z / nch;
   const int c0 = ch * CC, cc = min(CC, C - c0), RR = leg_rows(cc, M, LG_NT);
   R* ts = reinterpret_cast<R*>(xs + 2 * LG_T * cc);      // [2][RR][TS]
   const int tid = threadIdx.x, v0 = part * LG_NT, v = v0 + tid;
@@ -200,14 +200,14 @@ k_leg_anal(int M, int J, int C, int CC, int nch, const C2<R>* __restrict__ fa,
 // four[b][m][j][c] = sum_n ta[m][n][j] ca na[n] sa + sb sum_n tb cb nb[n] sb_
 template <typename R>
 __global__ void __launch_bounds__(LG_NTMAX)
-k_leg_synth(int M, int J, int C, int CC, int nch, const C2<R>* __restrict__ sa,
+k_leg_synth(int M, int J, int C, int CC, int nch, int z0, const C2<R>* __restrict__ sa,
             const R* __restrict__ ta, int ima, const R* __restrict__ na,
             const C2<R>* __restrict__ sbp, const R* __restrict__ tb, int imb,
             const R* __restrict__ nb, R sb, C2<R>* __restrict__ four) {
   extern __shared__ __align__(16) unsigned char smraw[];
   C2<R>* xs = reinterpret_cast<C2<R>*>(smraw);           // [2][LG_T][cc]
   const int m = blockIdx.x, b = blockIdx.y;
-  const int ch = blockIdx.z % nch, part = blockIdx.z / nch;
+  const int z = z0 + (int)blockIdx.z, ch = z % nch, part = z / nch;
   const int c0 = ch * CC, cc = min(CC, C - c0), NT = blockDim.x,
             RR = leg_rows(cc, J, NT);
   R* ts = reinterpret_cast<R*>(xs + 2 * LG_T * cc);      // [2][LG_T][RR]
@@ -293,6 +293,14 @@ int fourier_dispatch(bool fwd, int B, int J, int I, int C, int nmax, const void*
   }
 }
 
+// Launches of nz chunks and value parts, at most LG_ZMAX in the third dimension of a
+// grid: one launch up to 95 thousand columns at T85.
+constexpr int LG_ZMAX = 65535;
+template <typename F> void leg_launches(int M, int B, long nz, F launch) {
+  for (long z = 0; z < nz; z += LG_ZMAX)
+    launch(dim3(M, B, (unsigned)(nz - z < LG_ZMAX ? nz - z : LG_ZMAX)), (int)z);
+}
+
 template <typename R>
 static int leg_anal(int B, int nmax, int J, int C, const void* fa, const void* ta, int ima,
                     const void* fb, const void* tb, int imb, double sb, const void* nfac,
@@ -301,12 +309,14 @@ static int leg_anal(int B, int nmax, int J, int C, const void* fa, const void* t
   if (B < 1 || M < 1 || J < 2 || C < 1 || !fa || !ta || !spec || (fb && !tb))
     return LBM_ERR_ARG;
   const int CC = leg_cols(C), nch = (C + CC - 1) / CC;
-  const dim3 grid(M, B, nch * ((M * CC + LG_NT - 1) / LG_NT));
+  const long nz = (long)nch * ((M * CC + LG_NT - 1) / LG_NT);
   const size_t smem = leg_smem<R>(C, CC, M, LG_NT);
   allow_smem(k_leg_anal<R>);
-  k_leg_anal<R><<<grid, LG_NT, smem, st>>>(
-      M, J, C, CC, nch, (const C2<R>*)fa, (const R*)ta, ima, (const C2<R>*)fb, (const R*)tb, imb,
-      R(sb), (const R*)nfac, acc, (C2<R>*)spec);
+  leg_launches(M, B, nz, [&](dim3 grid, int z0) {
+    k_leg_anal<R><<<grid, LG_NT, smem, st>>>(
+        M, J, C, CC, nch, z0, (const C2<R>*)fa, (const R*)ta, ima, (const C2<R>*)fb,
+        (const R*)tb, imb, R(sb), (const R*)nfac, acc, (C2<R>*)spec);
+  });
   LBM_LAUNCH_CHECK();
   return LBM_OK;
 }
@@ -325,12 +335,14 @@ static int leg_synth(int B, int nmax, int J, int C, const void* sa, const void* 
                          leg_smem<R>(C, CC, J, LG_NTMAX) <= SMEM_BLOCK
                      ? LG_NTMAX
                      : LG_NT;
-  const dim3 grid(M, B, nch * ((J * CC + nt - 1) / nt));
+  const long nz = (long)nch * ((J * CC + nt - 1) / nt);
   const size_t smem = leg_smem<R>(C, CC, J, nt);
   allow_smem(k_leg_synth<R>);
-  k_leg_synth<R><<<grid, nt, smem, st>>>(
-      M, J, C, CC, nch, (const C2<R>*)sa, (const R*)ta, ima, (const R*)na, (const C2<R>*)sbp,
-      (const R*)tb, imb, (const R*)nb, R(sb), (C2<R>*)four);
+  leg_launches(M, B, nz, [&](dim3 grid, int z0) {
+    k_leg_synth<R><<<grid, nt, smem, st>>>(
+        M, J, C, CC, nch, z0, (const C2<R>*)sa, (const R*)ta, ima, (const R*)na,
+        (const C2<R>*)sbp, (const R*)tb, imb, (const R*)nb, R(sb), (C2<R>*)four);
+  });
   LBM_LAUNCH_CHECK();
   return LBM_OK;
 }
