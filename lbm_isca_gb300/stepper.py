@@ -134,8 +134,9 @@ class EnsembleStepper:
     #: keeps the T42L20 day-30 error at 6.3e-6 (with the Legendre
     #: contractions there too it reaches 1.1e-5, over the 1e-5 FP32 gate).
     TC_OFF = {"bf16x3": 3, "bf16split": 0}
-    #: largest FP64 grid-row workspace (20 MB per T42L20 member): bounds what
-    #: it adds to the 15 MB per member of the other buffers
+    #: largest FP64 grid-row workspace (20 MB per T42L20 member beside the 15 MB
+    #: of its other buffers): under a tenth of the device's memory, some 1 270
+    #: members of T42L20 or 160 of T85L40
     GRID_ROWS_BYTES = 24 << 30
 
     def __init__(self, sp, vg, bst, damping, semi, vdiff, nmem, precision="fp64",
@@ -234,16 +235,7 @@ class EnsembleStepper:
         # its plan applies (nlon <= 128, 9 kmax <= 256 rows)
         self.tc_dft = (tc_dft_image(N, I, dev) if self.legendre and I <= 128
                        and 9 * K <= 256 else None)
-        # grid rows between the longitude transforms and the column algebra
-        # (FP64: up to GRID_ROWS_BYTES, else the one-kernel grid part, which
-        # keeps them in shared memory and is about three times slower)
-        rows = E * J * (8 + 15 * K) * I
-        if precision != "fp64" or 8 * rows <= self.GRID_ROWS_BYTES:
-            f = lambda *s_: torch.zeros(s_, device=dev, dtype=rd)   # noqa: E731
-            self.grid6 = f(E, J, 6 + 6 * K, I)
-            self.grid9 = f(E, J, 2 + 9 * K, I)
-        else:
-            self.grid6 = self.grid9 = None
+        self.grid6, self.grid9 = self._grid_rows()
         self.err = torch.zeros(1, device=dev, dtype=torch.int32)
         self.err_member = torch.zeros(E, device=dev, dtype=torch.int32)
         self.frc3 = self.frcs = None
@@ -255,6 +247,23 @@ class EnsembleStepper:
         self._desc = None
         self._oargs = None
         self._null = torch.empty(0, device=dev, dtype=torch.float32)
+
+    def _grid_rows(self):
+        """Grid rows between the longitude transforms and the column algebra
+        (grid6, grid9).  FP64 runs without them, in one kernel that keeps them
+        in shared memory and is about three times slower, beyond
+        GRID_ROWS_BYTES and where the device has no room left for them."""
+        E, J, I, K = self.E, self.J, self.I, self.K
+        fp64 = self.precision == "fp64"
+        if fp64 and 8 * E * J * (8 + 15 * K) * I > self.GRID_ROWS_BYTES:
+            return None, None
+        f = lambda n: torch.zeros((E, J, n, I), device=self.dev, dtype=self.rd)   # noqa: E731
+        try:
+            return f(6 + 6 * K), f(2 + 9 * K)
+        except torch.cuda.OutOfMemoryError:
+            if not fp64:
+                raise
+            return None, None
 
     def _tc_anal_image(self):
         sp = self.sp

@@ -1,6 +1,6 @@
 """The fused step where its plans and buffers meet a limit: grids that fill a
 block's shared memory, steppers of different sizes side by side, arrays off their
-elements' alignment."""
+elements' alignment, FP64 without grid rows."""
 
 import ctypes as C
 import threading
@@ -8,7 +8,7 @@ import threading
 import pytest
 
 from lbm_isca_gb300 import configs
-from test_gpu_step_kernels import (_grid_stepper, _launch, _noise,
+from test_gpu_step_kernels import (_grid_stepper, _launch, _noise, _rel, _stepper,
                                    test_legendre_kernels_against_fp64_sums as _legendre_sums)
 
 pytestmark = pytest.mark.gpu
@@ -165,3 +165,20 @@ def test_alignment_that_kernels_need_is_checked(torch, precision, tc_off, name, 
     ctl = stp._ctl([(stp._dts[0], False, 0)])
     assert lib().lbm_stepper_prime(C.byref(d), s) == LBM_ERR_ARG
     assert lib().lbm_stepper_run(C.byref(d), ctl, 1, s) == LBM_ERR_ARG
+
+
+def test_fp64_run_without_grid_rows(torch, monkeypatch):
+    """EnsembleStepper past the limit of its grid rows: the one-kernel grid part
+    over 20 steps equals the split one to the round-off that the steps carry
+    along (1e-10 of a field's largest value)."""
+    from lbm_isca_gb300.stepper import EnsembleStepper
+    split = _stepper(torch, "T42", 20, 2, "fp64")
+    monkeypatch.setattr(EnsembleStepper, "GRID_ROWS_BYTES", 0)
+    whole = _stepper(torch, "T42", 20, 2, "fp64")
+    assert split.launches_per_step() == 6 and whole.launches_per_step() == 4
+    for s in (split, whole):
+        s.run([(600.0, True)] + [(600.0, False)] * 20)
+        torch.cuda.synchronize()
+        assert s.check_finite()
+    for f in range(4):
+        assert _rel(whole.sa3[:, f], split.sa3[:, f]) < 1e-10

@@ -1,5 +1,5 @@
 """Host side of the ensemble stepper on CPU tensors: packing of rectangles,
-forcings."""
+forcings, the grid-row workspace."""
 
 import contextlib
 import types
@@ -106,3 +106,26 @@ def test_replaced_buffers_outlive_the_queued_steps(host_stepper, monkeypatch):
     old = [t.data_ptr() for t in (s.minv, s.vdm)]
     s.set_timesteps([1200.0])
     assert {(p, id(s.stream)) for p in old} <= set(kept)
+
+
+@pytest.mark.parametrize("full", [(6 + 6 * 3,), (2 + 9 * 3,)])
+def test_fp64_without_room_for_grid_rows(host_stepper, monkeypatch, full):
+    """An FP64 stepper runs without the optional grid rows where the device has
+    no memory left for them, or they exceed the limit; FP32 needs them."""
+    s = host_stepper(4, 3, 2)
+    s.J, s.I, s.precision, s.rd = 6, 16, "fp64", torch.float64
+    assert [tuple(x.shape) for x in s._grid_rows()] == [(2, 6, 24, 16), (2, 6, 29, 16)]
+    s.GRID_ROWS_BYTES = 8 * 2 * 6 * 53 * 16 - 1
+    assert s._grid_rows() == (None, None)
+    del s.GRID_ROWS_BYTES
+    zeros = torch.zeros
+
+    def no_room(shape, **kw):
+        if shape[2] in full:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return zeros(shape, **kw)
+    monkeypatch.setattr(torch, "zeros", no_room)
+    assert s._grid_rows() == (None, None)
+    s.precision, s.rd = "fp32", torch.float32
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        s._grid_rows()
