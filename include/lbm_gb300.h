@@ -252,7 +252,9 @@ int lbm_implicit_step_adjoint(int prec, const lbm_implicit_adj_args* a, void* st
  *        grid kernel (may be NULL in FP64 mode)
  *   frc3 [Ef][4][NS][K], frcs [Ef][NS]: spectral forcing (NULL = none),
  *        Ef = E or 1 (frc_shared = 1)
- *   err [1] int: set nonzero when a non-finite value is produced
+ *   err [1] int, bits: 1 = a non-finite value was produced; 2 = a kernel gave
+ *        up waiting for its own copies or products (every such wait ends after
+ *        two seconds), in any precision: the results of the run are invalid
  *   err_member [E] int or NULL: when given, entry e is also set nonzero when
  *        member e produces a non-finite value, so that the host can name the
  *        members that blew up (the reference's FloatingPointError,
