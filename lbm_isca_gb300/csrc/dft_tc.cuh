@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(FTC_THREADS, 1)
 // latency of its loads: four points at a time; eight members a block, two while
 // those blocks would be fewer than two per SM.  us at T42, before -> after: 8 members
 // 17 -> 8.8, 512 members 87 either way; T21, 48 members 10 -> 6.5.
-inline int fsurf_eb(int E, int J) { return J * ((E + 7) / 8) < 2 * LF_SMS ? 2 : 8; }
+inline int fsurf_eb(int E, int J) { return J * ((E + 7) / 8) < 2 * FILL_SMS ? 2 : 8; }
 inline size_t fsurf_smem(int I, int EB) { return sizeof(float) * (size_t)I * (1 + 2 * EB); }
 
 template <int EB>

@@ -28,7 +28,7 @@ constexpr int IDFT_RG = 8;       // rows per thread item
 // One chunk of rows per block instead of a column's chunks in turn, while the
 // columns leave SMs idle.  us at T42L20, whole columns ->
 // chunks: 1 member 16.0 -> 9.7, 4 members 19.4 -> 16.7, 7 members 21.5 -> 24.
-inline bool idft_chunks(int E, int J) { return E * J < 2 * LF_SMS; }
+inline bool idft_chunks(int E, int J) { return E * J < 2 * FILL_SMS; }
 
 LBM_HD int idft_rows(int K) { return 6 + 6 * K; }
 LBM_HD int fdft_rows(int K) { return 2 + 9 * K; }

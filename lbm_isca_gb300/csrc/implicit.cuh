@@ -13,7 +13,7 @@ struct ImplPlan { int CC, nch, nt; };
 inline ImplPlan impl_plan(int E, int K, int N) {
   const int NP = (N + 2) / 2, most = IM_THREADS / K, nco = N + 2;
   int nch = (nco + most - 1) / most;
-  while (NP * E * nch < 2 * LF_SMS && (nco + nch) / (nch + 1) >= 4) ++nch;
+  while (NP * E * nch < 2 * FILL_SMS && (nco + nch) / (nch + 1) >= 4) ++nch;
   ImplPlan p;
   p.CC = (nco + nch - 1) / nch;
   p.nch = (nco + p.CC - 1) / p.CC;

@@ -100,6 +100,17 @@ LBM_HD int nspec(int N) { return (N + 1) * (N + 2) / 2; }
 
 template <typename R> LBM_D R ld(const R* p) { return __ldg(p); }
 
+// SMs that the rules on chunk and block sizes fill: a GB300's, whatever the device
+// has, so that a launch's shape depends on its sizes alone.
+constexpr int FILL_SMS = 152;
+// SMs of the current device.
+inline int device_sms() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms > 0 ? sms : 1;
+}
+
 // Raises a kernel's dynamic shared memory limit to all that a block can have beside
 // the kernel's `fixed` bytes of static arrays.  The limit is one per kernel and
 // device: set to a launch's own size, it would be lowered by the next caller under

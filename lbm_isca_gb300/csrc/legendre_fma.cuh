@@ -32,8 +32,6 @@
 
 namespace lbm {
 
-constexpr int LF_SMS = 152;           // SMs the chunk rules fill
-
 // ---- packed complex accumulators --------------------------------------------
 template <typename R> struct Cacc;
 template <> struct Cacc<float> {
@@ -236,7 +234,7 @@ struct Unit {
 
 // Members per block of the surface-only kernels.
 inline int members_per_block(int E, int units) {
-  const int eb = (E * units) / (8 * LF_SMS);
+  const int eb = (E * units) / (8 * FILL_SMS);
   return eb < 1 ? 1 : eb > 8 ? 8 : eb;
 }
 
@@ -281,7 +279,7 @@ template <typename R> AnalPlan anal_plan(int E, int J, int K, int N) {
   // few as AN_CW warps hold; more for small ensembles, down to four levels, while
   // units do not outnumber the SMs
   int nch = 1;
-  while (nch < (K + 3) / 4 && NP * E * (nch + 1) <= LF_SMS) ++nch;
+  while (nch < (K + 3) / 4 && NP * E * (nch + 1) <= FILL_SMS) ++nch;
   for (;; ++nch) {
     p.KC = (K + nch - 1) / nch;
     if (even) p.KC += p.KC & 1;
@@ -651,12 +649,13 @@ __global__ void __launch_bounds__(AN_NT, 1) k_anal(SD<R> d, AnalPlan pl) {
 
 template <typename R> void launch_anal(const SD<R>& d, cudaStream_t st, bool attrs) {
   const AnalPlan pl = anal_plan<R>(d.E, d.J, d.K, d.N);
-  const int grid = pl.units < LF_SMS ? pl.units : LF_SMS;
   auto go = [&](auto kern) {
-    if (attrs)
+    if (attrs) {
       allow_smem(kern);
-    else
-      kern<<<grid, 32 * (pl.CW + pl.HW + AN_FW), pl.smem, st>>>(d, pl);
+    } else {
+      const int sms = device_sms();
+      kern<<<pl.units < sms ? pl.units : sms, 32 * (pl.CW + pl.HW + AN_FW), pl.smem, st>>>(d, pl);
+    }
   };
   // 16-byte copies: FP32 rows of an even level count (and always in FP64)
   if constexpr (sizeof(R) == 8) {
@@ -703,7 +702,7 @@ template <typename R> SynthPlan synth_plan(int E, int J, int K, int N) {
   int qc = (sizeof(R) == 4 ? 1 : 3) * NW / p.NJQ;
   if (qc < 1) qc = 1;
   int nch = (nq + qc - 1) / qc;
-  int want = (2 * LF_SMS + NP * E - 1) / (NP * E);
+  int want = (2 * FILL_SMS + NP * E - 1) / (NP * E);
   if (want > nq) want = nq;
   if (nch < want) nch = want;
   auto layout = [&](int ntab, int qc_, int bufs) {
@@ -731,7 +730,7 @@ template <typename R> SynthPlan synth_plan(int E, int J, int K, int N) {
   }
   const int w = p.NJQ * p.QC;
   p.nt = 32 * (w < NW ? w : NW);
-  if (NP * E * p.nch <= 2 * LF_SMS && p.nt < 192) p.nt = 192;   // threads to stage with
+  if (NP * E * p.nch <= 2 * FILL_SMS && p.nt < 192) p.nt = 192;   // threads to stage with
   if (p.nt < 64) p.nt = 64;
   return p;
 }

@@ -438,7 +438,7 @@ namespace lbm {
 // 20.4, 106 against 140).
 template <typename R> int alg_seg(int E, int J, int I, int K) {
   const long warps = (long)E * J * (I / 32);
-  if (warps > 4 * LF_SMS || K < 2) return 0;
+  if (warps > 4 * FILL_SMS || K < 2) return 0;
   const int ls = sizeof(R) == 4 ? 2 : 5, least = (K + ALG_SEGMAX - 1) / ALG_SEGMAX;
   return ls > least ? ls : least;
 }

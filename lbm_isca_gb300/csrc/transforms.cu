@@ -96,7 +96,6 @@ k_fourier_inv(int J, int C, int M, const C2<R>* __restrict__ four, const R* __re
 // us at T42, 20 levels, before -> after: 32 members, analysis of two tables 559 -> 295,
 // of one 292 -> 154, synthesis (mean of three calls) 411 -> 260; one member, analysis
 // 56 -> 26, synthesis 65 -> 24.
-constexpr int LG_SMS = 152;     // SMs to fill
 constexpr int LG_NT = 128;      // threads of a block ...
 constexpr int LG_NTMAX = 512;   // ... of the synthesis of many batch items
 constexpr int LG_T = 32;        // summation indices per staged tile
@@ -331,7 +330,7 @@ static int leg_synth(int B, int nmax, int J, int C, const void* sa, const void* 
   const int CC = leg_cols(C), nch = (C + CC - 1) / CC;
   const int big = (J * CC + LG_NTMAX - 1) / LG_NTMAX;
   // (one column of many latitudes in FP64: LG_NTMAX rows of table exceed a block)
-  const int nt = (long)M * B * nch * big >= 8 * LG_SMS &&
+  const int nt = (long)M * B * nch * big >= 8 * FILL_SMS &&
                          leg_smem<R>(C, CC, J, LG_NTMAX) <= SMEM_BLOCK
                      ? LG_NTMAX
                      : LG_NT;
