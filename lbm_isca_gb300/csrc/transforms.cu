@@ -258,6 +258,102 @@ k_leg_synth(int M, int J, int C, int CC, int nch, int z0, const C2<R>* __restric
   if (act) four[(((size_t)b * M + m) * J + jj) * C + c0 + c] = acc;
 }
 
+// The same sums with the column values of a whole sum staged once: a block takes all
+// values of one (m, batch, LG_COLS columns), a thread every LG_ROWS-th n or j of one
+// column, its table rows read in place.  Fewer stagings and half the shared-memory
+// reads per product, but lanes without a column idle, a block walks its rows in
+// turn, and shared memory holds 454 indices in FP64.  leg_whole() gives the sizes
+// at which this form is the faster one; the results are the same bits.
+constexpr int LG_COLS = 16;     // columns of a block
+constexpr int LG_ROWS = 16;     // thread rows (n or j)
+
+// spec[b][m][n][c] (+)= nfac[n] (ca sum_j ta f_a + sb cb sum_j tb f_b)
+template <typename R>
+__global__ void __launch_bounds__(LG_COLS * LG_ROWS)
+k_leg_anal16(int M, int J, int C, const C2<R>* __restrict__ fa, const R* __restrict__ ta,
+           int ima, const C2<R>* __restrict__ fb, const R* __restrict__ tb, int imb, R sb,
+           const R* __restrict__ nfac, int accumulate, C2<R>* __restrict__ spec) {
+  extern __shared__ unsigned char smraw[];
+  C2<R>* sa = reinterpret_cast<C2<R>*>(smraw);   // [J][LG_COLS]
+  C2<R>* sbb = sa + J * LG_COLS;
+  const int m = blockIdx.x, b = blockIdx.y, c0 = blockIdx.z * LG_COLS;
+  const int cc = min(LG_COLS, C - c0);
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * LG_COLS + tx;
+  for (int idx = tid; idx < J * LG_COLS; idx += LG_COLS * LG_ROWS) {
+    const int jj = idx / LG_COLS, c = idx % LG_COLS;
+    const size_t g = (((size_t)b * M + m) * J + jj) * C + c0 + c;
+    sa[idx] = (c < cc) ? fa[g] : cmk<R>(0, 0);
+    if (fb) sbb[idx] = (c < cc) ? fb[g] : cmk<R>(0, 0);
+  }
+  __syncthreads();
+  if (tx >= cc) return;
+  const R mm = R(m);
+  for (int n = ty; n < M; n += LG_ROWS) {
+    const size_t o = (((size_t)b * M + m) * M + n) * C + c0 + tx;
+    if (n < m) {
+      if (!accumulate) spec[o] = cmk<R>(0, 0);
+      continue;
+    }
+    const R* pa = ta + ((size_t)m * M + n) * J;
+    C2<R> acc = cmk<R>(0, 0), accb = cmk<R>(0, 0);
+    for (int jj = 0; jj < J; ++jj) cfma(acc, pa[jj], sa[jj * LG_COLS + tx]);
+    if (ima) acc = im_mul(acc, mm);
+    if (fb) {
+      const R* pb = tb + ((size_t)m * M + n) * J;
+      for (int jj = 0; jj < J; ++jj) cfma(accb, pb[jj], sbb[jj * LG_COLS + tx]);
+      if (imb) accb = im_mul(accb, mm);
+      acc = acc + accb * sb;
+    }
+    if (nfac) acc = acc * nfac[n];
+    if (accumulate) acc = acc + spec[o];
+    spec[o] = acc;
+  }
+}
+
+// four[b][m][j][c] = sum_n ta[m][n][j] ca na[n] sa + sb sum_n tb cb nb[n] sb_
+template <typename R>
+__global__ void __launch_bounds__(LG_COLS * LG_ROWS)
+k_leg_synth16(int M, int J, int C, const C2<R>* __restrict__ sa, const R* __restrict__ ta,
+            int ima, const R* __restrict__ na, const C2<R>* __restrict__ sbp,
+            const R* __restrict__ tb, int imb, const R* __restrict__ nb, R sb,
+            C2<R>* __restrict__ four) {
+  extern __shared__ unsigned char smraw[];
+  C2<R>* xa = reinterpret_cast<C2<R>*>(smraw);   // [M][LG_COLS]
+  C2<R>* xb = xa + M * LG_COLS;
+  const int m = blockIdx.x, b = blockIdx.y, c0 = blockIdx.z * LG_COLS;
+  const int cc = min(LG_COLS, C - c0);
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * LG_COLS + tx;
+  const R mm = R(m);
+  for (int idx = tid; idx < M * LG_COLS; idx += LG_COLS * LG_ROWS) {
+    const int n = idx / LG_COLS, c = idx % LG_COLS;
+    C2<R> va = cmk<R>(0, 0), vb = cmk<R>(0, 0);
+    if (c < cc && n >= m) {
+      const size_t g = (((size_t)b * M + m) * M + n) * C + c0 + c;
+      va = sa[g];
+      if (ima) va = im_mul(va, mm);
+      if (na) va = va * na[n];
+      if (sbp) {
+        vb = sbp[g];
+        if (imb) vb = im_mul(vb, mm);
+        if (nb) vb = vb * nb[n];
+        vb = vb * sb;
+      }
+    }
+    xa[idx] = va;
+    xb[idx] = vb;
+  }
+  __syncthreads();
+  if (tx >= cc) return;
+  for (int jj = ty; jj < J; jj += LG_ROWS) {
+    C2<R> acc = cmk<R>(0, 0);
+    for (int n = m; n < M; ++n) {
+      cfma(acc, ta[((size_t)m * M + n) * J + jj], xa[n * LG_COLS + tx]);
+      if (sbp) cfma(acc, tb[((size_t)m * M + n) * J + jj], xb[n * LG_COLS + tx]);
+    }
+    four[(((size_t)b * M + m) * J + jj) * C + c0 + tx] = acc;
+  }
+}
+
 template <typename R, int I>
 int launch_fourier(bool fwd, int B, int J, int C, int M, const void* in, const void* js,
                    const void* tw, void* out, cudaStream_t st) {
@@ -300,6 +396,23 @@ template <typename F> void leg_launches(int M, int B, long nz, F launch) {
     launch(dim3(M, B, (unsigned)(nz - z < LG_ZMAX ? nz - z : LG_ZMAX)), (int)z);
 }
 
+// Whether the 16-column form takes a sum: batches that fill the SMs, and columns that
+// fill its chunks (at most `fill` lanes per 100 columns; idle lanes cost as much as
+// others).  us, flat values -> 16-column form.  FP32: T42, 32 items of 64 columns,
+// analysis of one table 97 -> 66, of two 140 -> 123, synthesis 95 -> 64 and 130 -> 113;
+// T21, 128 items of 48, 51 -> 30 and 64 -> 36.  FP64: T42, 32 items of 64 columns,
+// synthesis 476 -> 446 and 989 -> 897.  The flat form keeps, FP32: T21, 128 items of 20
+// columns, 23 (21) and T42, four items of 16, 6 (9); FP64: fewer items, more idle
+// lanes, and every analysis (T42, 32 items of 64: 448 (509)).
+template <typename R> bool leg_whole(bool synth, bool two, int n, int B, int C) {
+  const int nch = (C + LG_COLS - 1) / LG_COLS;
+  if (nch > 65535 || sizeof(C2<R>) * 2 * (size_t)n * LG_COLS > SMEM_BLOCK) return false;
+  if (sizeof(R) == 8) return synth && 100 * LG_COLS * nch <= 115 * C && (long)B * nch >= 40;
+  const int fill = synth ? (two ? 150 : 190) : (two ? 130 : 150);
+  const long most = synth ? (two ? 40 : 16) : 10;
+  return 100 * (long)LG_COLS * nch <= (long)fill * C && (long)B * nch >= most;
+}
+
 template <typename R>
 static int leg_anal(int B, int nmax, int J, int C, const void* fa, const void* ta, int ima,
                     const void* fb, const void* tb, int imb, double sb, const void* nfac,
@@ -307,6 +420,15 @@ static int leg_anal(int B, int nmax, int J, int C, const void* fa, const void* t
   const int M = nmax + 1;
   if (B < 1 || M < 1 || J < 2 || C < 1 || !fa || !ta || !spec || (fb && !tb))
     return LBM_ERR_ARG;
+  if (leg_whole<R>(false, fb != nullptr, J, B, C)) {
+    allow_smem(k_leg_anal16<R>);
+    k_leg_anal16<R><<<dim3(M, B, (C + LG_COLS - 1) / LG_COLS), dim3(LG_COLS, LG_ROWS),
+                      sizeof(C2<R>) * 2 * J * LG_COLS, st>>>(
+        M, J, C, (const C2<R>*)fa, (const R*)ta, ima, (const C2<R>*)fb, (const R*)tb, imb, R(sb),
+        (const R*)nfac, acc, (C2<R>*)spec);
+    LBM_LAUNCH_CHECK();
+    return LBM_OK;
+  }
   const int CC = leg_cols(C), nch = (C + CC - 1) / CC;
   const long nz = (long)nch * ((M * CC + LG_NT - 1) / LG_NT);
   const size_t smem = leg_smem<R>(C, CC, M, LG_NT);
@@ -327,10 +449,23 @@ static int leg_synth(int B, int nmax, int J, int C, const void* sa, const void* 
   const int M = nmax + 1;
   if (B < 1 || M < 1 || J < 2 || C < 1 || !sa || !ta || !four || (sbp && !tb))
     return LBM_ERR_ARG;
+  if (leg_whole<R>(true, sbp != nullptr, M, B, C)) {
+    allow_smem(k_leg_synth16<R>);
+    k_leg_synth16<R><<<dim3(M, B, (C + LG_COLS - 1) / LG_COLS), dim3(LG_COLS, LG_ROWS),
+                       sizeof(C2<R>) * 2 * M * LG_COLS, st>>>(
+        M, J, C, (const C2<R>*)sa, (const R*)ta, ima, (const R*)na, (const C2<R>*)sbp,
+        (const R*)tb, imb, (const R*)nb, R(sb), (C2<R>*)four);
+    LBM_LAUNCH_CHECK();
+    return LBM_OK;
+  }
   const int CC = leg_cols(C), nch = (C + CC - 1) / CC;
   const int big = (J * CC + LG_NTMAX - 1) / LG_NTMAX;
-  // (one column of many latitudes in FP64: LG_NTMAX rows of table exceed a block)
-  const int nt = (long)M * B * nch * big >= 8 * FILL_SMS &&
+  // LG_NTMAX values a block where those blocks are eight per SM; three for two tables
+  // in FP64, whose staged factors cost most (us with 128 -> 512, T42, two tables: one
+  // item of 100 columns 83 -> 64, four of 31 105 -> 90), but not for a few columns.
+  // (One column of many latitudes in FP64: that many table rows exceed a block.)
+  const int per_sm = sizeof(R) == 8 && sbp && CC >= 8 ? 3 : 8;
+  const int nt = (long)M * B * nch * big >= per_sm * FILL_SMS &&
                          leg_smem<R>(C, CC, J, LG_NTMAX) <= SMEM_BLOCK
                      ? LG_NTMAX
                      : LG_NT;
