@@ -71,12 +71,6 @@ template <> struct Cacc<double> {
   }
   LBM_D C2<double> get() const { return v; }
 };
-// Two adjacent complex values from shared memory (16-byte aligned).
-LBM_D void ld2(const C2<float>* p, unsigned long long& a, unsigned long long& b) {
-  const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p);
-  a = t.x;
-  b = t.y;
-}
 LBM_D void ld1(const C2<float>* p, unsigned long long& a) {
   a = *reinterpret_cast<const unsigned long long*>(p);
 }
@@ -93,10 +87,6 @@ LBM_D C2<double> ldc(const C2<double>* p) {
 }
 LBM_D void stc(C2<double>* p, C2<double> a) {
   *reinterpret_cast<double2*>(p) = make_double2(a.x, a.y);
-}
-LBM_D void ld2(const C2<double>* p, C2<double>& a, C2<double>& b) {
-  a = ldc(p);
-  b = ldc(p + 1);
 }
 LBM_D void ld1(const C2<double>* p, C2<double>& a) { a = ldc(p); }
 // One complex value to global memory; nat: the address is a multiple of its size.
@@ -254,7 +244,7 @@ template <typename R> struct AnalCfg;
 template <> struct AnalCfg<float> { static constexpr int RT = 3, LP = 2; };
 template <> struct AnalCfg<double> { static constexpr int RT = 1, LP = 1; };
 constexpr int AN_CW = 11;             // most consumer warps
-constexpr int AN_FW = 5;              // warps that copy (and fold); one with bulk copies
+constexpr int AN_FW = 5;              // warps that copy (FP64: and fold)
 constexpr int AN_NV = 8;              // most vectors of a stage per copying thread
 constexpr int AN_NS = 6, AN_DEPTH = 4;   // stages of the ring, and how many are being loaded
 constexpr int AN_NT = 32 * (AN_CW + AN_FW);

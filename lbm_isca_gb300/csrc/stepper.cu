@@ -428,7 +428,6 @@ __global__ void k_ps_flush(SD<R> d, int ps_mode) {
 namespace lbm {
 
 // ---- launch configuration ------------------------------------------------------
-// Resident k_alg blocks of I threads (see the kernel).
 // Levels per segment of k_alg, 0 for whole columns: segments while the columns are
 // less than a warp per SM partition (one member of T42: 256 of 608).  Two
 // levels in FP32, bound by latency (T42L20, one member, us: 22 whole, 9.0, 10.6, 11.6
