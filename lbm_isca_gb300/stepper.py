@@ -321,8 +321,8 @@ class EnsembleStepper:
         packed = [None if x is None else self._gather(x, x is not frc_pi) for x in fields]
         # to the buffers' sizes, which refuses a wrong one before the first write:
         # a refused call leaves the forcing as it was
-        sizes = [(Ef, self.NS, self.K)] * 4 + [(Ef, self.NS)]
-        packed = [p if p is None else p.expand(n) for p, n in zip(packed, sizes)]
+        packed = [p if p is None or p.shape[0] == Ef else p.expand(Ef, *p.shape[1:])
+                  for p in packed]
         cur = torch.cuda.current_stream(self.dev)
         new_ptrs = self.frc3 is None or self.frc3.shape[0] != Ef
         if new_ptrs:
