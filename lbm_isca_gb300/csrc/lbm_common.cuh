@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include "../../include/lbm_gb300.h"
 
 #define LBM_HD __host__ __device__ __forceinline__
@@ -103,12 +104,16 @@ template <typename R> LBM_D R ld(const R* p) { return __ldg(p); }
 // SMs that the rules on chunk and block sizes fill: a GB300's, whatever the device
 // has, so that a launch's shape depends on its sizes alone.
 constexpr int FILL_SMS = 152;
-// SMs of the current device.
+// SMs of the current device (asked once: a launch-bound step feels the query).
 inline int device_sms() {
+  static std::atomic<int> known[64];
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms > 0 ? sms : 1;
+  if (sms < 1) return 1;
+  if (dev >= 0 && dev < 64) known[dev].store(sms, std::memory_order_relaxed);
+  return sms;
 }
 
 // Raises a kernel's dynamic shared memory limit to all that a block can have beside
